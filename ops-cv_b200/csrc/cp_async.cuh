@@ -12,6 +12,10 @@ __device__ __forceinline__ void CpAsync16(void* smem, const void* gmem)
                  "l"(gmem)
                  : "memory");
 }
+__device__ __forceinline__ void CpAsync16(uint32_t smem, const void* gmem)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void CpAsync4(void* smem, const void* gmem)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(

@@ -147,6 +147,10 @@ bool BilinearFwdTakesPitch(Dt dt, Layout lay, const void* x, const void* y, Shap
 cudaError_t BilinearBwdGather(Dt dtIn, Dt dtOut, Layout lay, const void* go, void* gi, Shape4 sh, LerpAxis th,
                               LerpAxis tw, RangeAxis rh, RangeAxis rw, const BilinearPlan& plan, cudaStream_t s,
                               bool buildTables = false, const ViewStrides* gradsPitch = nullptr);
+// The row walks that serve any up-scale (bilinear_backward_walk.cu): launches one and returns true, or returns false
+// without a launch (down-scales, user scales that run past the input, rows too long for a block).
+bool BilinearBwdWalk(Dt dtIn, Dt dtOut, Layout lay, const void* go, void* gi, Shape4 sh, AxisGeom gh, AxisGeom gw,
+                     bool halfPixel, cudaStream_t s);
 bool BilinearBwdTakesPitch(Dt dtIn, Dt dtOut, Layout lay, const void* go, const void* gi, Shape4 sh,
                            const BilinearPlan& plan, const ViewStrides& grads);
 // Scatter backward with fp32 atomics into `acc` (fp32, N*C*hin*win, zeroed by this call). If dtOut is fp32 the

@@ -1551,6 +1551,12 @@ int32_t RowsForOccupancy(int64_t threadsPerTileRowSet, int32_t rows)
     return static_cast<int32_t>(std::max<int64_t>({8, CeilDiv(rows, tiles), CeilDiv(rows, 65535)}));
 }
 
+template <typename T>
+constexpr Dt DtOf()
+{
+    return std::is_same<T, float>::value ? Dt::F32 : (std::is_same<T, __half>::value ? Dt::F16 : Dt::BF16);
+}
+
 template <typename TIn, typename TOut>
 cudaError_t LaunchGather(Layout lay, const void* go, void* gi, Shape4 sh, LerpAxis th, LerpAxis tw, RangeAxis rh,
                          RangeAxis rw, const BilinearPlan& plan, cudaStream_t s, bool buildTables,
@@ -1673,6 +1679,8 @@ cudaError_t LaunchGather(Layout lay, const void* go, void* gi, Shape4 sh, LerpAx
                 BilinearBwdW2Kernel<TIn, TOut><<<grid, block, 0, s>>>(pg, po, planes, sh.hin, sh.win, sh.hout, th, tw,
                                                                       rh, tileRows);
             }
+        } else if (BilinearBwdWalk(DtOf<TIn>(), DtOf<TOut>(), lay, go, gi, sh, plan.geomH, plan.geomW, plan.halfPixel, s)) {
+            // launched
         } else if (plan.schedule != BilinearPlan::kDirect && plan.tileRows > 0) {
             needTables();
             const int32_t tiles = static_cast<int32_t>(CeilDiv(sh.hin, plan.tileRows));
@@ -1703,7 +1711,7 @@ cudaError_t LaunchGather(Layout lay, const void* go, void* gi, Shape4 sh, LerpAx
                 }
             });
         }
-    } else {
+    } else if (!BilinearBwdWalk(DtOf<TIn>(), DtOf<TOut>(), lay, go, gi, sh, plan.geomH, plan.geomW, plan.halfPixel, s)) {
         needTables();
         const int elem = sizeof(TIn) > sizeof(TOut) ? sizeof(TIn) : sizeof(TOut);
         const int v = PickVec(elem, sh.c, {go, gi});
