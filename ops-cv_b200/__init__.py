@@ -1,19 +1,23 @@
-"""opscv_b200: ctypes caller of libopscv_b200.so, the B200 implementation of the ops-cv resampling aclnn API.
+"""opscv_b200: Python caller of libopscv_b200.so, the B200 implementation of the ops-cv resampling aclnn API.
 
 The product is the shared library (C ABI declared in include/aclnn_resample.h and include/opscv_acl.h). This
 package is the thin Python caller used by the tests and the benchmark, playing the part that the reference's
 ATK `pyaclnn` backend plays for the original library: it builds aclTensor handles over torch CUDA tensors
-(device memory and streams only), runs the two-phase calls and raises on any non-zero status. It contains no
-arithmetic and no fallback: if the library is missing, loading fails.
+(device memory and streams only), runs the two-phase calls and raises on any non-zero status. The operators go through
+a native binding (_opscv_torch.so, one call per operator); the objects of the C API are reachable through ctypes as
+well. It contains no arithmetic and no fallback: if a library is missing, loading fails.
 
 The directory name has a hyphen, so import it through `__graft_entry__.load_package()` (registers it as the
 module `opscv_b200`).
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libopscv_b200.so")
+NATIVE_PATH = os.path.join(_HERE, "lib", "_opscv_torch.so")
 CSRC_DIR = os.path.join(_HERE, "csrc")
 
 # aclDataType / aclFormat values (include/opscv_acl.h)
@@ -129,6 +133,19 @@ def lib():
             fn.argtypes = argtypes
         _lib = handle
     return _lib
+
+
+def native_module():
+    """Load the native binding of the operators. Raises OSError if it has not been built."""
+    lib()
+    if not os.path.exists(NATIVE_PATH):
+        raise OSError(f"{NATIVE_PATH} not found: build it with __graft_entry__.build() or `make -C {CSRC_DIR}`")
+    import torch  # noqa: F401  (the binding links against torch's libraries, which this loads)
+    loader = importlib.machinery.ExtensionFileLoader("_opscv_torch", NATIVE_PATH)
+    spec = importlib.util.spec_from_loader("_opscv_torch", loader)
+    module = importlib.util.module_from_spec(spec)
+    loader.exec_module(module)
+    return module
 
 
 from .aclnn import *  # noqa: E402,F401,F403

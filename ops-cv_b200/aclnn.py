@@ -5,7 +5,7 @@ import torch
 
 from . import (ACL_BF16, ACL_DOUBLE, ACL_FLOAT, ACL_FLOAT16, ACL_FORMAT_NCDHW, ACL_FORMAT_NCHW, ACL_FORMAT_NCL, ACL_FORMAT_ND,
                ACL_FORMAT_NDHWC, ACL_FORMAT_NHWC,
-               ACL_INT32, ACL_INT64, ACL_OPT_DETERMINISTIC, ACL_UINT8, lib)
+               ACL_INT32, ACL_INT64, ACL_OPT_DETERMINISTIC, ACL_UINT8, lib, native_module)
 
 __all__ = [
     "AclnnError", "acl_tensor", "int_array", "bool_array", "float_array", "resize", "two_phase", "set_deterministic", "set_backward_algo",
@@ -29,6 +29,19 @@ class AclnnError(RuntimeError):
     def __init__(self, api, status):
         self.status = status
         super().__init__(f"{api} returned {status}: {last_error()}")
+
+
+_native = None
+
+
+def native():
+    """The native binding (loaded once; OSError if it has not been built)."""
+    global _native
+    if _native is None:
+        module = native_module()
+        module.set_error_class(AclnnError)
+        _native = module
+    return _native
 
 
 def last_error():
@@ -169,34 +182,20 @@ def _out_shape(x, out_hw, fmt):
 
 
 # ---- operators ------------------------------------------------------------------------------------------------
+# Each wrapper is one call of the native binding (csrc/py_binding.cpp), which allocates the result unless `out` is given,
+# builds the acl objects and runs both phases on the current stream of the tensor's device.
 
 def upsample_nearest2d(x, out_hw, fmt="NCHW", scales=None, out=None, workspace=None):
-    out = torch.empty(_out_shape(x, out_hw, fmt), dtype=x.dtype, device=x.device) if out is None else out
-    tx, ty, size = acl_tensor(x, fmt), acl_tensor(out, fmt), int_array(out_hw)
-    if scales is None:
-        two_phase("aclnnUpsampleNearest2d", [tx.ptr, size.ptr, ty.ptr], x.device, workspace)
-    else:
-        two_phase("aclnnUpsampleNearest2dV2", [tx.ptr, size.ptr, float(scales[0]), float(scales[1]), ty.ptr],
-                  x.device, workspace)
-    return out
+    return native().upsample_nearest2d(x, out_hw, fmt, scales, out, workspace)
 
 
 def upsample_nearest2d_backward(grad_out, out_hw, input_size, fmt="NCHW", scales=(0.0, 0.0), out=None,
                                 workspace=None):
-    out = torch.empty(tuple(input_size), dtype=grad_out.dtype, device=grad_out.device) if out is None else out
-    tg, ty = acl_tensor(grad_out, fmt), acl_tensor(out, fmt)
-    osz, isz = int_array(out_hw), int_array(input_size)
-    two_phase("aclnnUpsampleNearest2dBackward", [tg.ptr, osz.ptr, isz.ptr, float(scales[0]), float(scales[1]), ty.ptr],
-              grad_out.device, workspace)
-    return out
+    return native().upsample_nearest2d_backward(grad_out, out_hw, input_size, fmt, scales, out, workspace)
 
 
 def upsample_bilinear2d(x, out_hw, align_corners=False, fmt="NCHW", scales=(0.0, 0.0), out=None, workspace=None):
-    out = torch.empty(_out_shape(x, out_hw, fmt), dtype=x.dtype, device=x.device) if out is None else out
-    tx, ty, size = acl_tensor(x, fmt), acl_tensor(out, fmt), int_array(out_hw)
-    two_phase("aclnnUpsampleBilinear2d", [tx.ptr, size.ptr, bool(align_corners), float(scales[0]), float(scales[1]),
-                                          ty.ptr], x.device, workspace)
-    return out
+    return native().upsample_bilinear2d(x, out_hw, align_corners, fmt, scales, out, workspace)
 
 
 def upsample_bilinear2d_no_alloc(x, out_hw, align_corners=False, fmt="NCHW", scales=(0.0, 0.0), out=None):
@@ -215,149 +214,76 @@ def upsample_bilinear2d_no_alloc(x, out_hw, align_corners=False, fmt="NCHW", sca
 
 def upsample_bilinear2d_backward(grad_out, out_hw, input_size, align_corners=False, fmt="NCHW", scales=(0.0, 0.0),
                                  out=None, out_dtype=None, v2=False, workspace=None):
-    if out is None:
-        out = torch.empty(tuple(input_size), dtype=out_dtype or grad_out.dtype, device=grad_out.device)
-    tg, ty = acl_tensor(grad_out, fmt), acl_tensor(out, fmt)
-    osz, isz = int_array(out_hw), int_array(input_size)
-    name = "aclnnUpsampleBilinear2dBackwardV2" if v2 else "aclnnUpsampleBilinear2dBackward"
-    two_phase(name, [tg.ptr, osz.ptr, isz.ptr, bool(align_corners), float(scales[0]), float(scales[1]), ty.ptr],
-              grad_out.device, workspace)
-    return out
+    if out is None and out_dtype is not None:
+        out = torch.empty(tuple(input_size), dtype=out_dtype, device=grad_out.device)
+    run = native().upsample_bilinear2d_backward_v2 if v2 else native().upsample_bilinear2d_backward
+    return run(grad_out, out_hw, input_size, align_corners, fmt, scales, out, workspace)
 
 
 def upsample_bicubic2d_aa(x, out_hw, align_corners=False, scales=(0.0, 0.0), out=None, workspace=None):
-    out = torch.empty(_out_shape(x, out_hw, "NCHW"), dtype=x.dtype, device=x.device) if out is None else out
-    tx, ty, size = acl_tensor(x, "NCHW"), acl_tensor(out, "NCHW"), int_array(out_hw)
-    two_phase("aclnnUpsampleBicubic2dAA", [tx.ptr, size.ptr, bool(align_corners), float(scales[0]), float(scales[1]),
-                                           ty.ptr], x.device, workspace)
-    return out
+    return native().upsample_bicubic2d_aa(x, out_hw, align_corners, "NCHW", scales, out, workspace)
 
 
 def upsample_bicubic2d_aa_grad(grad_out, out_hw, input_size, align_corners=False, scales=(0.0, 0.0), out=None,
                                workspace=None):
-    out = torch.empty(tuple(input_size), dtype=grad_out.dtype, device=grad_out.device) if out is None else out
-    tg, ty = acl_tensor(grad_out, "NCHW"), acl_tensor(out, "NCHW")
-    osz, isz = int_array(out_hw), int_array(input_size)
-    two_phase("aclnnUpsampleBicubic2dAAGrad", [tg.ptr, osz.ptr, isz.ptr, bool(align_corners), float(scales[0]),
-                                               float(scales[1]), ty.ptr], grad_out.device, workspace)
-    return out
+    return native().upsample_bicubic2d_aa_grad(grad_out, out_hw, input_size, align_corners, "NCHW", scales, out,
+                                               workspace)
 
 
 def upsample_nearest_exact2d(x, out_hw, fmt="NCHW", scales=(0.0, 0.0), out=None, workspace=None):
-    out = torch.empty(_out_shape(x, out_hw, fmt), dtype=x.dtype, device=x.device) if out is None else out
-    tx, ty, size = acl_tensor(x, fmt), acl_tensor(out, fmt), int_array(out_hw)
-    two_phase("aclnnUpsampleNearestExact2d", [tx.ptr, size.ptr, float(scales[0]), float(scales[1]), ty.ptr], x.device,
-              workspace)
-    return out
+    return native().upsample_nearest_exact2d(x, out_hw, fmt, scales, out, workspace)
 
 
 def upsample_nearest_exact2d_backward(grad_out, out_hw, input_size, scales=(0.0, 0.0), out=None, workspace=None):
-    out = torch.empty(tuple(input_size), dtype=grad_out.dtype, device=grad_out.device) if out is None else out
-    tg, ty = acl_tensor(grad_out, "NCHW"), acl_tensor(out, "NCHW")
-    osz, isz = int_array(out_hw), int_array(input_size)
-    two_phase("aclnnUpsampleNearestExact2dBackward", [tg.ptr, osz.ptr, isz.ptr, float(scales[0]), float(scales[1]),
-                                                      ty.ptr], grad_out.device, workspace)
-    return out
+    return native().upsample_nearest_exact2d_backward(grad_out, out_hw, input_size, "NCHW", scales, out, workspace)
 
 
 def upsample_nearest_exact1d(x, out_l, scale=0.0, fmt="NCL", out=None, workspace=None):
-    out = torch.empty((x.shape[0], x.shape[1], out_l), dtype=x.dtype, device=x.device) if out is None else out
-    tx, ty, size = acl_tensor(x, fmt), acl_tensor(out, fmt), int_array([out_l])
-    two_phase("aclnnUpsampleNearestExact1d", [tx.ptr, size.ptr, float(scale), ty.ptr], x.device, workspace)
-    return out
+    return native().upsample_nearest_exact1d(x, out_l, scale, fmt, out, workspace)
 
 
 def upsample_nearest_exact1d_backward(grad_out, out_l, input_size, scale=0.0, fmt="NCL", out=None, workspace=None):
-    out = torch.empty(tuple(input_size), dtype=grad_out.dtype, device=grad_out.device) if out is None else out
-    tg, ty = acl_tensor(grad_out, fmt), acl_tensor(out, fmt)
-    osz, isz = int_array([out_l]), int_array(input_size)
-    two_phase("aclnnUpsampleNearestExact1dBackward", [tg.ptr, osz.ptr, isz.ptr, float(scale), ty.ptr],
-              grad_out.device, workspace)
-    return out
+    return native().upsample_nearest_exact1d_backward(grad_out, out_l, input_size, scale, fmt, out, workspace)
 
 
 def upsample_nearest3d(x, out_dhw, fmt="NCDHW", scales=(0.0, 0.0, 0.0), exact=False, out=None, workspace=None):
-    if out is None:
-        shape = (x.shape[0], *out_dhw, x.shape[4]) if fmt == "NDHWC" else (x.shape[0], x.shape[1], *out_dhw)
-        out = torch.empty(shape, dtype=x.dtype, device=x.device)
-    tx, ty, size = acl_tensor(x, fmt), acl_tensor(out, fmt), int_array(list(out_dhw))
-    name = "aclnnUpsampleNearestExact3d" if exact else "aclnnUpsampleNearest3d"
-    two_phase(name, [tx.ptr, size.ptr, float(scales[0]), float(scales[1]), float(scales[2]), ty.ptr], x.device,
-              workspace)
-    return out
+    return native().upsample_nearest3d(x, out_dhw, fmt, scales, exact, out, workspace)
 
 
 def upsample_nearest3d_backward(grad_out, out_dhw, input_size, fmt="NCDHW", scales=(0.0, 0.0, 0.0), exact=False,
                                 out=None, workspace=None):
-    out = torch.empty(tuple(input_size), dtype=grad_out.dtype, device=grad_out.device) if out is None else out
-    tg, ty = acl_tensor(grad_out, fmt), acl_tensor(out, fmt)
-    osz, isz = int_array(list(out_dhw)), int_array(list(input_size))
-    name = "aclnnUpsampleNearestExact3dBackward" if exact else "aclnnUpsampleNearest3dBackward"
-    two_phase(name, [tg.ptr, osz.ptr, isz.ptr, float(scales[0]), float(scales[1]), float(scales[2]), ty.ptr],
-              grad_out.device, workspace)
-    return out
+    return native().upsample_nearest3d_backward(grad_out, out_dhw, input_size, fmt, scales, out, workspace, exact)
 
 
 def upsample_trilinear3d(x, out_dhw, align_corners=False, fmt="NCDHW", scales=(0.0, 0.0, 0.0), out=None,
                          workspace=None):
-    if out is None:
-        shape = (x.shape[0], *out_dhw, x.shape[4]) if fmt == "NDHWC" else (x.shape[0], x.shape[1], *out_dhw)
-        out = torch.empty(shape, dtype=x.dtype, device=x.device)
-    tx, ty, size = acl_tensor(x, fmt), acl_tensor(out, fmt), int_array(list(out_dhw))
-    two_phase("aclnnUpsampleTrilinear3d", [tx.ptr, size.ptr, bool(align_corners), float(scales[0]), float(scales[1]),
-                                           float(scales[2]), ty.ptr], x.device, workspace)
-    return out
+    return native().upsample_trilinear3d(x, out_dhw, align_corners, fmt, scales, out, workspace)
 
 
 def upsample_trilinear3d_backward(grad_out, out_dhw, input_size, align_corners=False, fmt="NCDHW",
                                   scales=(0.0, 0.0, 0.0), out=None, workspace=None):
     """input_size is (N, C, D, H, W) in either format, as in the reference."""
-    if out is None:
-        n, c, d, h, w = input_size
-        shape = (n, d, h, w, c) if fmt == "NDHWC" else (n, c, d, h, w)
-        out = torch.empty(shape, dtype=grad_out.dtype, device=grad_out.device)
-    tg, ty = acl_tensor(grad_out, fmt), acl_tensor(out, fmt)
-    osz, isz = int_array(list(out_dhw)), int_array(list(input_size))
-    two_phase("aclnnUpsampleTrilinear3dBackward", [tg.ptr, osz.ptr, isz.ptr, bool(align_corners), float(scales[0]),
-                                                   float(scales[1]), float(scales[2]), ty.ptr], grad_out.device,
-              workspace)
-    return out
+    return native().upsample_trilinear3d_backward(grad_out, out_dhw, input_size, align_corners, fmt, scales, out,
+                                                  workspace)
 
 
 def upsample_bilinear2d_aa(x, out_hw, align_corners=False, scales=(0.0, 0.0), out=None, workspace=None):
-    out = torch.empty(_out_shape(x, out_hw, "NCHW"), dtype=x.dtype, device=x.device) if out is None else out
-    tx, ty, size = acl_tensor(x, "NCHW"), acl_tensor(out, "NCHW"), int_array(out_hw)
-    two_phase("aclnnUpsampleBilinear2dAA", [tx.ptr, size.ptr, bool(align_corners), float(scales[0]), float(scales[1]),
-                                            ty.ptr], x.device, workspace)
-    return out
+    return native().upsample_bilinear2d_aa(x, out_hw, align_corners, "NCHW", scales, out, workspace)
 
 
 def upsample_bilinear2d_aa_backward(grad_out, out_hw, input_size, align_corners=False, scales=(0.0, 0.0), out=None,
                                     workspace=None):
-    out = torch.empty(tuple(input_size), dtype=grad_out.dtype, device=grad_out.device) if out is None else out
-    tg, ty = acl_tensor(grad_out, "NCHW"), acl_tensor(out, "NCHW")
-    osz, isz = int_array(out_hw), int_array(input_size)
-    two_phase("aclnnUpsampleBilinear2dAABackward", [tg.ptr, osz.ptr, isz.ptr, bool(align_corners), float(scales[0]),
-                                                    float(scales[1]), ty.ptr], grad_out.device, workspace)
-    return out
+    return native().upsample_bilinear2d_aa_backward(grad_out, out_hw, input_size, align_corners, "NCHW", scales, out,
+                                                    workspace)
 
 
 def upsample_bicubic2d(x, out_hw, align_corners=False, fmt="NCHW", scales=(0.0, 0.0), out=None, workspace=None):
-    out = torch.empty(_out_shape(x, out_hw, fmt), dtype=x.dtype, device=x.device) if out is None else out
-    tx, ty, size = acl_tensor(x, fmt), acl_tensor(out, fmt), int_array(out_hw)
-    two_phase("aclnnUpsampleBicubic2d", [tx.ptr, size.ptr, bool(align_corners), float(scales[0]), float(scales[1]),
-                                         ty.ptr], x.device, workspace)
-    return out
+    return native().upsample_bicubic2d(x, out_hw, align_corners, fmt, scales, out, workspace)
 
 
 def upsample_bicubic2d_backward(grad_out, out_hw, input_size, align_corners=False, fmt="NCHW", scales=(0.0, 0.0),
                                 out=None, workspace=None):
-    out = torch.empty(tuple(input_size), dtype=grad_out.dtype, device=grad_out.device) if out is None else out
-    tg, ty = acl_tensor(grad_out, fmt), acl_tensor(out, fmt)
-    osz, isz = int_array(out_hw), int_array(input_size)
-    two_phase("aclnnUpsampleBicubic2dBackward", [tg.ptr, osz.ptr, isz.ptr, bool(align_corners), float(scales[0]),
-                                                 float(scales[1]), ty.ptr], grad_out.device, workspace)
-    return out
+    return native().upsample_bicubic2d_backward(grad_out, out_hw, input_size, align_corners, fmt, scales, out, workspace)
 
 
 def resize(x, scales, mode="bilinear", fmt="NCHW", out=None, workspace=None):
@@ -372,42 +298,20 @@ def resize(x, scales, mode="bilinear", fmt="NCHW", out=None, workspace=None):
 
 
 def grid_sampler2d(x, grid, interpolation=0, padding=0, align_corners=False, out=None, workspace=None):
-    if out is None:
-        out = torch.empty((x.shape[0], x.shape[1], grid.shape[1], grid.shape[2]), dtype=x.dtype, device=x.device)
-    tx, tg, ty = acl_tensor(x, "NCHW"), acl_tensor(grid, "ND"), acl_tensor(out, "NCHW")
-    two_phase("aclnnGridSampler2D", [tx.ptr, tg.ptr, int(interpolation), int(padding), bool(align_corners), ty.ptr],
-              x.device, workspace)
-    return out
+    return native().grid_sampler(x, grid, interpolation, padding, align_corners, None, out, workspace)
 
 
 def grid_sampler2d_backward(grad_out, x, grid, interpolation=0, padding=0, align_corners=False, mask=(True, True),
                             input_grad=None, grid_grad=None, workspace=None):
-    input_grad = torch.empty_like(x) if input_grad is None else input_grad
-    grid_grad = torch.empty_like(grid) if grid_grad is None else grid_grad
-    tgo, tx, tg = acl_tensor(grad_out, "NCHW"), acl_tensor(x, "NCHW"), acl_tensor(grid, "ND")
-    tgi, tgg, m = acl_tensor(input_grad, "NCHW"), acl_tensor(grid_grad, "ND"), bool_array(list(mask))
-    two_phase("aclnnGridSampler2DBackward", [tgo.ptr, tx.ptr, tg.ptr, int(interpolation), int(padding),
-                                             bool(align_corners), m.ptr, tgi.ptr, tgg.ptr], x.device, workspace)
-    return input_grad, grid_grad
+    return native().grid_sampler_backward(grad_out, x, grid, interpolation, padding, align_corners, mask, None,
+                                          input_grad, grid_grad, workspace)
 
 
 def grid_sampler3d(x, grid, interpolation=0, padding=0, align_corners=False, fmt="NCDHW", out=None, workspace=None):
-    if out is None:
-        n, do, ho, wo = grid.shape[0], grid.shape[1], grid.shape[2], grid.shape[3]
-        shape = (n, do, ho, wo, x.shape[4]) if fmt == "NDHWC" else (n, x.shape[1], do, ho, wo)
-        out = torch.empty(shape, dtype=x.dtype, device=x.device)
-    tx, tg, ty = acl_tensor(x, fmt), acl_tensor(grid, "ND"), acl_tensor(out, fmt)
-    two_phase("aclnnGridSampler3D", [tx.ptr, tg.ptr, int(interpolation), int(padding), bool(align_corners), ty.ptr],
-              x.device, workspace)
-    return out
+    return native().grid_sampler(x, grid, interpolation, padding, align_corners, fmt, out, workspace)
 
 
 def grid_sampler3d_backward(grad_out, x, grid, interpolation=0, padding=0, align_corners=False, mask=(True, True),
                             fmt="NCDHW", input_grad=None, grid_grad=None, workspace=None):
-    input_grad = torch.empty_like(x) if input_grad is None else input_grad
-    grid_grad = torch.empty_like(grid) if grid_grad is None else grid_grad
-    tgo, tx, tg = acl_tensor(grad_out, fmt), acl_tensor(x, fmt), acl_tensor(grid, "ND")
-    tgi, tgg, m = acl_tensor(input_grad, fmt), acl_tensor(grid_grad, "ND"), bool_array(list(mask))
-    two_phase("aclnnGridSampler3DBackward", [tgo.ptr, tx.ptr, tg.ptr, int(interpolation), int(padding),
-                                             bool(align_corners), m.ptr, tgi.ptr, tgg.ptr], x.device, workspace)
-    return input_grad, grid_grad
+    return native().grid_sampler_backward(grad_out, x, grid, interpolation, padding, align_corners, mask, fmt,
+                                          input_grad, grid_grad, workspace)

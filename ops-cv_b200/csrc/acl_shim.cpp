@@ -327,14 +327,16 @@ aclTensor* aclCreateTensor(const int64_t* viewDims, uint64_t viewDimsNum, aclDat
     if (stride != nullptr) {
         t->strides.assign(stride, stride + viewDimsNum);
     } else {
-        t->strides.assign(viewDimsNum, 1);
+        t->strides = t->dims;
+        if (viewDimsNum > 0) {
+            t->strides[viewDimsNum - 1] = 1;
+        }
         for (int64_t i = static_cast<int64_t>(viewDimsNum) - 2; i >= 0; --i) {
             t->strides[i] = t->strides[i + 1] * t->dims[i + 1];
         }
     }
-    if (storageDims != nullptr) {
-        t->storageDims.assign(storageDims, storageDims + storageDimsNum);
-    }
+    (void)storageDims; // a view needs only its own extents, strides and offset here
+    (void)storageDimsNum;
     t->offset = offset;
     t->dtype = dataType;
     t->format = format;

@@ -111,7 +111,6 @@ bool PermutedDense(const aclTensor* t, aclTensor& alt)
         alt.strides = {c * h * w, h * w, w, 1};
         alt.format = ACL_FORMAT_NCHW;
     }
-    alt.storageDims = alt.dims;
     return true;
 }
 

@@ -2,18 +2,53 @@
 // reporting, the executor (a frozen list of launch steps), workspace planning and strided-view staging.
 #pragma once
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdint>
 #include <functional>
+#include <initializer_list>
 #include <vector>
 
 #include "../../include/aclnn_resample.h"
 #include "kernels.h"
 
+namespace opscv {
+
+// The extents or strides of a view: at most eight, held in place (a call builds several of these).
+class Extents {
+public:
+    static constexpr size_t kMost = 8;
+    size_t size() const { return n_; }
+    int64_t operator[](size_t i) const { return v_[i]; }
+    int64_t& operator[](size_t i) { return v_[i]; }
+    const int64_t* begin() const { return v_; }
+    const int64_t* end() const { return v_ + n_; }
+    template <typename It>
+    void assign(It first, It last) // at most kMost values
+    {
+        n_ = 0;
+        for (; first != last && n_ < kMost; ++first) {
+            v_[n_++] = *first;
+        }
+    }
+    Extents& operator=(std::initializer_list<int64_t> l)
+    {
+        assign(l.begin(), l.end());
+        return *this;
+    }
+    bool operator==(const Extents& o) const { return n_ == o.n_ && std::equal(begin(), end(), o.begin()); }
+    bool operator!=(const Extents& o) const { return !(*this == o); }
+
+private:
+    int64_t v_[kMost] = {};
+    size_t n_ = 0;
+};
+
+} // namespace opscv
+
 struct aclTensor {
-    std::vector<int64_t> dims;
-    std::vector<int64_t> strides;
-    std::vector<int64_t> storageDims;
+    opscv::Extents dims;
+    opscv::Extents strides;
     int64_t offset = 0;
     aclDataType dtype = ACL_FLOAT;
     aclFormat format = ACL_FORMAT_ND;
