@@ -1345,23 +1345,21 @@ static aclnnStatus PlanAAForward(const char* api, int filter, const aclTensor* x
     const Dt dt = ToDt(x->dtype);
     const AxisGeom gh{sh.hin, sh.hout, ah.scale}, gw{sh.win, sh.wout, aw.scale};
     const AAOffsets oh = AllocAA(ws, sh.hout, ah.taps), ow = AllocAA(ws, sh.wout, aw.taps);
-    const AAFwdPlan plan = MakeAAFwdPlan(dt, sh, ah.scale, aw.taps);
+    const AAFwdPlan plan = MakeAAFwdPlan(dt, sh, ah.scale, aw.taps, filter);
     const RangeOffsets rh = AllocRange(ws, sh.hin), rw = AllocRange(ws, sh.win);
     const uint64_t wrowOff = ws.Alloc(plan.wrowBytes);
     ex->steps.push_back([=](char* w, cudaStream_t s) {
         const AAAxis th = AAAt(w, oh, ah.taps), tw = AAAt(w, ow, aw.taps);
         const RangeAxis qh = RangeAt(w, rh), qw = RangeAt(w, rw);
-        cudaError_t e = BuildAATables(gh, gw, ah.inv, aw.inv, ah.support, aw.support, th, tw, false, filter, s);
+        float* rec = reinterpret_cast<float*>(w + wrowOff);
+        const cudaError_t e =
+            plan.stream ? BuildAATablesAndRanges(gh, gw, ah.inv, aw.inv, ah.support, aw.support, th, tw, false, filter, qh,
+                                                 qw, rec, nullptr, s)
+                        : BuildAATables(gh, gw, ah.inv, aw.inv, ah.support, aw.support, th, tw, false, filter, s);
         if (e != cudaSuccess) {
             return e;
         }
-        if (plan.stream) {
-            e = BuildAABwdRanges(gh, gw, th, tw, qh, qw, s);
-            if (e != cudaSuccess) {
-                return e;
-            }
-        }
-        return BicubicAAFwd(dt, xin.At(w), y.At(w), sh, th, tw, qh, reinterpret_cast<float*>(w + wrowOff), plan, s);
+        return BicubicAAFwd(dt, xin.At(w), y.At(w), sh, th, tw, rec, plan, s);
     });
     FinishOutput(out, y, ex);
     ex->workspaceSize = ws.Size();
@@ -1492,21 +1490,20 @@ static aclnnStatus PlanAABackward(const char* api, int filter, const aclTensor* 
         });
     } else {
         const RangeOffsets rh = AllocRange(ws, sh.hin), rw = AllocRange(ws, sh.win);
-        const AABwdPlan plan = MakeAABwdPlan(dt, sh, ah.scale, aw.scale);
+        const AABwdPlan plan = MakeAABwdPlan(dt, sh, ah.scale, aw.scale, filter);
         const uint64_t wrowH = ws.Alloc(plan.wrowBytesH), wrowW = ws.Alloc(plan.wrowBytesW);
         ex->steps.push_back([=](char* w, cudaStream_t s) {
             const AAAxis th = AAAt(w, oh, ah.taps), tw = AAAt(w, ow, aw.taps);
             const RangeAxis qh = RangeAt(w, rh), qw = RangeAt(w, rw);
-            cudaError_t e = BuildAATables(gh, gw, ah.inv, aw.inv, ah.support, aw.support, th, tw, bwdCentre, filter, s);
+            float* recH = reinterpret_cast<float*>(w + wrowH);
+            float* recW = reinterpret_cast<float*>(w + wrowW);
+            const cudaError_t e =
+                BuildAATablesAndRanges(gh, gw, ah.inv, aw.inv, ah.support, aw.support, th, tw, bwdCentre, filter, qh, qw,
+                                       plan.band ? recH : nullptr, plan.band ? recW : nullptr, s);
             if (e != cudaSuccess) {
                 return e;
             }
-            e = BuildAABwdRanges(gh, gw, th, tw, qh, qw, s);
-            if (e != cudaSuccess) {
-                return e;
-            }
-            return BicubicAABwdGather(dt, g.At(w), y.At(w), sh, th, tw, qh, qw, reinterpret_cast<float*>(w + wrowH),
-                                      reinterpret_cast<float*>(w + wrowW), plan, s);
+            return BicubicAABwdGather(dt, g.At(w), y.At(w), sh, th, tw, qh, qw, recH, recW, plan, s);
         });
     }
     FinishOutput(out, y, ex);

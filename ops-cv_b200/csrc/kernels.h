@@ -62,9 +62,13 @@ cudaError_t BuildLerpBwdRanges(AxisGeom h, AxisGeom w, LerpAxis th, LerpAxis tw,
 // filter: 0 Keys cubic (UpsampleBicubic2dAA), 1 triangle (UpsampleBilinear2dAA).
 cudaError_t BuildAATables(AxisGeom h, AxisGeom w, float invH, float invW, float supH, float supW, AAAxis th,
                           AAAxis tw, bool backward, int filter, cudaStream_t s);
-// For every forward-input index y: [start, end) = output indices whose window covers y.
-cudaError_t BuildAABwdRanges(AxisGeom h, AxisGeom w, AAAxis th, AAAxis tw, RangeAxis rh, RangeAxis rw,
-                             cudaStream_t s);
+// The same tables, and for every forward-input index y: [start, end) = output indices whose window covers y, and (rec not
+// null, only for a scale >= 1) a record of the weights of the outputs of that run (at most five, see the kernels).
+constexpr int kAASlots = 6;
+constexpr int kAASlotStride = 8; // floats per record: the weights, start and run length as integer bit patterns
+cudaError_t BuildAATablesAndRanges(AxisGeom h, AxisGeom w, float invH, float invW, float supH, float supW, AAAxis th,
+                                   AAAxis tw, bool backward, int filter, RangeAxis rh, RangeAxis rw, float* recH,
+                                   float* recW, cudaStream_t s);
 
 // ---- resampling kernels ----------------------------------------------------------------------------------
 struct Shape4 {
@@ -162,15 +166,16 @@ struct AAFwdPlan {
     bool stream;        // streaming down-scale kernel (else one thread per output element)
     bool regWeights;    // horizontal weights of all output columns fit in shared memory
     int32_t metaRows;   // most input rows a band touches (sizes the shared slot-weight records)
-    int32_t cols;       // input columns per thread of the streaming kernel (4 or 8)
+    int32_t slots;      // output rows whose windows may cover one input row (5 cubic, 3 triangle)
+    int32_t cols;       // input columns per thread of the bulk-copy variant (4 or 8)
     int32_t ringGroups; // > 0: rows arrive by bulk asynchronous copies into a shared ring of this many 4-row groups
     int32_t threads;    // block size of the streaming kernel
     int32_t bandRows;   // output rows per block
     uint64_t wrowBytes; // workspace for the per-input-row vertical weights
 };
-AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW);
-// rh (ranges of outputs covering each input row) and wrow are only used by the streaming kernel.
-cudaError_t BicubicAAFwd(Dt dt, const void* x, void* y, Shape4 sh, AAAxis th, AAAxis tw, RangeAxis rh, float* wrow,
+AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW, int filter);
+// wrow (records of the input rows) is only used by the streaming kernel.
+cudaError_t BicubicAAFwd(Dt dt, const void* x, void* y, Shape4 sh, AAAxis th, AAAxis tw, const float* wrow,
                          const AAFwdPlan& plan, cudaStream_t s);
 // Bounded waits on asynchronous copies that ran out since the library was loaded (0 in a healthy run).
 uint32_t AsyncCopyTimeouts();
@@ -180,11 +185,13 @@ struct AABwdPlan {
     int32_t threads;   // block size
     int32_t bandRows;  // grad_input rows per block
     int32_t stageRows; // grads rows staged in shared memory per block
+    int32_t colSlots;  // grads columns that may reach four adjacent grad_input columns (6 or 8)
     uint64_t wrowBytesH, wrowBytesW; // workspace for the per-row / per-column slot weights
 };
-AABwdPlan MakeAABwdPlan(Dt dt, Shape4 sh, float scaleH, float scaleW);
+AABwdPlan MakeAABwdPlan(Dt dt, Shape4 sh, float scaleH, float scaleW, int filter);
 cudaError_t BicubicAABwdGather(Dt dt, const void* go, void* gi, Shape4 sh, AAAxis th, AAAxis tw, RangeAxis rh,
-                               RangeAxis rw, float* wrowH, float* wrowW, const AABwdPlan& plan, cudaStream_t s);
+                               RangeAxis rw, const float* wrowH, const float* wrowW, const AABwdPlan& plan,
+                               cudaStream_t s);
 cudaError_t BicubicAABwdAtomic(Dt dt, const void* go, void* gi, float* acc, Shape4 sh, AAAxis th, AAAxis tw,
                                cudaStream_t s);
 

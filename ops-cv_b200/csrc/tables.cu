@@ -6,6 +6,9 @@
 // intrinsics from common.cuh, so the integer tables (source indices, window bounds) and the fp32 weights can be
 // checked bit for bit against a CPU statement of the same formulas.
 #include <algorithm>
+
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "lerp_entry.cuh"
@@ -214,18 +217,9 @@ __device__ __forceinline__ float FilterAA(int filter, float m)
 
 // upsample_bicubic2d_aa_simt_base.h:70-124 and upsample_bilinear2d_aa_simt_base.h:52-88: window
 // [xmin, xmin+xsize), weights normalised by their sum. filter: 0 Keys cubic, 1 triangle.
-__global__ void AATableKernel(AxisGeom gh, AxisGeom gw, float invH, float invW, float supH, float supW, AAAxis th,
-                              AAAxis tw, int backward, int filter)
+__device__ __forceinline__ void AATableEntry(const AxisGeom& g, const AAAxis& t, float inv, float support, int backward,
+                                             int filter, int32_t i)
 {
-    const bool isH = blockIdx.y == 0;
-    const AxisGeom g = isH ? gh : gw;
-    const AAAxis t = isH ? th : tw;
-    const float inv = isH ? invH : invW;
-    const float support = isH ? supH : supW;
-    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= g.out) {
-        return;
-    }
     // The backward kernel places the centre at 0.5 when the scale is 0 (align_corners with a single output,
     // upsample_bicubic2d_aa_grad_simt_base.h:38); the forward kernel does not (simt_base.h:72-73).
     float center = Mul(g.scale, Add(static_cast<float>(i), 0.5f));
@@ -246,35 +240,36 @@ __global__ void AATableKernel(AxisGeom gh, AxisGeom gw, float invH, float invW, 
     t.xmin[i] = static_cast<int32_t>(lo);
     t.xsize[i] = static_cast<int32_t>(size);
     float total = 0.0f;
+    float* w = t.w + static_cast<int64_t>(i) * t.taps;
     for (int32_t j = 0; j < size; ++j) {
         const float dist = Mul(Add(Sub(static_cast<float>(lo + j), center), 0.5f), inv);
-        total = Add(total, FilterAA(filter, dist));
-    }
-    float* w = t.w + static_cast<int64_t>(i) * t.taps;
-    for (int32_t j = 0; j < t.taps; ++j) {
-        float wj = 0.0f;
-        if (j < size) {
-            const float dist = Mul(Add(Sub(static_cast<float>(lo + j), center), 0.5f), inv);
-            wj = FilterAA(filter, dist);
-            if (total != 0.0f) {
-                wj = Div(wj, total);
-            }
-        }
+        const float wj = FilterAA(filter, dist);
         w[j] = wj;
+        total = Add(total, wj);
+    }
+    for (int32_t j = 0; j < t.taps; ++j) {
+        if (j >= size) {
+            w[j] = 0.0f;
+        } else if (total != 0.0f) {
+            w[j] = Div(w[j], total);
+        }
+    }
+}
+
+__global__ void AATableKernel(AxisGeom gh, AxisGeom gw, float invH, float invW, float supH, float supW, AAAxis th,
+                              AAAxis tw, int backward, int filter)
+{
+    const bool isH = blockIdx.y == 0;
+    const AxisGeom g = isH ? gh : gw;
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < g.out) {
+        AATableEntry(g, isH ? th : tw, isH ? invH : invW, isH ? supH : supW, backward, filter, i);
     }
 }
 
 // Output indices whose window covers forward-input index y. xmin and xmin+xsize are non-decreasing in i.
-__global__ void AABwdRangeKernel(AxisGeom gh, AxisGeom gw, AAAxis th, AAAxis tw, RangeAxis rh, RangeAxis rw)
+__device__ __forceinline__ void AARangeEntry(const AxisGeom& g, const AAAxis& t, int32_t y, int32_t& start, int32_t& end)
 {
-    const bool isH = blockIdx.y == 0;
-    const AxisGeom g = isH ? gh : gw;
-    const AAAxis t = isH ? th : tw;
-    const RangeAxis r = isH ? rh : rw;
-    const int32_t y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= g.in) {
-        return;
-    }
     int32_t a = 0, b = g.out;
     while (a < b) { // first i with xmin[i] + xsize[i] > y
         const int32_t m = a + ((b - a) >> 1);
@@ -294,8 +289,60 @@ __global__ void AABwdRangeKernel(AxisGeom gh, AxisGeom gw, AAAxis th, AAAxis tw,
             a = m + 1;
         }
     }
-    r.start[y] = first;
-    r.end[y] = a > first ? a : first;
+    start = first;
+    end = a > first ? a : first;
+}
+
+// Tables, ranges and slot records of both axes in one launch: one cluster per axis, whose blocks meet at the cluster
+// barrier between the entries per output index and the entries per input index that are searched from them (the
+// barrier orders the global writes before the reads of the other blocks). As three or four dependent launches this
+// preparation took 12 to 18 us of a call, most of it launch latency; in one launch 5 to 10 us.
+// Record of input index y (kAASlotStride floats): weight at y of output start + a for a < kAASlots (0 past the run),
+// then start and the run length as integer bit patterns.
+constexpr int kAAClusterBlocks = 8;
+constexpr int kAAClusterThreads = 256;
+
+__global__ void __cluster_dims__(kAAClusterBlocks, 1, 1) __launch_bounds__(kAAClusterThreads)
+    AATablesAndRangesKernel(AxisGeom gh, AxisGeom gw, float invH, float invW, float supH, float supW, AAAxis th, AAAxis tw,
+                            int backward, int filter, RangeAxis rh, RangeAxis rw, float* __restrict__ recH,
+                            float* __restrict__ recW)
+{
+    const bool isH = blockIdx.y == 0;
+    const AxisGeom g = isH ? gh : gw;
+    const AAAxis t = isH ? th : tw;
+    // consecutive indices go to different blocks: a short axis keeps all eight SMs busy
+    const int32_t first = threadIdx.x * kAAClusterBlocks + blockIdx.x, step = kAAClusterBlocks * kAAClusterThreads;
+    for (int32_t i = first; i < g.out; i += step) {
+        AATableEntry(g, t, isH ? invH : invW, isH ? supH : supW, backward, filter, i);
+    }
+    cooperative_groups::this_cluster().sync();
+    const RangeAxis r = isH ? rh : rw;
+    float* rec = isH ? recH : recW;
+    for (int32_t y = first; y < g.in; y += step) {
+        int32_t s, e;
+        AARangeEntry(g, t, y, s, e);
+        r.start[y] = s;
+        r.end[y] = e;
+        if (rec == nullptr) {
+            continue;
+        }
+        float slot[kAASlotStride];
+#pragma unroll
+        for (int a = 0; a < kAASlots; ++a) {
+            slot[a] = 0.0f;
+            if (s + a < e) {
+                const int32_t k = y - t.xmin[s + a];
+                if (k >= 0 && k < t.xsize[s + a]) {
+                    slot[a] = t.w[static_cast<int64_t>(s + a) * t.taps + k];
+                }
+            }
+        }
+        slot[kAASlots] = __int_as_float(s);
+        slot[kAASlots + 1] = __int_as_float(min(e - s, kAASlots));
+        float4* out = reinterpret_cast<float4*>(rec + static_cast<int64_t>(y) * kAASlotStride);
+        out[0] = make_float4(slot[0], slot[1], slot[2], slot[3]);
+        out[1] = make_float4(slot[4], slot[5], slot[6], slot[7]);
+    }
 }
 
 } // namespace
@@ -349,10 +396,12 @@ cudaError_t BuildAATables(AxisGeom h, AxisGeom w, float invH, float invW, float 
     return cudaGetLastError();
 }
 
-cudaError_t BuildAABwdRanges(AxisGeom h, AxisGeom w, AAAxis th, AAAxis tw, RangeAxis rh, RangeAxis rw,
-                             cudaStream_t s)
+cudaError_t BuildAATablesAndRanges(AxisGeom h, AxisGeom w, float invH, float invW, float supH, float supW, AAAxis th,
+                                   AAAxis tw, bool backward, int filter, RangeAxis rh, RangeAxis rw, float* recH,
+                                   float* recW, cudaStream_t s)
 {
-    AABwdRangeKernel<<<TableGrid(h.in, w.in), kTableThreads, 0, s>>>(h, w, th, tw, rh, rw);
+    AATablesAndRangesKernel<<<dim3(kAAClusterBlocks, 2), kAAClusterThreads, 0, s>>>(
+        h, w, invH, invW, supH, supW, th, tw, backward ? 1 : 0, filter, rh, rw, recH, recW);
     CountLaunch();
     return cudaGetLastError();
 }

@@ -63,39 +63,15 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // ---- forward, streaming (down-scaling) -----------------------------------------------------------------------
-// Per input row r, the outputs whose vertical window covers r form a short run [start(r), end(r)): for scale >= 1 an
-// output covers r iff |centre - (r + 0.5)| < support + 0.5, a span of 4*scale + 1 input pixels that holds at most
-// 4 + 1/scale + 1 <= 6 = kSlots centres. AARowWeightKernel tabulates, once per call, the weight of output
-// start(r) + a at row r for a < kSlots (0 past the run), followed by start(r) and the run length as integer bit
-// patterns: one 32-byte record per input row.
-constexpr int kSlots = 6;
-constexpr int kSlotStride = 8;
+// Per input row r, the outputs whose vertical window covers r form a short run: an output covers r iff its centre lies in
+// [r + 0.5 - support, r + 0.5 + support). Centres are `scale` apart and support is 2 * scale (cubic) or scale (triangle),
+// so for scale >= 1 that is 4 or 2 outputs, one more through rounding: NS = 5 or 3 open sums. The table launch writes, once
+// per call, one 32-byte record per input row (AATablesAndRangesKernel): the weights of the run, its start and its length.
+constexpr int kSlots = kAASlots;
+constexpr int kSlotStride = kAASlotStride;
 constexpr int kFlushBatch = 4;        // output rows per horizontal pass of the streaming forward kernel
-constexpr int kStreamMaxThreads = 256; // up to 255 registers per thread for the accumulator ring and the row queue
-
-__global__ void AARowWeightKernel(AAAxis th, RangeAxis rh, int32_t hin, float* __restrict__ wrow)
-{
-    const int32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= hin) {
-        return;
-    }
-    const int32_t s = __ldg(rh.start + r), e = __ldg(rh.end + r);
-#pragma unroll
-    for (int a = 0; a < kSlots; ++a) {
-        const int32_t i = s + a;
-        float w = 0.0f;
-        if (i < e) {
-            const int32_t t = r - __ldg(th.xmin + i);
-            if (t >= 0 && t < __ldg(th.xsize + i)) {
-                w = __ldg(th.w + static_cast<int64_t>(i) * th.taps + t);
-            }
-        }
-        wrow[static_cast<int64_t>(r) * kSlotStride + a] = w;
-    }
-    // the run itself rides along in the two spare floats of the row, so that one 32-byte read gives everything
-    wrow[static_cast<int64_t>(r) * kSlotStride + 6] = __int_as_float(s);
-    wrow[static_cast<int64_t>(r) * kSlotStride + 7] = __int_as_float(min(e - s, kSlots));
-}
+constexpr int kStreamThreads = 512;   // most threads of a block of the register-prefetch variant (64 registers each)
+constexpr int kRingThreads = 256;     // the bulk-copy variant: up to 255 registers per thread
 
 // ---- bulk asynchronous copies (global -> shared) with mbarrier completion ----------------------------------------
 // Used by the streaming forward kernel to keep whole input rows in flight without holding them in registers.
@@ -146,26 +122,32 @@ __device__ __forceinline__ bool BarrierWait(uint64_t* bar, uint32_t parity, uint
 __host__ __device__ __forceinline__ int32_t Skew(int32_t col) { return col + (col >> 5); }
 __host__ __device__ __forceinline__ int32_t ParkedRowFloats(int32_t win) { return (Skew(win) + 4) & ~3; }
 
-// grid = (planes, bands); a band is `bandRows` output rows. A thread owns VC input columns of every row (one or two
-// 16-byte groups) and keeps one partial sum per open output row (kSlots of them) for each.
-// Shared memory: the vertically filtered row being flushed, the slot-weight rows of the band's input rows, and
-// (wTaps > 0) the horizontal weights of all output columns, transposed.
+// grid = (planes, bands); a band is `bandRows` output rows. A thread owns VC input columns of every row, in groups of
+// LV adjacent ones, and keeps one partial sum per open output row (NS of them) for each. LV is the widest load that every
+// row of the plane is aligned for (rows of an odd width start at every element offset: LV = 1); the groups of a thread
+// are a block width apart, so a load instruction of a warp reads one contiguous run at any LV.
+// What bounds it is instruction issue and the latency of the row loads (photographs, fp32: 96 instructions per warp and
+// row before sums were kept in packed pairs, with 56 % of the issue slots busy). 16x3x720x1280 fp16 -> 333x592, whole
+// call: 112 -> 87 us with four columns per thread (three blocks per SM) instead of eight and a band per model.
+// Shared memory: the vertically filtered row being flushed, the records of the band's input rows with every weight twice
+// (the operand of a packed multiply-add needs no register moves), and (wTaps > 0) the horizontal weights of all output
+// columns, transposed.
 // Two ways of bringing the input rows in:
 //   BULK = false: every thread loads its own columns, PF rows ahead, into registers;
 //   BULK = true : thread 0 starts one bulk asynchronous copy per row into a ring of ringGroups * PF row slots in
 //                 shared memory (completion on one mbarrier per slot); the rows of a group of PF are consumed by all
 //                 threads from shared memory, and after a block barrier the group's slots are refilled with the rows
 //                 ringGroups groups ahead. Whole rows are in flight at no register cost.
-template <typename T, int VC, int MAXT, bool BULK>
-__global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
+template <typename T, int NS, int VC, int LV, int MAXT, bool BULK>
+__global__ void __launch_bounds__(MAXT, BULK ? 1 : 2)
     AAFwdStreamKernel(const T* __restrict__ x, T* __restrict__ y, int32_t hin, int32_t win, int32_t hout,
                       int32_t wout, AAAxis th, AAAxis tw, const float* __restrict__ wrow, int32_t bandRows,
                       int32_t metaRows, int32_t wTaps, int32_t ringGroups)
 {
-    // input rows in flight per thread / rows per ring group (two keep the 4-column variant within 64 registers without spills)
-    constexpr int PF = (VC == 4 && !BULK) ? 2 : 4;
-    constexpr int LV = 16 / sizeof(T);     // elements per 16-byte load
-    constexpr int NL = VC / LV;            // 16-byte loads per row
+    // input rows in flight per thread / rows per ring group: what 64 registers hold without spills beside the sums
+    constexpr int PF = (BULK || (NS == 3 && LV * sizeof(T) >= 4 && LV > 1) || (sizeof(T) == 2 && LV == 4)) ? 4 : 2;
+    constexpr int NL = VC / LV;            // loads per row
+    constexpr int RW = (NS + 1) / 2;       // 16-byte words per shared record: NS weights twice, start, run length
     extern __shared__ __align__(16) float smemAll[];
     // BULK: the ring comes first (16-byte aligned slots of one row each), then the slot barriers
     const uint32_t rowBytes = static_cast<uint32_t>(win) * sizeof(T);
@@ -175,20 +157,29 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
     float* smemF = reinterpret_cast<float*>(bars + ((ringSlots + 1) & ~1));
     const int32_t winPad = ParkedRowFloats(win);
     float* rowbufs = smemF;                                           // [kFlushBatch][winPad]
-    float4* msm = reinterpret_cast<float4*>(smemF + kFlushBatch * winPad); // [metaRows][2]
-    float* wsm = reinterpret_cast<float*>(msm + 2 * metaRows);        // [wTaps][wout]
+    ulonglong2* msm = reinterpret_cast<ulonglong2*>(smemF + kFlushBatch * winPad); // [metaRows][RW]
+    float* wsm = reinterpret_cast<float*>(msm + RW * metaRows);       // [wTaps][wout]
     const int64_t p = blockIdx.x;
     const int32_t i0 = blockIdx.y * bandRows, i1 = min(hout, i0 + bandRows);
-    const int32_t rlo = __ldg(th.xmin + i0);
-    const int32_t rhi = min(__ldg(th.xmin + i1 - 1) + __ldg(th.xsize + i1 - 1), rlo + metaRows);
-    // Column ownership: 16-byte load l of a thread covers columns l * (blockDim.x * LV) + threadIdx.x * LV ..,
-    // so every load instruction of a warp reads one contiguous 512-byte run.
+    // a window of a user scale may start past the input: it is empty, and a band of such windows reads no rows
+    const int32_t rlo = min(__ldg(th.xmin + i0), hin);
+    const int32_t rhi = min(min(__ldg(th.xmin + i1 - 1) + __ldg(th.xsize + i1 - 1), rlo + metaRows), hin);
+    // Column ownership: load l of a thread covers columns l * (blockDim.x * LV) + threadIdx.x * LV ..
     const int32_t groupSpan = blockDim.x * LV;
     const int32_t c = threadIdx.x * LV;
     T* yp = y + p * hout * static_cast<int64_t>(wout);
 
-    for (int32_t e = threadIdx.x; e < 2 * (rhi - rlo); e += blockDim.x) {
-        msm[e] = __ldg(reinterpret_cast<const float4*>(wrow) + static_cast<int64_t>(rlo) * 2 + e);
+    for (int32_t e = threadIdx.x; e < rhi - rlo; e += blockDim.x) {
+        const float* src = wrow + static_cast<int64_t>(rlo + e) * kSlotStride;
+        float* dst = reinterpret_cast<float*>(msm + e * RW);
+#pragma unroll
+        for (int a = 0; a < NS; ++a) {
+            const float w = __ldg(src + a);
+            dst[2 * a] = w;
+            dst[2 * a + 1] = w;
+        }
+        dst[2 * NS] = __ldg(src + kSlots);
+        dst[2 * NS + 1] = __ldg(src + kSlots + 1);
     }
     for (int32_t j = threadIdx.x; j < wout && wTaps > 0; j += blockDim.x) {
         const int32_t n = min(__ldg(tw.xsize + j), wTaps);
@@ -198,12 +189,12 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
     }
     __syncthreads();
 
-    float acc[kSlots][VC];
+    F2 acc[NS][VC / 2];
 #pragma unroll
-    for (int a = 0; a < kSlots; ++a) {
+    for (int a = 0; a < NS; ++a) {
 #pragma unroll
-        for (int k = 0; k < VC; ++k) {
-            acc[a][k] = 0.0f;
+        for (int k = 0; k < VC / 2; ++k) {
+            acc[a][k] = MakeF2(0.0f, 0.0f);
         }
     }
     // Completed output rows (vertical results, taken from the oldest accumulator slot) are parked in shared memory,
@@ -259,15 +250,20 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
             batchRow0 = i;
         }
         float* rowbuf = rowbufs + pending * winPad;
+        float done[VC];
 #pragma unroll
-        for (int k = 0; k < VC; k += 4) {
-            const int32_t col = (k / LV) * groupSpan + c + k % LV;
-            if (col < win) { // four scalar stores: under the skew they are conflict-free across the warp
-                const int32_t sc = Skew(col); // col is a multiple of 4: its four columns share one skew
-                rowbuf[sc] = acc[0][k];
-                rowbuf[sc + 1] = acc[0][k + 1];
-                rowbuf[sc + 2] = acc[0][k + 2];
-                rowbuf[sc + 3] = acc[0][k + 3];
+        for (int k = 0; k < VC / 2; ++k) {
+            SplitF2(acc[0][k], done[2 * k], done[2 * k + 1]);
+        }
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+            const int32_t col = l * groupSpan + c;
+            if (col < win) { // scalar stores: under the skew they are conflict-free across the warp
+                const int32_t sc = Skew(col); // col is a multiple of LV: its LV <= 8 columns share one skew
+#pragma unroll
+                for (int k = 0; k < LV; ++k) {
+                    rowbuf[sc + k] = done[l * LV + k];
+                }
             }
         }
         if (++pending == kFlushBatch) {
@@ -276,15 +272,15 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
     };
     auto shift = [&]() {
 #pragma unroll
-        for (int a = 0; a + 1 < kSlots; ++a) {
+        for (int a = 0; a + 1 < NS; ++a) {
 #pragma unroll
-            for (int k = 0; k < VC; ++k) {
+            for (int k = 0; k < VC / 2; ++k) {
                 acc[a][k] = acc[a + 1][k];
             }
         }
 #pragma unroll
-        for (int k = 0; k < VC; ++k) {
-            acc[kSlots - 1][k] = 0.0f;
+        for (int k = 0; k < VC / 2; ++k) {
+            acc[NS - 1][k] = MakeF2(0.0f, 0.0f);
         }
     };
     // Input rows are fetched PF rows ahead into fixed registers (the row loop is unrolled by PF; rotating a queue
@@ -337,7 +333,7 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
             fetch(q[f]);
         }
     }
-    int32_t curStart = __float_as_int(msm[1].z);
+    int32_t curStart = rlo < rhi ? static_cast<int32_t>(msm[RW - 1].y & 0xffffffffu) : i0;
     for (int32_t r0 = rlo; r0 < rhi; r0 += PF) {
         const int32_t grp = (r0 - rlo) / PF;
         const int32_t slot0 = BULK ? (grp % ringGroups) * PF : 0;
@@ -371,8 +367,9 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
         for (int f = 0; f < PF; ++f) {
             const int32_t r = r0 + f;
             if (r < rhi) {
-                const float4 m0 = msm[2 * (r - rlo)], m1 = msm[2 * (r - rlo) + 1];
-                const int32_t s = __float_as_int(m1.z), cnt = __float_as_int(m1.w);
+                const ulonglong2* m = msm + (r - rlo) * RW;
+                const ulonglong2 mLast = m[RW - 1];
+                const int32_t s = static_cast<int32_t>(mLast.y & 0xffffffffu), cnt = static_cast<int32_t>(mLast.y >> 32);
                 while (curStart < s) { // outputs before start(r) no longer receive rows: complete
                     if (curStart >= i0 && curStart < i1) {
                         flush(curStart);
@@ -380,7 +377,6 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
                     shift();
                     ++curStart;
                 }
-                const float w[kSlots] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y};
                 float xv[VC];
                 if (BULK) {
                     const T* srow = reinterpret_cast<const T*>(ring + static_cast<size_t>(slot0 + f) * rowBytes);
@@ -409,11 +405,12 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
                     }
                 }
 #pragma unroll
-                for (int a = 0; a < kSlots; ++a) {
+                for (int a = 0; a < NS; ++a) {
+                    const F2 w = a == NS - 1 ? F2{mLast.x} : (a % 2 == 0 ? F2{m[a / 2].x} : F2{m[a / 2].y});
                     if (a < cnt) { // slots past the run are not touched (an Inf / NaN input must not leak in)
 #pragma unroll
-                        for (int k = 0; k < VC; ++k) {
-                            acc[a][k] = fmaf(w[a], xv[k], acc[a][k]);
+                        for (int k = 0; k < VC / 2; ++k) {
+                            acc[a][k] = Fma2(w, MakeF2(xv[2 * k], xv[2 * k + 1]), acc[a][k]);
                         }
                     }
                 }
@@ -429,8 +426,7 @@ __global__ void __launch_bounds__(MAXT, (VC == 4 && !BULK) ? 4 : (BULK ? 1 : 2))
             }
         }
     }
-    const int32_t lastEnd = __float_as_int(msm[2 * (rhi - 1 - rlo) + 1].z) + __float_as_int(msm[2 * (rhi - 1 - rlo) + 1].w);
-    while (curStart < i1 && curStart < lastEnd) {
+    while (curStart < i1) { // sums that no further row reaches, and the zeros of empty windows
         if (curStart >= i0) {
             flush(curStart);
         }
@@ -488,33 +484,77 @@ __global__ void __launch_bounds__(kThreads)
 // gi[y][x] = sum_i wH(i,y) * sum_j wW(j,x) * go[i][j]. For scale >= 1 only a few outputs cover any input row or
 // column, so the sum is done separably per block: the grads rows feeding a band of grad_input rows are staged in
 // shared memory (fp32); for kBwdRows grad_input rows at a time the block first reduces vertically
-// (t[y][j] = sum_i wH * go[i][j], one thread per (row, grads column)), then every thread expands horizontally for
-// its four grad_input columns with the column weights it keeps in registers, and stores 16 bytes per row.
-// Vertical and horizontal weights come from the slot tables built by AARowWeightKernel for both axes.
-constexpr int kBwdRows = 4;   // grad_input rows per synchronisation
-constexpr int kBwdColSlots = 8; // grads columns covering four consecutive grad_input columns (<= kSlots + 2)
+// (t[y][j] = sum_i wH * go[i][j]: a thread takes one grads column for the rows of the step, reads each grads row that
+// reaches any of them once and adds it to two packed pairs of sums, the four weights of a grads row being one 16-byte
+// word of a table that the block builds first), then every thread expands horizontally for its four grad_input columns
+// with the column weights it keeps in registers as packed pairs. Weights come from the slot records of both axes; a
+// weight that does not exist is 0 and its product changes nothing while the grads are finite.
+// What bounds it is instruction issue: 125 instructions per warp and row (photographs, fp32) while every row walked its
+// own grads rows and sums were single, 68 % of the issue slots busy. 64x3x1024x1024 <-> 224x224 fp32, both directions: 529 -> 487 us.
+constexpr int kBwdRows = 4;     // grad_input rows per synchronisation
+constexpr int kBwdRowSlots = 8; // grads rows that reach four consecutive grad_input rows (4 + ceil(3 / scale) + 1)
+constexpr int kBwdGroupBytes = (kBwdRowSlots + 1) * 16; // weights of a step, its first grads row and their count
 
-template <typename T>
+// Rows parked by the VEC = false variant: [kBwdRows][OutPitch] of T.
+__host__ __device__ __forceinline__ int32_t OutPitch(int32_t win) { return (win + 7) & ~7; }
+// Staged grads rows, the step's vertical sums and the zeros behind them that the last columns' slots may read.
+__host__ __device__ __forceinline__ int64_t BwdStagedFloats(int32_t stageRows, int32_t wout)
+{
+    return ((static_cast<int64_t>(stageRows) + kBwdRows) * wout + kBwdRowSlots + 3) & ~3LL;
+}
+
+// VEC: every row of grad_input is aligned for the four-column store of a thread. Otherwise (odd widths, an odd base) the
+// rows of a step are parked in shared memory and written from there, adjacent lanes to adjacent words: four scalar
+// stores per thread would touch every sector of the row four times.
+// CS: grads columns that may reach a thread's four columns.
+template <typename T, bool VEC, int CS>
 __global__ void __launch_bounds__(1024)
     AABwdBandKernel(const T* __restrict__ go, T* __restrict__ gi, int32_t hin, int32_t win, int32_t hout,
                     int32_t wout, RangeAxis rh, RangeAxis rw, const float* __restrict__ wrowH,
                     const float* __restrict__ wrowW, int32_t bandRows, int32_t stageRows)
 {
     extern __shared__ __align__(16) float smemF[];
-    float4* msm = reinterpret_cast<float4*>(smemF);            // [bandRows][2] vertical slot records of the band's rows
-    float* gos = smemF + static_cast<int64_t>(bandRows) * 8;   // [stageRows][wout] grads rows of the band
-    float* tbuf = gos + static_cast<int64_t>(stageRows) * wout; // [kBwdRows][wout]
+    const int32_t groups = bandRows / kBwdRows;
+    float4* gw = reinterpret_cast<float4*>(smemF);                   // [groups][kBwdRowSlots] weights of the step's rows
+    int4* gmeta = reinterpret_cast<int4*>(gw + groups * kBwdRowSlots); // [groups] first grads row (relative), count
+    float* gos = reinterpret_cast<float*>(gmeta + groups);           // [stageRows][wout] grads rows of the band
+    float* tbuf = gos + static_cast<int64_t>(stageRows) * wout;      // [kBwdRows][wout], then zeros
+    T* obuf = reinterpret_cast<T*>(gos + BwdStagedFloats(stageRows, wout));
     const int64_t p = blockIdx.x;
     const int32_t y0 = blockIdx.y * bandRows, y1 = min(hin, y0 + bandRows);
-    for (int32_t e = threadIdx.x; e < 2 * (y1 - y0); e += blockDim.x) {
-        msm[e] = __ldg(reinterpret_cast<const float4*>(wrowH) + static_cast<int64_t>(y0) * 2 + e);
-    }
     const int32_t i0 = __ldg(rh.start + y0);
     const int32_t i1 = min(max(i0, __ldg(rh.end + y1 - 1)), i0 + stageRows);
+    for (int32_t e = threadIdx.x; e < groups * kBwdRowSlots; e += blockDim.x) {
+        const int32_t grp = e / kBwdRowSlots, u = e - grp * kBwdRowSlots;
+        const int32_t yb = y0 + grp * kBwdRows;
+        if (yb >= y1) {
+            break;
+        }
+        const int32_t first = __ldg(rh.start + yb), last = min(yb + kBwdRows, y1) - 1;
+        float w[kBwdRows];
+#pragma unroll
+        for (int ry = 0; ry < kBwdRows; ++ry) {
+            w[ry] = 0.0f;
+            if (yb + ry < y1) {
+                const float* rec = wrowH + static_cast<int64_t>(yb + ry) * kSlotStride;
+                const int32_t a = first + u - __float_as_int(__ldg(rec + kSlots));
+                if (a >= 0 && a < __float_as_int(__ldg(rec + kSlots + 1))) {
+                    w[ry] = __ldg(rec + a);
+                }
+            }
+        }
+        gw[e] = make_float4(w[0], w[1], w[2], w[3]);
+        if (u == 0) {
+            gmeta[grp] = make_int4(first - i0, max(0, min(min(__ldg(rh.end + last), i1) - first, kBwdRowSlots)), 0, 0);
+        }
+    }
+    for (int32_t e = threadIdx.x; e < kBwdRowSlots; e += blockDim.x) {
+        tbuf[kBwdRows * wout + e] = 0.0f;
+    }
     const T* gp = go + (p * hout + i0) * static_cast<int64_t>(wout);
-    // While staging, note whether the band's grads rows hold an Inf / NaN: then the horizontal step takes a path that
-    // only touches the sources covering each column, so that a non-finite value reaches exactly the columns it
-    // reaches in the reference (the fast path multiplies uncovered sources by 0).
+    // While staging, note whether the band's grads rows hold an Inf / NaN: then both steps take a path that only touches
+    // the sources with a weight of their own (the gather kernel skips zero weights), so that a non-finite value reaches
+    // exactly the elements it reaches in the reference.
     bool sawNonFinite = false;
     for (int32_t e = threadIdx.x; e < (i1 - i0) * wout; e += blockDim.x) {
         const float v = DType<T>::Load(gp + e);
@@ -525,47 +565,69 @@ __global__ void __launch_bounds__(1024)
     const int32_t x = threadIdx.x * 4;
     const bool hasCols = x < win;
     int32_t j0 = 0;
-    float wreg[4][kBwdColSlots];
+    F2 wreg[CS][2];
     if (hasCols) {
         j0 = __ldg(rw.start + x);
+        float w[4][CS];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int32_t sk = __ldg(rw.start + x + k), ek = __ldg(rw.end + x + k);
+            const bool in = VEC || x + k < win;
+            const int32_t sk = in ? __ldg(rw.start + x + k) : 0, ek = in ? __ldg(rw.end + x + k) : 0;
 #pragma unroll
-            for (int u = 0; u < kBwdColSlots; ++u) {
+            for (int u = 0; u < CS; ++u) {
                 const int32_t a = j0 + u - sk; // slot of grads column j0 + u in column x + k's own table
-                wreg[k][u] = (a >= 0 && a < kSlots && j0 + u < ek)
-                                 ? __ldg(wrowW + static_cast<int64_t>(x + k) * kSlotStride + a)
-                                 : 0.0f;
+                w[k][u] = (a >= 0 && a < kSlots && j0 + u < ek)
+                              ? __ldg(wrowW + static_cast<int64_t>(x + k) * kSlotStride + a)
+                              : 0.0f;
             }
         }
+#pragma unroll
+        for (int u = 0; u < CS; ++u) {
+            wreg[u][0] = MakeF2(w[0][u], w[1][u]);
+            wreg[u][1] = MakeF2(w[2][u], w[3][u]);
+        }
+        j0 = min(j0, wout); // a user scale can leave columns without any source
     }
-    const int32_t jcnt = hasCols ? min(kBwdColSlots, __ldg(rw.end + x + 3) - j0) : 0;
-    const bool masked = __syncthreads_or(sawNonFinite) != 0; // also: the staged rows and records are visible
+    const bool masked = __syncthreads_or(sawNonFinite) != 0; // also: the staged rows and tables are visible
     T* op = gi + p * hin * static_cast<int64_t>(win);
     for (int32_t yb = y0; yb < y1; yb += kBwdRows) {
-        // vertical: a thread takes one grads column for the kBwdRows rows of the step; the rows' slot records
-        // (weights, first grads row, count) are block-uniform shared-memory reads
+        const int32_t grp = (yb - y0) / kBwdRows;
+        const int4 meta = gmeta[grp];
+        const ulonglong2* wg = reinterpret_cast<const ulonglong2*>(gw + grp * kBwdRowSlots);
         for (int32_t j = threadIdx.x; j < wout; j += blockDim.x) {
+            F2 v01 = MakeF2(0.0f, 0.0f), v23 = v01;
+            const float* gcol = gos + meta.x * wout + j;
+#pragma unroll
+            for (int u = 0; u < kBwdRowSlots; ++u) {
+                if (u >= meta.y) { // the same for every thread of the block
+                    break;
+                }
+                const float g = gcol[u * wout];
+                const ulonglong2 w = wg[u];
+                if (!masked) {
+                    const F2 gg = MakeF2(g, g);
+                    v01 = Fma2(F2{w.x}, gg, v01);
+                    v23 = Fma2(F2{w.y}, gg, v23);
+                } else {
+                    float ws[4], vs[4];
+                    SplitF2(F2{w.x}, ws[0], ws[1]);
+                    SplitF2(F2{w.y}, ws[2], ws[3]);
+                    SplitF2(v01, vs[0], vs[1]);
+                    SplitF2(v23, vs[2], vs[3]);
+#pragma unroll
+                    for (int ry = 0; ry < kBwdRows; ++ry) {
+                        vs[ry] = ws[ry] != 0.0f ? fmaf(ws[ry], g, vs[ry]) : vs[ry];
+                    }
+                    v01 = MakeF2(vs[0], vs[1]);
+                    v23 = MakeF2(vs[2], vs[3]);
+                }
+            }
+            float v[kBwdRows];
+            SplitF2(v01, v[0], v[1]);
+            SplitF2(v23, v[2], v[3]);
 #pragma unroll
             for (int ry = 0; ry < kBwdRows; ++ry) {
-                const int32_t y = yb + ry;
-                float v = 0.0f;
-                if (y < y1) {
-                    const float4 m0 = msm[2 * (y - y0)], m1 = msm[2 * (y - y0) + 1];
-                    const int32_t s = __float_as_int(m1.z), cnt = __float_as_int(m1.w);
-                    const float w[kSlots] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y};
-                    const float* gcol = gos + (s - i0) * wout + j;
-                    const int32_t run = min(cnt, i1 - s); // slots past the run (or past the staged rows) are not read
-#pragma unroll
-                    for (int a = 0; a < kSlots; ++a) {
-                        if (a >= run) { // the same for every thread of the block
-                            break;
-                        }
-                        v = fmaf(w[a], gcol[a * wout], v);
-                    }
-                }
-                tbuf[ry * wout + j] = v;
+                tbuf[ry * wout + j] = v[ry];
             }
         }
         __syncthreads();
@@ -575,37 +637,60 @@ __global__ void __launch_bounds__(1024)
 #pragma unroll
             for (int ry = 0; ry < kBwdRows; ++ry) {
                 if (yb + ry < y1) {
-                    float out[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    F2 o01 = MakeF2(0.0f, 0.0f), o23 = o01;
+                    float out[4];
                     if (!masked) {
 #pragma unroll
-                        for (int u = 0; u < kBwdColSlots; ++u) {
-                            if (u < jcnt) { // slots past the run are not read
-                                const float t = tr[u];
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    out[k] = fmaf(wreg[k][u], t, out[k]);
-                                }
-                            }
+                        for (int u = 0; u < CS; ++u) {
+                            const F2 tt = MakeF2(tr[u], tr[u]);
+                            o01 = Fma2(wreg[u][0], tt, o01);
+                            o23 = Fma2(wreg[u][1], tt, o23);
                         }
-                    } else { // same sums, but a source is only multiplied into the columns it covers
+                        SplitF2(o01, out[0], out[1]);
+                        SplitF2(o23, out[2], out[3]);
+                    } else {
+                        out[0] = out[1] = out[2] = out[3] = 0.0f;
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int32_t sk = __ldg(rw.start + x + k), ek = __ldg(rw.end + x + k);
+                        for (int u = 0; u < CS; ++u) {
+                            float w[4];
+                            SplitF2(wreg[u][0], w[0], w[1]);
+                            SplitF2(wreg[u][1], w[2], w[3]);
 #pragma unroll
-                            for (int u = 0; u < kBwdColSlots; ++u) {
-                                if (u < jcnt && j0 + u >= sk && j0 + u < ek) {
-                                    out[k] = fmaf(wreg[k][u], tr[u], out[k]);
-                                }
+                            for (int k = 0; k < 4; ++k) {
+                                out[k] = w[k] != 0.0f ? fmaf(w[k], tr[u], out[k]) : out[k];
                             }
                         }
                     }
-                    StorePack<T, 4>(dst, out);
+                    StorePack<T, 4>(VEC ? dst : obuf + ry * OutPitch(win) + x, out);
                 }
                 dst += win;
                 tr += wout;
             }
         }
         __syncthreads();
+        if (!VEC) { // the next writes to obuf come after the barrier behind the next vertical step
+            const int32_t rows = min(kBwdRows, y1 - yb);
+            for (int32_t ry = 0; ry < rows; ++ry) {
+                const T* src = obuf + ry * OutPitch(win);
+                T* row = op + static_cast<int64_t>(yb + ry) * win;
+                if constexpr (sizeof(T) == 2) {
+                    const int32_t lead = static_cast<int32_t>(reinterpret_cast<uintptr_t>(row) >> 1) & 1; // elements before a word
+                    for (int32_t e = 2 * static_cast<int32_t>(threadIdx.x) - lead; e < win; e += 2 * blockDim.x) {
+                        if (e >= 0 && e + 1 < win) {
+                            const Pack<T, 2> w{{src[e], src[e + 1]}};
+                            *reinterpret_cast<Pack<T, 2>*>(row + e) = w;
+                        } else {
+                            const int32_t one = e < 0 ? 0 : e;
+                            row[one] = src[one];
+                        }
+                    }
+                } else {
+                    for (int32_t e = threadIdx.x; e < win; e += blockDim.x) {
+                        row[e] = src[e];
+                    }
+                }
+            }
+        }
     }
 }
 
@@ -646,43 +731,48 @@ __global__ void __launch_bounds__(kThreads)
 
 } // namespace
 
-AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW)
+AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW, int filter)
 {
     AAFwdPlan plan{};
-    // Streaming needs: every input row covered by at most kSlots outputs (true for scale >= 1), rows that one
-    // block can own (8 columns per thread) and 16-byte aligned rows.
+    // Streaming needs every input row covered by at most NS outputs (true for scale >= 1) and rows that one block can own
+    // (four columns per thread). Wider rows and up-scales take a thread per output element.
     const int es = DtSize(dt);
-    plan.stream = scaleH >= 1.0f && sh.win % 8 == 0 && sh.win <= 8 * kStreamMaxThreads && (sh.win * es) % 16 == 0;
+    plan.stream = scaleH >= 1.0f && sh.win <= 4 * kStreamThreads;
     if (!plan.stream) {
         return plan;
     }
-    // fp32 rows of up to 1024 columns: four columns per thread (twice the warps of the 8-column variant at the same
-    // number of resident blocks measured ~8 % faster); 16-bit rows and longer rows: eight columns (one or two
-    // 16-byte loads per thread and row).
-    plan.cols = (es == 4 && sh.win <= 4 * kStreamMaxThreads) ? 4 : 8;
-    const int32_t threads = std::max(64, static_cast<int32_t>((CeilDiv(sh.win, plan.cols) + 31) & ~31));
-    plan.threads = std::min(kStreamMaxThreads, threads);
-    // Bands: pick the number of bands per plane whose block count fills whole waves of resident blocks best
-    // (every band re-reads the input rows of its first window, so no more than 8, and at least 16 rows each).
+    plan.slots = filter == 0 ? 5 : 3;
+    plan.threads = std::max(64, static_cast<int32_t>((CeilDiv(sh.win, 4) + 31) & ~31));
+    const size_t recBytes = static_cast<size_t>(plan.slots + 1) * 8;
+    const size_t rowBufs = kFlushBatch * static_cast<size_t>(ParkedRowFloats(sh.win)) * sizeof(float);
+    const size_t wBytes = static_cast<size_t>(tapsW) * sh.wout * sizeof(float);
+    auto metaRows = [&](int64_t bandRows) { // a band's windows span bandRows * scale + 2 * support (+ rounding) rows
+        return static_cast<int32_t>(std::min<double>(
+            sh.hin, std::ceil(static_cast<double>(bandRows) * scaleH + 4.0 * scaleH + 4.0)));
+    };
+    // Bands per plane: least time by a model of the walk. A block alone takes a load latency per step (about 0.3 us a
+    // row with the rows in flight that its registers hold); the blocks of an SM share its issue slots (about 50
+    // instructions per warp and row). Every band re-reads the rows of its first window and pays a fixed start.
     const int64_t planes = std::max<int64_t>(sh.n * sh.c, 1);
-    const int64_t resident = static_cast<int64_t>(NumSMs()) * (plan.cols == 4 ? 4 : std::max(1, 512 / plan.threads));
-    int64_t bestBands = 1;
-    double bestEff = 0.0;
-    for (int64_t b = 1; b <= 8 && sh.hout / b >= 16; ++b) {
-        const int64_t blocks = planes * b;
-        const double eff = static_cast<double>(blocks) / (static_cast<double>(CeilDiv(blocks, resident)) * resident);
-        if (eff > bestEff + 0.02) {
-            bestEff = eff;
-            bestBands = b;
+    const double warps = plan.threads / 32;
+    double bestTime = 0.0;
+    for (int64_t b = 1; b == 1 || (b <= 256 && sh.hout / b >= 4); ++b) {
+        const int64_t band = CeilDiv(sh.hout, b);
+        const size_t smem = rowBufs + static_cast<size_t>(metaRows(band)) * recBytes + 64 + (wBytes <= 48 * 1024 ? wBytes : 0);
+        const int64_t perSm = std::max<int64_t>(
+            1, std::min<int64_t>(1024 / plan.threads, static_cast<int64_t>((225 * 1024) / (smem + 1024))));
+        const int64_t blocks = planes * CeilDiv(sh.hout, band);
+        const double k = static_cast<double>(CeilDiv(blocks, NumSMs()));
+        const double rows = static_cast<double>(metaRows(band)) + 10.0;
+        const double time = rows * std::max(0.3 * std::ceil(k / static_cast<double>(perSm)), 0.0065 * k * warps);
+        if (b == 1 || time < bestTime * 0.98) {
+            bestTime = time;
+            plan.bandRows = static_cast<int32_t>(band);
         }
     }
-    plan.bandRows = static_cast<int32_t>(CeilDiv(sh.hout, bestBands));
-    // input rows of a band: its windows span bandRows * scale + 2 * support (+ rounding) rows
-    plan.metaRows = static_cast<int32_t>(
-        std::min<double>(sh.hin, std::ceil(static_cast<double>(plan.bandRows) * scaleH + 4.0 * scaleH + 4.0)));
-    // horizontal weights in shared memory if they fit beside the row buffer and the slot records
-    const size_t wBytes = static_cast<size_t>(tapsW) * sh.wout * sizeof(float);
-    const size_t rest = (kFlushBatch * static_cast<size_t>(ParkedRowFloats(sh.win)) + static_cast<size_t>(plan.metaRows) * 8 + 8) * sizeof(float);
+    plan.metaRows = metaRows(plan.bandRows);
+    // horizontal weights in shared memory if they fit beside the row buffer and the records
+    const size_t rest = rowBufs + static_cast<size_t>(plan.metaRows) * recBytes + 32;
     plan.regWeights = wBytes + rest <= 96 * 1024;
     if (rest > 96 * 1024) {
         plan.stream = false;
@@ -694,10 +784,13 @@ AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW)
     plan.ringGroups = 0;
     if (const char* o = getenv("OPSCV_AA_RING")) {
         const int groups = atoi(o);
+        const int32_t cols = (es == 4 && sh.win <= 4 * kRingThreads) ? 4 : 8;
         const size_t ring = static_cast<size_t>(groups) * 4 * sh.win * es + 64;
         const size_t used = rest + (plan.regWeights ? wBytes : 0);
-        if (groups >= 2 && groups <= 4 && used + ring <= 200 * 1024) {
+        if (groups >= 2 && groups <= 4 && used + ring <= 200 * 1024 && sh.win % 8 == 0 && sh.win <= 8 * kRingThreads) {
             plan.ringGroups = groups;
+            plan.cols = cols;
+            plan.threads = std::max(64, static_cast<int32_t>((CeilDiv(sh.win, cols) + 31) & ~31));
         }
     }
     return plan;
@@ -712,16 +805,17 @@ uint32_t AsyncCopyTimeouts()
     return v;
 }
 
-cudaError_t BicubicAAFwd(Dt dt, const void* x, void* y, Shape4 sh, AAAxis th, AAAxis tw, RangeAxis rh,
-                         float* wrow, const AAFwdPlan& plan, cudaStream_t s)
+cudaError_t BicubicAAFwd(Dt dt, const void* x, void* y, Shape4 sh, AAAxis th, AAAxis tw, const float* wrow,
+                         const AAFwdPlan& plan, cudaStream_t s)
 {
     const int64_t planes = sh.n * sh.c;
-    const bool stream = plan.stream && Aligned(x, 16) && planes < (1LL << 31) && CeilDiv(sh.hout, plan.bandRows) <= 65535;
+    const bool stream = plan.stream && (plan.ringGroups == 0 || Aligned(x, 16)) && planes < (1LL << 31) &&
+                        CeilDiv(sh.hout, plan.bandRows) <= 65535;
     if (stream) {
-        AARowWeightKernel<<<static_cast<unsigned>(CeilDiv(sh.hin, 128)), 128, 0, s>>>(th, rh, sh.hin, wrow);
         const dim3 grid(static_cast<unsigned>(planes), static_cast<unsigned>(CeilDiv(sh.hout, plan.bandRows)));
         const int32_t wTaps = plan.regWeights ? tw.taps : 0;
-        const size_t base = (kFlushBatch * static_cast<size_t>(ParkedRowFloats(sh.win)) + static_cast<size_t>(plan.metaRows) * 8 +
+        const size_t base = (kFlushBatch * static_cast<size_t>(ParkedRowFloats(sh.win)) +
+                             static_cast<size_t>(plan.metaRows) * 2 * (plan.slots + 1) +
                              static_cast<size_t>(wTaps) * sh.wout) * sizeof(float);
         cudaError_t e = cudaSuccess;
         OPSCV_DISPATCH_DT(dt, T, {
@@ -741,21 +835,33 @@ cudaError_t BicubicAAFwd(Dt dt, const void* x, void* y, Shape4 sh, AAAxis th, AA
                                                             plan.bandRows, plan.metaRows, wTaps, plan.ringGroups);
                 }
             };
-            if (plan.cols == 4) {
-                if constexpr (sizeof(T) == 4) {
-                    if (plan.ringGroups > 0) {
-                        launch(AAFwdStreamKernel<T, 4, kStreamMaxThreads, true>);
+            constexpr int kVec = 16 / sizeof(T);
+            auto pick = [&](auto slots) {
+                constexpr int NS = decltype(slots)::value;
+                if (plan.ringGroups > 0) {
+                    if (sizeof(T) == 4 && plan.cols == 4) {
+                        launch(AAFwdStreamKernel<T, NS, kVec, kVec, kRingThreads, true>);
                     } else {
-                        launch(AAFwdStreamKernel<T, 4, kStreamMaxThreads, false>);
+                        launch(AAFwdStreamKernel<T, NS, 8, kVec, kRingThreads, true>);
                     }
+                    return;
                 }
-            } else if (plan.ringGroups > 0) {
-                launch(AAFwdStreamKernel<T, 8, kStreamMaxThreads, true>);
+                const int v = std::min(4, PickVec(static_cast<int>(sizeof(T)), sh.win, {x}));
+                if (v == 4) {
+                    launch(AAFwdStreamKernel<T, NS, 4, 4, kStreamThreads, false>);
+                } else if (v == 2) {
+                    launch(AAFwdStreamKernel<T, NS, 4, 2, kStreamThreads, false>);
+                } else {
+                    launch(AAFwdStreamKernel<T, NS, 4, 1, kStreamThreads, false>);
+                }
+            };
+            if (plan.slots == 5) {
+                pick(std::integral_constant<int, 5>{});
             } else {
-                launch(AAFwdStreamKernel<T, 8, kStreamMaxThreads, false>);
+                pick(std::integral_constant<int, 3>{});
             }
         });
-        CountLaunch(2);
+        CountLaunch();
         return e != cudaSuccess ? e : cudaGetLastError();
     }
     const int64_t total = planes * sh.hout * static_cast<int64_t>(sh.wout);
@@ -768,33 +874,39 @@ cudaError_t BicubicAAFwd(Dt dt, const void* x, void* y, Shape4 sh, AAAxis th, AA
 }
 
 // Shared memory of one block of the band kernel: slot records of the band's rows, staged grads rows, step buffer.
-static size_t AABwdSmem(int32_t bandRows, int32_t stageRows, int32_t wout)
+// and, for rows that are parked before they are written, those rows.
+static size_t AABwdSmem(int32_t bandRows, int32_t stageRows, int32_t wout, int32_t win, int es, bool parked)
 {
-    return (static_cast<size_t>(bandRows) * 8 + (static_cast<size_t>(stageRows) + kBwdRows) * wout) * sizeof(float);
+    const size_t groups = static_cast<size_t>(bandRows) / kBwdRows;
+    return groups * kBwdGroupBytes + static_cast<size_t>(BwdStagedFloats(stageRows, wout)) * sizeof(float) +
+           (parked ? static_cast<size_t>(kBwdRows) * OutPitch(win) * es : 0);
 }
 
-AABwdPlan MakeAABwdPlan(Dt dt, Shape4 sh, float scaleH, float scaleW)
+AABwdPlan MakeAABwdPlan(Dt dt, Shape4 sh, float scaleH, float scaleW, int filter)
 {
     AABwdPlan plan{};
     const int es = DtSize(dt);
     // Same covering bound as the forward streaming kernel, on both axes; one block owns whole grad_input rows.
-    plan.band = scaleH >= 1.0f && scaleW >= 1.0f && sh.win % 4 == 0 && sh.win <= 4096 && (sh.win * es) % 8 == 0;
+    plan.band = scaleH >= 1.0f && scaleW >= 1.0f && sh.win <= 4096;
     if (!plan.band) {
         return plan;
     }
+    // grads columns that reach four adjacent columns: centres in a span of 2 * support + 3, one more through rounding
+    plan.colSlots = (filter == 1 || scaleW >= 3.0f) ? 6 : 8;
     plan.threads = std::min(1024, std::max(128, static_cast<int32_t>((CeilDiv(sh.win, 4) + 31) & ~31)));
     // Bands per plane: the split whose blocks fill whole waves of resident blocks best (up to four 256-thread
     // blocks per SM, fewer if the staged grads rows need more shared memory). t grad_input rows are fed by at most
     // t / scale + kSlots + 2 grads rows.
     const int64_t planes = std::max<int64_t>(sh.n * sh.c, 1);
     double bestScore = 0.0;
-    for (int32_t b = 1; b <= 64 && (b == 1 || sh.hin / b >= 4 * kBwdRows); ++b) {
+    for (int32_t b = 1; b <= 256 && (b == 1 || sh.hin / b >= 4 * kBwdRows); ++b) {
         int32_t band = static_cast<int32_t>(CeilDiv(sh.hin, b));
         band = (band + kBwdRows - 1) / kBwdRows * kBwdRows;
         const int32_t stage = static_cast<int32_t>(
             std::min<int64_t>(static_cast<int64_t>(band / static_cast<double>(scaleH)) + kSlots + 2, sh.hout));
-        const size_t smem = AABwdSmem(band, stage, sh.wout);
-        if (smem > 200 * 1024) {
+        const size_t smem = AABwdSmem(band, stage, sh.wout, sh.win, es, sh.win % 4 != 0);
+        // (an unaligned grad_input parks its rows too)
+        if (smem > 200 * 1024 || AABwdSmem(band, stage, sh.wout, sh.win, es, true) > 224 * 1024) {
             continue;
         }
         const int64_t perSm = std::min<int64_t>({4, 2048 / plan.threads, static_cast<int64_t>((225 * 1024) / (smem + 1024))});
@@ -819,28 +931,34 @@ AABwdPlan MakeAABwdPlan(Dt dt, Shape4 sh, float scaleH, float scaleW)
 }
 
 cudaError_t BicubicAABwdGather(Dt dt, const void* go, void* gi, Shape4 sh, AAAxis th, AAAxis tw, RangeAxis rh,
-                               RangeAxis rw, float* wrowH, float* wrowW, const AABwdPlan& plan, cudaStream_t s)
+                               RangeAxis rw, const float* wrowH, const float* wrowW, const AABwdPlan& plan,
+                               cudaStream_t s)
 {
     const int64_t planes = sh.n * sh.c;
-    const bool band = plan.band && Aligned(gi, 16) && planes < (1LL << 31) && CeilDiv(sh.hin, plan.bandRows) <= 65535;
+    const bool band = plan.band && planes < (1LL << 31) && CeilDiv(sh.hin, plan.bandRows) <= 65535;
     if (band) {
-        AARowWeightKernel<<<static_cast<unsigned>(CeilDiv(sh.hin, 128)), 128, 0, s>>>(th, rh, sh.hin, wrowH);
-        AARowWeightKernel<<<static_cast<unsigned>(CeilDiv(sh.win, 128)), 128, 0, s>>>(tw, rw, sh.win, wrowW);
         const dim3 grid(static_cast<unsigned>(planes), static_cast<unsigned>(CeilDiv(sh.hin, plan.bandRows)));
-        const size_t smem = AABwdSmem(plan.bandRows, plan.stageRows, sh.wout);
+        const bool vec = sh.win % 4 == 0 && Aligned(gi, 16);
+        const size_t smem = AABwdSmem(plan.bandRows, plan.stageRows, sh.wout, sh.win, DtSize(dt), !vec);
         cudaError_t e = cudaSuccess;
         OPSCV_DISPATCH_DT(dt, T, {
-            if (smem > 48 * 1024) {
-                e = cudaFuncSetAttribute(AABwdBandKernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
-            }
-            if (e == cudaSuccess) {
-                AABwdBandKernel<T><<<grid, plan.threads, smem, s>>>(static_cast<const T*>(go), static_cast<T*>(gi), sh.hin,
-                                                                   sh.win, sh.hout, sh.wout, rh, rw, wrowH, wrowW,
-                                                                   plan.bandRows, plan.stageRows);
+            auto launch = [&](auto kernel) {
+                if (smem > 48 * 1024) {
+                    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+                }
+                if (e == cudaSuccess) {
+                    kernel<<<grid, plan.threads, smem, s>>>(static_cast<const T*>(go), static_cast<T*>(gi), sh.hin, sh.win,
+                                                            sh.hout, sh.wout, rh, rw, wrowH, wrowW, plan.bandRows,
+                                                            plan.stageRows);
+                }
+            };
+            if (plan.colSlots == 6) {
+                launch(vec ? AABwdBandKernel<T, true, 6> : AABwdBandKernel<T, false, 6>);
+            } else {
+                launch(vec ? AABwdBandKernel<T, true, 8> : AABwdBandKernel<T, false, 8>);
             }
         });
-        CountLaunch(3);
+        CountLaunch();
         return e != cudaSuccess ? e : cudaGetLastError();
     }
     const int64_t total = planes * sh.hin * static_cast<int64_t>(sh.win);

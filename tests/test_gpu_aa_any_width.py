@@ -1,0 +1,86 @@
+"""Anti-aliased down-scaling at any width and alignment: the streaming forward at every load width, the band backward with
+and without parked rows, bands that hold one output row, and windows of a user scale that lie past the input.
+
+Bars: fp32 against the oracle rtol 1e-5 / atol 1e-6 (same terms, sums split by axis: at most 25 x 25 products of weights
+that sum to one, each rounding 6e-8). fp16 / bf16: half an ulp of the storage type around the oracle's fp32 value, plus the
+fp32 bar."""
+import numpy as np
+import pytest
+import torch
+
+from test_gpu_parity import DTYPES, _poison, _same_nonfinite, gen, quant
+
+pytestmark = pytest.mark.gpu
+
+# (n, c, h, w, oh, ow): widths of every remainder modulo 4, one column, two, a block's last thread partly used, the widest
+# row of one block and the first that is too wide, scales of exactly one and just above
+SHAPES = [(1, 3, 37, 61, 11, 17), (2, 1, 40, 62, 13, 40), (1, 2, 33, 63, 5, 9), (3, 1, 64, 130, 31, 129),
+          (1, 1, 9, 1, 4, 1), (1, 1, 30, 2, 7, 2), (1, 1, 20, 513, 3, 100), (1, 1, 7, 2047, 2, 341),
+          (1, 1, 6, 2049, 3, 700), (1, 1, 301, 5, 299, 4), (1, 1, 12, 4095, 4, 1365), (1, 1, 12, 4098, 4, 1365),
+          (1, 1, 23, 50, 23, 49), (1, 1, 100, 96, 99, 95)]
+HALF_ULP = {torch.float32: 0.0, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}
+
+
+def close(got, ref, dtype):
+    got = got.detach().cpu().float().numpy().astype(np.float64)
+    bar = 1e-6 + 1e-5 * np.abs(ref) + HALF_ULP[dtype] * np.abs(ref) * (1 + 1e-4)
+    if dtype == torch.float16:
+        bar = bar + 2.0 ** -25
+    assert (np.abs(got - ref) <= bar).all(), float((np.abs(got - ref) - bar).max())
+
+
+def off_by(t, dev, shift):
+    """The same values in a buffer whose first element is `shift` elements past an aligned address."""
+    flat = torch.empty(t.numel() + shift, dtype=t.dtype, device=dev)
+    view = flat[shift:].view(t.shape)
+    view.copy_(t)
+    return view
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("filt", ["bicubic", "bilinear"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_any_width(ops, oracle, dev, dtype, filt, shape):
+    n, c, h, w, oh, ow = shape
+    fwd, bwd, ofwd, obwd = {
+        "bicubic": (ops.upsample_bicubic2d_aa, ops.upsample_bicubic2d_aa_grad, oracle.bicubic_aa_fwd,
+                    oracle.bicubic_aa_bwd),
+        "bilinear": (ops.upsample_bilinear2d_aa, ops.upsample_bilinear2d_aa_backward, oracle.bilinear_aa_fwd,
+                     oracle.bilinear_aa_bwd)}[filt]
+    x, x32 = quant(torch.rand((n, c, h, w), generator=gen(90)), dtype)
+    ref = ofwd(x32, (oh, ow), False)
+    for shift in (0, 1, 2):
+        close(fwd(off_by(x, dev, shift), (oh, ow), False), ref, dtype)
+    g, g32 = quant(torch.rand((n, c, oh, ow), generator=gen(91)), dtype)
+    ref = obwd(g32, (h, w), False, definition="gather")
+    close(bwd(g.to(dev), (oh, ow), (n, c, h, w), False), ref, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_grad_input_at_any_alignment(ops, oracle, dev, dtype):
+    g, g32 = quant(torch.rand((1, 2, 9, 21), generator=gen(92)), dtype)
+    ref = oracle.bicubic_aa_bwd(g32, (30, 64), False, definition="gather")
+    for shift in (0, 1, 2, 3):
+        out = off_by(torch.full((1, 2, 30, 64), 7.0, dtype=dtype), dev, shift)
+        ops.upsample_bicubic2d_aa_grad(g.to(dev), (9, 21), (1, 2, 30, 64), False, out=out)
+        close(out, ref, dtype)
+
+
+def test_windows_past_the_input_give_zero(ops, oracle, dev):
+    x = torch.rand((1, 2, 24, 33), generator=gen(93))
+    for size in ((30, 40), (12, 15)):
+        y = ops.upsample_bicubic2d_aa(x.to(dev), size, False, scales=(0.25, 0.4))
+        close(y, oracle.bicubic_aa_fwd(x.numpy(), size, False, (0.25, 0.4)), torch.float32)
+        g = torch.rand((1, 2) + size, generator=gen(97))
+        gi = ops.upsample_bicubic2d_aa_grad(g.to(dev), size, (1, 2, 24, 33), False, scales=(0.25, 0.4))
+        close(gi, oracle.bicubic_aa_bwd(g.numpy(), (24, 33), False, (0.25, 0.4), definition="gather"), torch.float32)
+
+
+def test_non_finite_values_at_odd_widths(ops, oracle, dev):
+    rng = np.random.default_rng(94)
+    x = _poison(torch.rand((1, 2, 41, 57), generator=gen(95)), rng, 6)
+    _same_nonfinite(ops.upsample_bicubic2d_aa(x.to(dev), (13, 19), False), oracle.bicubic_aa_fwd(x.numpy(), (13, 19), False),
+                    "forward")
+    g = _poison(torch.rand((1, 2, 13, 19), generator=gen(96)), rng, 4)
+    _same_nonfinite(ops.upsample_bicubic2d_aa_grad(g.to(dev), (13, 19), (1, 2, 41, 57), False),
+                    oracle.bicubic_aa_bwd(g.numpy(), (41, 57), False, definition="gather"), "backward")
