@@ -231,6 +231,7 @@ __global__ void __launch_bounds__(kThreads) Bicubic2dFwdKernel(const T* __restri
 // The sums are the expressions of the kernel above in the same order, so the bits are the same; what changes is
 // that a tap is loaded and converted once per block instead of once per output column that uses it, and that the
 // column coefficients live in registers for all the rows of the tile.
+constexpr int kFwdWalk = 16; // output rows that a thread walks in the narrow vertical pass
 struct BicubicTile {
     int32_t bandRows; // output rows per item
     int32_t bands;
@@ -352,8 +353,57 @@ __global__ void __launch_bounds__(kThreads) Bicubic2dFwdTileKernel(const T* __re
             }
         }
         __syncthreads();
-        // vertical combination, V adjacent outputs per thread
         T* py = y + (plane * g.hout + h0) * static_cast<int64_t>(g.wout);
+        if constexpr (V <= 2) {
+            // Rows that allow no wider store than two elements: a thread walks kFwdWalk output rows down its columns with
+            // the four sums in registers. An up-scale moves the window on by at most one source row per output row, so
+            // most rows load one sum or none; with four loads and four row offsets per output the pass was bound by
+            // instruction issue (fp32 8x64 planes 60x80 -> 150x199: 80 instructions per output, 81 % of the issue slots; 46 -> 37 us).
+            // Columns and segments of rows share one index, so that no thread is idle at any width.
+            const int32_t segs = (nOut + kFwdWalk - 1) / kFwdWalk;
+            for (int32_t i = tid; i < packs * segs; i += kThreads) {
+                const int32_t seg = i / packs, p = i - seg * packs;
+                const int32_t r1 = min(nOut, (seg + 1) * kFwdWalk);
+                const float* col = sA + p * V;
+                T* dst = py + static_cast<int64_t>(seg * kFwdWalk) * g.wout + p * V;
+                int32_t cur = INT32_MIN / 2;
+                float a[4][V];
+                auto load = [&](int32_t row, float (&v)[V]) {
+                    const float* src = col + (ClampIdx32(row, g.hin - 1) - srcLo) * g.wout;
+#pragma unroll
+                    for (int e = 0; e < V; ++e) {
+                        v[e] = src[e];
+                    }
+                };
+                for (int32_t r = seg * kFwdWalk; r < r1; ++r, dst += g.wout) {
+                    const int32_t top = sTop[r];
+                    const float4 ch = *reinterpret_cast<const float4*>(sCh + 4 * r);
+                    if (top == cur + 1) {
+#pragma unroll
+                        for (int e = 0; e < V; ++e) {
+                            a[0][e] = a[1][e];
+                            a[1][e] = a[2][e];
+                            a[2][e] = a[3][e];
+                        }
+                        load(top + 2, a[3]);
+                    } else if (top != cur) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            load(top - 1 + k, a[k]);
+                        }
+                    }
+                    cur = top;
+                    float out[V];
+#pragma unroll
+                    for (int e = 0; e < V; ++e) {
+                        out[e] = Add(Add(Add(Mul(a[0][e], ch.x), Mul(a[1][e], ch.y)), Mul(a[2][e], ch.z)), Mul(a[3][e], ch.w));
+                    }
+                    StorePack<T, V>(dst, out);
+                }
+            }
+            continue;
+        }
+        // vertical combination, V adjacent outputs per thread
         constexpr int C = V / 4 > 0 ? V / 4 : 1;
         constexpr int L = V < 4 ? V : 4;
         for (int32_t p = px_; p < packs; p += tile.pw) {
@@ -480,26 +530,33 @@ __device__ float BwdElementDirect(const T* __restrict__ pg, const BicubicGeom& g
 
 // The gather with the column side of the walk cached. A thread owns one element position of a grad_input row
 // (column yw; for NHWC also its channel) and keeps it while the block moves over rows and planes. It first walks
-// the grads columns once, exactly as the reference does, and stores every term it would add for one grads row as
-// an entry (grads column, coefficient) in its own column of a shared-memory table: one entry per grads column for
-// an interior yw, one per matching tap for a first or last yw. For each grads row h of the row walk it then has
-// one coefficient (interior yh) or the matching tap coefficients in tap order (first or last yh), and adds
-// (g * cH) * cW over the entries, grouped by grads column with the row taps outside the column taps. That is the
-// order and the rounding of the reference's four walks, so the sum has the same bits.
+// the grads columns once, exactly as the reference does, and stores every grads column that reaches it with its
+// coefficients (one for an interior yw, up to three matching taps in tap order for a first or last yw) in its own
+// column of a shared-memory table. For each grads row h of the row walk it then has one coefficient (interior yh) or
+// the matching tap coefficients in tap order (first or last yh), and adds (g * cH) * cW over the columns, for each of
+// them with the row taps outside the column taps. That is the order and the rounding of the reference's four walks,
+// so the sum has the same bits. The additions of a thread are one chain; what it must not wait for one by one are the
+// loads, so the grads values of kListBatch columns are fetched before the first of them is used (border columns of
+// fp32 8x64 planes 60x80 <- 150x199: 58 us with one load at a time, 38 us in batches).
 // colsPB: element positions of a row that a block covers (its threads beyond that take further rows);
 // borderOnly: the block's positions are those of the first and the last column only.
+constexpr int kListBatch = 8;
+constexpr int kListTaps = 3;                       // a fourth needs an extent of 1
+constexpr int kListBytes = 4 + 4 * kListTaps;      // per column and thread
+constexpr int kListThreads = 128;
+
 template <typename T, bool NHWC>
-__global__ void __launch_bounds__(kThreads) Bicubic2dBwdListKernel(const T* __restrict__ go, T* __restrict__ gi, BicubicGeom g,
-                                                                    int32_t maxW, int32_t colsPB, int32_t borderOnly)
+__device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __restrict__ gi, const BicubicGeom& g, int32_t maxW,
+                                             int32_t colsPB, bool borderOnly, float* sList, int32_t blockX, int64_t blockY,
+                                             int64_t blocksY)
 {
-    extern __shared__ float sList[];
     const int32_t nt = blockDim.x, tid = threadIdx.x;
-    float* sCoef = sList;
-    int32_t* sCol = reinterpret_cast<int32_t*>(sList + static_cast<size_t>(maxW) * nt);
+    float* sCoef = sList; // [maxW][kListTaps][nt]
+    int32_t* sCol = reinterpret_cast<int32_t*>(sList + static_cast<size_t>(maxW) * kListTaps * nt); // column << 2 | taps
     const int32_t inner = g.win * g.chan;
     const int32_t rowsPB = nt / colsPB;
     const int32_t rowLane = tid / colsPB;
-    const int32_t pos = blockIdx.x * colsPB + (tid - rowLane * colsPB);
+    const int32_t pos = blockX * colsPB + (tid - rowLane * colsPB);
     if (rowLane >= rowsPB || pos >= (borderOnly ? 2 * g.chan : inner)) {
         return;
     }
@@ -529,35 +586,38 @@ __global__ void __launch_bounds__(kThreads) Bicubic2dBwdListKernel(const T* __re
                 }
                 float cwTap[4];
                 TapCoeff(Sub(rw, static_cast<float>(fw)), cwTap);
+                int n = 0;
+                overflow = cnt >= maxW || w >= (1 << 29);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    if (ClampIdx(fw - 1 + j, g.win - 1) == yw) {
-                        if (cnt < maxW) {
-                            sCoef[cnt * nt + tid] = cwTap[j];
-                            sCol[cnt * nt + tid] = w;
-                            ++cnt;
+                    if (!overflow && ClampIdx(fw - 1 + j, g.win - 1) == yw) {
+                        if (n < kListTaps) {
+                            sCoef[(cnt * kListTaps + n) * nt + tid] = cwTap[j];
+                            ++n;
                         } else {
                             overflow = true;
                         }
                     }
                 }
+                if (n > 0 && !overflow) {
+                    sCol[cnt * nt + tid] = w << 2 | n;
+                    ++cnt;
+                }
             } else {
                 if (!(rw < Add(static_cast<float>(yw), 2.0f))) {
                     break;
                 }
-                if (cnt < maxW) {
-                    sCoef[cnt * nt + tid] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
-                    sCol[cnt * nt + tid] = w;
+                overflow = cnt >= maxW || w >= (1 << 29);
+                if (!overflow) {
+                    sCoef[cnt * kListTaps * nt + tid] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
+                    sCol[cnt * nt + tid] = w << 2 | 1;
                     ++cnt;
-                } else {
-                    overflow = true;
                 }
             }
         }
     }
 
-    for (int64_t row = static_cast<int64_t>(blockIdx.y) * rowsPB + rowLane; row < g.rows;
-         row += static_cast<int64_t>(gridDim.y) * rowsPB) {
+    for (int64_t row = blockY * rowsPB + rowLane; row < g.rows; row += blocksY * rowsPB) {
         const int64_t plane = row / g.hin;
         const int32_t yh = static_cast<int32_t>(row - plane * g.hin);
         const T* pg = go + plane * planeGo;
@@ -572,167 +632,58 @@ __global__ void __launch_bounds__(kThreads) Bicubic2dBwdListKernel(const T* __re
         float add = 0.0f;
         for (int32_t h = hStart; h < g.hout; ++h, rh = BwdSrc(g.scaleH, h, g.align)) {
             const T* prow = pg + h * rowGo + c;
+            float chv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            int nH = 1;
             if (!borderH) {
                 if (!(rh < Add(static_cast<float>(yh), 2.0f))) {
                     break;
                 }
-                const float ch = PointCoeff(fabsf(Sub(rh, static_cast<float>(yh))));
-                // one row coefficient: the entries in list order are already the reference's order
-                for (int32_t k = 0; k < cnt; ++k) {
-                    const float gv = DType<T>::Load(prow + static_cast<int64_t>(sCol[k * nt + tid]) * g.chan);
-                    add = Add(add, Mul(Mul(gv, ch), sCoef[k * nt + tid]));
-                }
-                continue;
-            }
-            const long long fh = static_cast<long long>(floorf(rh));
-            if (yh == 0 && fh > 1 && g.hin > 1) {
-                break;
-            }
-            float chTap[4];
-            TapCoeff(Sub(rh, static_cast<float>(fh)), chTap);
-            float chv[4];
-            int nH = 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (ClampIdx(fh - 1 + i, g.hin - 1) == yh) {
-                    // compacted in tap order without dynamic register indexing
-                    chv[3] = chTap[i];
-                    if (nH == 0) chv[0] = chTap[i];
-                    if (nH == 1) chv[1] = chTap[i];
-                    if (nH == 2) chv[2] = chTap[i];
-                    ++nH;
-                }
-            }
-            int32_t k = 0;
-            while (k < cnt) {
-                const int32_t w = sCol[k * nt + tid];
-                int32_t k1 = k + 1;
-                while (k1 < cnt && sCol[k1 * nt + tid] == w) {
-                    ++k1;
-                }
-                const float gv = DType<T>::Load(prow + static_cast<int64_t>(w) * g.chan);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (i < nH) {
-                        const float gc = Mul(gv, i == 3 ? chv[3] : (i == 2 ? chv[2] : (i == 1 ? chv[1] : chv[0])));
-                        for (int32_t kk = k; kk < k1; ++kk) {
-                            add = Add(add, Mul(gc, sCoef[kk * nt + tid]));
-                        }
-                    }
-                }
-                k = k1;
-            }
-        }
-        po[t] = DType<T>::FromF(add);
-    }
-}
-
-// The same gather for the interior columns (1 .. win - 2), whose walk has one coefficient per grads column and at
-// most K columns (every up-scale factor up to (K - 1) / 4, and every down-scale): the list lives in registers and
-// the loop over it is unrolled. The first and the last column go through the list kernel in a launch of their own.
-// Terms, their order and their rounding are those of the list kernel.
-template <typename T, bool NHWC, int K>
-__global__ void __launch_bounds__(kThreads) Bicubic2dBwdRegKernel(const T* __restrict__ go, T* __restrict__ gi, BicubicGeom g)
-{
-    const int32_t inner = g.win * g.chan;
-    const int32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos >= inner - 2 * g.chan) {
-        return;
-    }
-    const int32_t t = pos + g.chan; // skip column 0
-    const int32_t yw = NHWC ? t / g.chan : t;
-    const int32_t c = NHWC ? t - yw * g.chan : 0;
-    const int64_t planeGo = static_cast<int64_t>(g.hout) * g.wout * g.chan;
-    const int64_t rowGo = static_cast<int64_t>(g.wout) * g.chan;
-    const float offset = g.align ? 0.0f : 0.5f;
-
-    float cw[K];
-    int32_t cnt = 0;
-    bool overflow = false;
-    const int32_t wStart = WalkStart(yw, g.invW, offset);
-    {
-        bool done = false;
-#pragma unroll
-        for (int k = 0; k < K + 1; ++k) {
-            const int32_t w = wStart + k;
-            if (k < K) {
-                cw[k] = 0.0f;
-            }
-            if (!done && w < g.wout) {
-                const float rw = k == 0 ? Sub(Mul(Add(static_cast<float>(wStart), offset), g.scaleW), offset)
-                                        : BwdSrc(g.scaleW, w, g.align);
-                if (!(rw < Add(static_cast<float>(yw), 2.0f))) {
-                    done = true;
-                } else if (k == K) {
-                    overflow = true;
-                } else {
-                    cw[k < K ? k : 0] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
-                    cnt = k + 1;
-                }
-            }
-        }
-    }
-    const int32_t colStep = NHWC ? g.chan : 1; // a compile-time 1 for NCHW: the taps of a row are pw[0 .. K)
-
-    for (int64_t row = blockIdx.y; row < g.rows; row += gridDim.y) {
-        const int64_t plane = row / g.hin;
-        const int32_t yh = static_cast<int32_t>(row - plane * g.hin);
-        const T* pg = go + plane * planeGo;
-        T* po = gi + row * inner;
-        if (overflow) {
-            po[t] = DType<T>::FromF(BwdElementDirect<T>(pg, g, yh, yw, c, rowGo, offset));
-            continue;
-        }
-        const bool borderH = yh == 0 || yh == g.hin - 1; // uniform over the block
-        const int32_t hStart = WalkStart(yh, g.invH, offset);
-        float rh = Sub(Mul(Add(static_cast<float>(hStart), offset), g.scaleH), offset);
-        float add = 0.0f;
-        const T* pw0 = pg + c + static_cast<int64_t>(wStart) * colStep; // K * chan fits 32 bits (W * C does)
-        if (!borderH) {
-            for (int32_t h = hStart; h < g.hout; ++h, rh = BwdSrc(g.scaleH, h, g.align)) {
-                if (!(rh < Add(static_cast<float>(yh), 2.0f))) {
-                    break;
-                }
-                const float ch = PointCoeff(fabsf(Sub(rh, static_cast<float>(yh))));
-                const T* pw = pw0 + h * rowGo;
-                float gv[K];
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    gv[k] = k < cnt ? DType<T>::Load(pw + k * colStep) : 0.0f;
-                }
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    gv[k] = Mul(Mul(gv[k], ch), cw[k]); // independent of the running sum: issued ahead of it
-                }
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    if (k < cnt) {
-                        add = Add(add, gv[k]);
-                    }
-                }
-            }
-        } else {
-            for (int32_t h = hStart; h < g.hout; ++h, rh = BwdSrc(g.scaleH, h, g.align)) {
+                chv[0] = PointCoeff(fabsf(Sub(rh, static_cast<float>(yh))));
+            } else {
                 const long long fh = static_cast<long long>(floorf(rh));
                 if (yh == 0 && fh > 1 && g.hin > 1) {
                     break;
                 }
                 float chTap[4];
                 TapCoeff(Sub(rh, static_cast<float>(fh)), chTap);
-                bool hit[4];
+                nH = 0;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    hit[i] = ClampIdx(fh - 1 + i, g.hin - 1) == yh;
+                    if (ClampIdx(fh - 1 + i, g.hin - 1) == yh) {
+                        // compacted in tap order without dynamic register indexing
+                        chv[3] = chTap[i];
+                        if (nH == 0) chv[0] = chTap[i];
+                        if (nH == 1) chv[1] = chTap[i];
+                        if (nH == 2) chv[2] = chTap[i];
+                        ++nH;
+                    }
                 }
-                const T* pw = pw0 + h * rowGo;
+            }
+            for (int32_t k0 = 0; k0 < cnt; k0 += kListBatch) {
+                float gv[kListBatch];
+                int32_t taps[kListBatch];
 #pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    if (k < cnt) {
-                        const float gvk = DType<T>::Load(pw + k * colStep);
+                for (int u = 0; u < kListBatch; ++u) {
+                    gv[u] = 0.0f;
+                    taps[u] = 0;
+                    if (k0 + u < cnt) {
+                        const int32_t col = sCol[(k0 + u) * nt + tid];
+                        gv[u] = DType<T>::Load(prow + static_cast<int64_t>(col >> 2) * g.chan);
+                        taps[u] = col & 3;
+                    }
+                }
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            if (hit[i]) {
-                                add = Add(add, Mul(Mul(gvk, chTap[i]), cw[k]));
+                for (int u = 0; u < kListBatch; ++u) {
+                    if (taps[u] == 0) {
+                        break;
+                    }
+                    const float* cu = sCoef + (k0 + u) * kListTaps * nt + tid;
+                    for (int i = 0; i < nH; ++i) {
+                        const float gc = Mul(gv[u], i == 0 ? chv[0] : (i == 1 ? chv[1] : (i == 2 ? chv[2] : chv[3])));
+#pragma unroll
+                        for (int j = 0; j < kListTaps; ++j) {
+                            if (j < taps[u]) {
+                                add = Add(add, Mul(gc, cu[j * nt]));
                             }
                         }
                     }
@@ -740,6 +691,273 @@ __global__ void __launch_bounds__(kThreads) Bicubic2dBwdRegKernel(const T* __res
             }
         }
         po[t] = DType<T>::FromF(add);
+    }
+}
+
+template <typename T, bool NHWC>
+__global__ void __launch_bounds__(kListThreads) Bicubic2dBwdListKernel(const T* __restrict__ go, T* __restrict__ gi, BicubicGeom g,
+                                                                        int32_t maxW, int32_t colsPB)
+{
+    extern __shared__ __align__(16) float sList[];
+    BwdListBlock<T, NHWC>(go, gi, g, maxW, colsPB, false, sList, blockIdx.x, blockIdx.y, gridDim.y);
+}
+
+// ---- the same gather for the interior columns (1 .. win - 2): a walk down the grads rows --------------------------
+// A thread owns one element position of a grad_input row and a block a band of grad_input rows. The thread walks down
+// the grads rows that feed the band and keeps one sum open for every grad_input row whose walk includes the current
+// grads row (at most kOpen: the walk spans four source pixels, one more through rounding), so a grads value is loaded
+// and converted once per column that it feeds instead of once per term. A grad_input row takes its terms in ascending
+// grads row and, within one, ascending grads column, each (g * cH) * cW with its own roundings: the order and the bits
+// of the reference's walk. What bounds the kernel is instruction issue on those terms: two packed products per pair of
+// terms and one add per term, which cannot be packed because the terms of a sum follow one another.
+// The column side of the walk (at most K columns, one coefficient each) stays in registers; the row side is evaluated
+// once per block into shared-memory records. First and last rows take up to four taps per grads row: they ride along
+// in the blocks whose band holds them. The first and the last column are list blocks, the first blocks of the same grid,
+// so that their long chains run under the walk. fp32 8x64 planes 60x80 <- 150x199: 230 us as two launches that loaded
+// every term -> 82 us.
+constexpr int kOpen = 5;
+constexpr int kWalkThreads = 128;
+constexpr int kWalkMaxRows = 448; // grads rows that a band may read (their records stay below 48 KB)
+
+struct WalkRecord {
+    float c[kOpen];   // coefficients of the open rows, from `first` on
+    int32_t first, count;
+    int32_t edge;     // bits 0..3: taps of this grads row that land on row 0, bits 4..7: on row hin - 1
+    float tap[4];     // their coefficients
+    float pad[4];
+};
+static_assert(sizeof(WalkRecord) == 64, "records are read as 16-byte words");
+static_assert(kListThreads == kWalkThreads, "list blocks and walk blocks share a grid");
+
+// walkX: blocks of one band; the first listX * listY blocks of the grid are list blocks.
+struct WalkShape {
+    int64_t positions; // planes * interior element positions of a row
+    int32_t bandRows, maxRows, walkX, listX, listY, listCols, listMax;
+};
+
+template <typename T, bool NHWC, int K>
+__global__ void __launch_bounds__(kWalkThreads, (NHWC && K > 14) ? 3 : ((NHWC || K > 14) ? 4 : 5))
+    Bicubic2dBwdWalkKernel(const T* __restrict__ go, T* __restrict__ gi, BicubicGeom g, WalkShape ws)
+{
+    extern __shared__ __align__(16) float sWalk[];
+    const int32_t lists = ws.listX * ws.listY;
+    if (static_cast<int32_t>(blockIdx.x) < lists) {
+        BwdListBlock<T, NHWC>(go, gi, g, ws.listMax, ws.listCols, true, sWalk, static_cast<int32_t>(blockIdx.x) % ws.listX,
+                              static_cast<int32_t>(blockIdx.x) / ws.listX, ws.listY);
+        return;
+    }
+    const int32_t walkBlock = static_cast<int32_t>(blockIdx.x) - lists;
+    const int32_t band = walkBlock / ws.walkX;
+    WalkRecord* rec = reinterpret_cast<WalkRecord*>(sWalk);
+    int32_t* rowStart = reinterpret_cast<int32_t*>(rec + ws.maxRows);
+    int32_t* rowEnd = rowStart + ws.bandRows;
+    const float offset = g.align ? 0.0f : 0.5f;
+    const int32_t y0 = band * ws.bandRows, y1 = min(y0 + ws.bandRows, g.hin);
+    const int32_t yi0 = max(y0, 1), yi1 = min(y1, g.hin - 1); // interior rows of the band
+    for (int32_t r = threadIdx.x; r < y1 - y0; r += blockDim.x) {
+        const int32_t y = y0 + r;
+        const int32_t h0 = min(WalkStart(y, g.invH, offset), g.hout);
+        int32_t h = h0;
+        if (y == g.hin - 1) {
+            h = g.hout;
+        } else {
+            while (h < g.hout) {
+                const float rh = BwdSrc(g.scaleH, h, g.align);
+                if (y == 0 ? static_cast<long long>(floorf(rh)) > 1 : !(rh < Add(static_cast<float>(y), 2.0f))) {
+                    break;
+                }
+                ++h;
+            }
+        }
+        rowStart[r] = h0;
+        rowEnd[r] = h;
+    }
+    __syncthreads();
+    int32_t hLo = rowStart[0], hHi = rowEnd[0];
+    for (int32_t r = 1; r < y1 - y0; ++r) {
+        hLo = min(hLo, rowStart[r]);
+        hHi = max(hHi, rowEnd[r]);
+    }
+    hHi = min(hHi, hLo + ws.maxRows);
+    for (int32_t h = hLo + threadIdx.x; h < hHi; h += blockDim.x) {
+        const float rh = BwdSrc(g.scaleH, h, g.align);
+        WalkRecord w{};
+        int32_t y = yi0;
+        while (y < yi1 && rowEnd[y - y0] <= h) {
+            ++y;
+        }
+        w.first = y;
+#pragma unroll
+        for (int a = 0; a < kOpen; ++a) {
+            if (y + a < yi1 && rowStart[y + a - y0] <= h) {
+                w.c[a] = PointCoeff(fabsf(Sub(rh, static_cast<float>(y + a))));
+                w.count = a + 1;
+            }
+        }
+        const bool top = y0 == 0 && h >= rowStart[0] && h < rowEnd[0];
+        const bool bottom = y1 == g.hin && h >= rowStart[y1 - 1 - y0] && h < rowEnd[y1 - 1 - y0];
+        if (top || bottom) {
+            const long long fh = static_cast<long long>(floorf(rh));
+            TapCoeff(Sub(rh, static_cast<float>(fh)), w.tap);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int32_t dst = ClampIdx(fh - 1 + i, g.hin - 1);
+                w.edge |= (top && dst == 0) ? 1 << i : 0;
+                w.edge |= (bottom && dst == g.hin - 1) ? 16 << i : 0;
+            }
+        }
+        rec[h - hLo] = w;
+    }
+    __syncthreads();
+
+    const int64_t pos = static_cast<int64_t>(walkBlock - band * ws.walkX) * blockDim.x + threadIdx.x;
+    if (pos >= ws.positions) {
+        return;
+    }
+    const int32_t inner = g.win * g.chan;
+    const int32_t perPlane = inner - 2 * g.chan;
+    const int64_t plane = ws.positions <= INT32_MAX
+                              ? static_cast<int64_t>(static_cast<uint32_t>(pos) / static_cast<uint32_t>(perPlane))
+                              : pos / perPlane;
+    const int32_t t = static_cast<int32_t>(pos - plane * perPlane) + g.chan; // skip column 0
+    const int32_t yw = NHWC ? t / g.chan : t;
+    const int32_t c = NHWC ? t - yw * g.chan : 0;
+    const int64_t rowGo = static_cast<int64_t>(g.wout) * g.chan;
+    const T* pg = go + plane * g.hout * rowGo;
+    T* po = gi + plane * g.hin * static_cast<int64_t>(inner) + t;
+
+    // the column walk, once; slots past it keep the coefficient 0
+    F2 cw[K / 2];
+    int32_t cnt = 0;
+    const int32_t wStart = WalkStart(yw, g.invW, offset);
+    {
+        float cws[K];
+        bool done = false;
+#pragma unroll
+        for (int k = 0; k < K + 1; ++k) {
+            const int32_t w = wStart + k;
+            if (k < K) {
+                cws[k < K ? k : 0] = 0.0f;
+            }
+            if (!done && w < g.wout) {
+                const float rw = BwdSrc(g.scaleW, w, g.align);
+                if (!(rw < Add(static_cast<float>(yw), 2.0f))) {
+                    done = true;
+                } else if (k == K) {
+                    cnt = -1; // does not fit the registers
+                } else {
+                    cws[k < K ? k : 0] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
+                    cnt = k + 1;
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < K / 2; ++k) {
+            cw[k] = MakeF2(cws[2 * k], cws[2 * k + 1]);
+        }
+    }
+    if (cnt < 0) {
+        for (int32_t y = y0; y < y1; ++y) {
+            po[static_cast<int64_t>(y) * inner] = DType<T>::FromF(BwdElementDirect<T>(pg, g, y, yw, c, rowGo, offset));
+        }
+        return;
+    }
+    const int32_t colStep = NHWC ? g.chan : 1; // a compile-time 1 for NCHW
+    const T* pw = pg + hLo * rowGo + static_cast<int64_t>(wStart) * colStep + c;
+
+    float acc[kOpen];
+#pragma unroll
+    for (int a = 0; a < kOpen; ++a) {
+        acc[a] = 0.0f;
+    }
+    float top = 0.0f, bottom = 0.0f;
+    int32_t cur = yi0;
+    auto finish = [&]() { // the oldest open row is complete
+        po[static_cast<int64_t>(cur) * inner] = DType<T>::FromF(acc[0]);
+#pragma unroll
+        for (int a = 0; a + 1 < kOpen; ++a) {
+            acc[a] = acc[a + 1];
+        }
+        acc[kOpen - 1] = 0.0f;
+        ++cur;
+    };
+    T raw[K]; // the next grads row, in flight; slots past the walk stay 0
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        raw[k] = DType<T>::FromF(0.0f);
+        if (k < cnt && hLo < hHi) {
+            raw[k] = __ldg(pw + k * colStep);
+        }
+    }
+    for (int32_t h = hLo; h < hHi; ++h) {
+        F2 gv[K / 2];
+#pragma unroll
+        for (int k = 0; k < K / 2; ++k) {
+            gv[k] = MakeF2(DType<T>::ToF(raw[2 * k]), DType<T>::ToF(raw[2 * k + 1]));
+        }
+        pw += rowGo;
+        if (h + 1 < hHi) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                if (k < cnt) {
+                    raw[k] = __ldg(pw + k * colStep);
+                }
+            }
+        }
+        const WalkRecord& r = rec[h - hLo];
+        const float4 r0 = *reinterpret_cast<const float4*>(&r);
+        const float4 r1 = *(reinterpret_cast<const float4*>(&r) + 1);
+        const float ch[kOpen] = {r0.x, r0.y, r0.z, r0.w, r1.x};
+        const int32_t first = __float_as_int(r1.y), count = __float_as_int(r1.z), edge = __float_as_int(r1.w);
+        while (cur < first) {
+            finish();
+        }
+#pragma unroll
+        for (int a = 0; a < kOpen; ++a) {
+            if (a < count) { // the same for the whole block
+                const F2 c2 = MakeF2(ch[a], ch[a]);
+#pragma unroll
+                for (int k = 0; k < K / 2; ++k) {
+                    float p0, p1;
+                    SplitF2(Mul2(Mul2(gv[k], c2), cw[k]), p0, p1);
+                    // a slot past the walk gives a zero, which cannot change a sum that started from +0
+                    acc[a] = Add(acc[a], p0);
+                    acc[a] = Add(acc[a], p1);
+                }
+            }
+        }
+        if (edge != 0) { // first or last row: the taps of one grads value before those of the next
+#pragma unroll
+            for (int k = 0; k < K / 2; ++k) {
+                float gs[2], cs[2];
+                SplitF2(gv[k], gs[0], gs[1]);
+                SplitF2(cw[k], cs[0], cs[1]);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (2 * k + u < cnt) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float term = Mul(Mul(gs[u], r.tap[i]), cs[u]);
+                            if ((edge >> i) & 1) {
+                                top = Add(top, term);
+                            }
+                            if ((edge >> (i + 4)) & 1) {
+                                bottom = Add(bottom, term);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+    while (cur < yi1) {
+        finish();
+    }
+    if (y0 == 0) {
+        po[0] = DType<T>::FromF(top);
+    }
+    if (y1 == g.hin) {
+        po[static_cast<int64_t>(g.hin - 1) * inner] = DType<T>::FromF(bottom);
     }
 }
 
@@ -1479,33 +1697,47 @@ cudaError_t Bicubic2dBwd(Dt dt, Layout lay, const void* go, void* gi, Shape4 sh,
     const double perScale = invW > 0.0f ? static_cast<double>(invW) : 1.0;
     // columns of the longest interior walk: 4 / scale within two source pixels either side, one more for rounding
     const int64_t walk = static_cast<int64_t>(std::ceil(4.0 * perScale)) + 1;
-    const bool split = walk <= 17 && sh.win > 2; // interior columns from registers, the two border columns apart
-    // Entries of one column list: an interior column takes the grads columns of its walk, a first or last column
-    // up to three taps of each column within two and a half source pixels (at most 6 / scale + a few). Lists that
-    // would not fit make their thread fall back to the uncached walk, so the bound only has to be good, not safe;
-    // a single-column image (every grads column is a tap) always falls back.
-    int64_t maxW = static_cast<int64_t>(std::ceil(6.0 * perScale)) + 8;
+    // Interior columns by the row walk, the two border columns apart. The walk's bound on open rows holds while the
+    // start of a walk (from the inverse scale) and its end (from the scale) speak of the same positions; the last row's
+    // walk runs to the end of the grads, which a user scale can put anywhere.
+    const double rowsPerRow = invH;
+    const double drift = invH > 0.0f && scaleH > 0.0f ? std::fabs(static_cast<double>(scaleH) * invH - 1.0) *
+                                                            (static_cast<double>(sh.hin) + 2.0 * rowsPerRow + 4.0)
+                                                      : 1.0;
+    const bool split = walk <= 17 && sh.win > 2 && sh.hin > 2 && drift < 0.25 && 8.0 * rowsPerRow + 8.0 < kWalkMaxRows &&
+                       static_cast<double>(sh.hout) <= (static_cast<double>(sh.hin) + 2.0) * rowsPerRow + 2.0;
+    // Columns of one list: the grads columns of an interior walk; a first or last column takes those within two and a
+    // half source pixels. Lists that would not fit make their thread fall back to the uncached walk, so the bound only
+    // has to be good, not safe; a single-column image (every grads column is a tap) always falls back.
+    const int64_t maxW = static_cast<int64_t>(std::ceil(4.0 * perScale)) + 4;
     cudaError_t err = cudaSuccess;
-    auto launchList = [&](bool borderOnly) {
+    struct ListLaunch {
+        int32_t colsPB, entries, x, y;
+        size_t smem;
+    };
+    auto planList = [&](bool borderOnly) {
         const int64_t positions = borderOnly ? 2LL * g.chan : inner;
-        const int colsPB = static_cast<int>(std::min<int64_t>(kThreads, positions));
-        const int threads = static_cast<int>(std::min<int64_t>(kThreads, (std::max<int64_t>(colsPB, 64) + 31) / 32 * 32));
-        const int rowsPB = threads / colsPB;
-        const int64_t cap = 96 * 1024 / (8 * threads);
-        const int64_t entries = std::max<int64_t>(4, std::min<int64_t>(maxW, cap));
-        const size_t smem = static_cast<size_t>(entries) * threads * 8;
-        const int64_t gx = CeilDiv(positions, colsPB);
-        const int64_t rowBlocks = CeilDiv(g.rows, rowsPB);
-        const int64_t gyCap = std::max<int64_t>(static_cast<int64_t>(NumSMs()) * 32 / gx, 1);
-        const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(std::min<int64_t>(std::min<int64_t>(rowBlocks, gyCap), 65535)), 1);
+        ListLaunch l;
+        l.colsPB = static_cast<int32_t>(std::min<int64_t>(kListThreads, positions));
+        const int rowsPB = kListThreads / l.colsPB;
+        const int64_t cap = 96 * 1024 / (kListBytes * kListThreads);
+        l.entries = static_cast<int32_t>(std::max<int64_t>(4, std::min<int64_t>(maxW, cap)));
+        l.smem = static_cast<size_t>(l.entries) * kListThreads * kListBytes;
+        l.x = static_cast<int32_t>(CeilDiv(positions, l.colsPB));
+        const int64_t gyCap = std::max<int64_t>(static_cast<int64_t>(NumSMs()) * 32 / l.x, 1);
+        l.y = static_cast<int32_t>(std::min<int64_t>(std::min<int64_t>(CeilDiv(g.rows, rowsPB), gyCap), 65535));
+        return l;
+    };
+    auto launchList = [&]() {
+        const ListLaunch l = planList(false);
         OPSCV_DISPATCH_DT(dt, T, {
             auto kernel = nhwc ? Bicubic2dBwdListKernel<T, true> : Bicubic2dBwdListKernel<T, false>;
-            if (smem > 48 * 1024) {
-                err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            if (l.smem > 48 * 1024) {
+                err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(l.smem));
             }
             if (err == cudaSuccess) {
-                kernel<<<grid, threads, smem, s>>>(static_cast<const T*>(go), static_cast<T*>(gi), g,
-                                                   static_cast<int32_t>(entries), colsPB, borderOnly ? 1 : 0);
+                kernel<<<dim3(l.x, l.y), kListThreads, l.smem, s>>>(static_cast<const T*>(go), static_cast<T*>(gi), g, l.entries,
+                                                                    l.colsPB);
             }
         });
         CountLaunch();
@@ -1538,35 +1770,70 @@ cudaError_t Bicubic2dBwd(Dt dt, Layout lay, const void* go, void* gi, Shape4 sh,
         return cudaGetLastError();
     }
     if (!split) {
-        launchList(false);
+        launchList();
         return err != cudaSuccess ? err : cudaGetLastError();
     }
-    {
-        const int64_t positions = inner - 2LL * g.chan;
-        const int threads = static_cast<int>(std::min<int64_t>(kThreads, (positions + 31) / 32 * 32));
-        const int64_t gx = CeilDiv(positions, threads);
-        const int64_t gyCap = std::max<int64_t>(static_cast<int64_t>(NumSMs()) * 32 / gx, 1);
-        const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(std::min<int64_t>(std::min<int64_t>(g.rows, gyCap), 65535)), 1);
-        OPSCV_DISPATCH_DT(dt, T, {
-            const T* pgo = static_cast<const T*>(go);
-            T* pgi = static_cast<T*>(gi);
-            if (walk <= 9) {
-                if (nhwc) {
-                    Bicubic2dBwdRegKernel<T, true, 9><<<grid, threads, 0, s>>>(pgo, pgi, g);
-                } else {
-                    Bicubic2dBwdRegKernel<T, false, 9><<<grid, threads, 0, s>>>(pgo, pgi, g);
-                }
-            } else {
-                if (nhwc) {
-                    Bicubic2dBwdRegKernel<T, true, 17><<<grid, threads, 0, s>>>(pgo, pgi, g);
-                } else {
-                    Bicubic2dBwdRegKernel<T, false, 17><<<grid, threads, 0, s>>>(pgo, pgi, g);
-                }
-            }
-        });
-        CountLaunch();
+    const int64_t planes = g.rows / g.hin;
+    const ListLaunch l = planList(true);
+    WalkShape ws{};
+    ws.positions = planes * (inner - 2LL * g.chan);
+    const int64_t gx = CeilDiv(ws.positions, kWalkThreads);
+    // grads rows of a band: four source pixels beyond it, and the rounding of its ends
+    auto bandReads = [&](int64_t band) { return static_cast<int64_t>((static_cast<double>(band) + 5.0) * rowsPerRow) + 4; };
+    // Bands: every band re-reads four source pixels' worth of grads rows; fewer than five blocks per SM leave each of them
+    // waiting on its own loads (about 0.25 us a row), more share the issue slots (about 0.06 us a row).
+    double bestTime = 0.0;
+    for (int64_t b = 1; b <= sh.hin && b <= 256; ++b) {
+        const int64_t band = CeilDiv(sh.hin, b);
+        const int64_t reads = bandReads(band);
+        if (reads > kWalkMaxRows) {
+            continue;
+        }
+        const double k = static_cast<double>(CeilDiv(gx * CeilDiv(sh.hin, band), NumSMs()));
+        const double time = (static_cast<double>(reads) + 8.0) * std::max(0.25 * std::ceil(k / 5.0), 0.06 * k);
+        if (ws.bandRows == 0 || time < bestTime * 0.98) {
+            ws.bandRows = static_cast<int32_t>(band);
+            bestTime = time;
+        }
     }
-    launchList(true);
+    const int64_t bands = ws.bandRows > 0 ? CeilDiv(sh.hin, ws.bandRows) : 0;
+    const int64_t blocks = gx * bands + static_cast<int64_t>(l.x) * l.y;
+    if (ws.bandRows == 0 || blocks > INT32_MAX) {
+        launchList();
+        return err != cudaSuccess ? err : cudaGetLastError();
+    }
+    ws.maxRows = static_cast<int32_t>(bandReads(ws.bandRows));
+    ws.walkX = static_cast<int32_t>(gx);
+    ws.listX = l.x;
+    ws.listY = l.y;
+    ws.listCols = l.colsPB;
+    ws.listMax = l.entries;
+    const size_t smem = std::max(l.smem, static_cast<size_t>(ws.maxRows) * sizeof(WalkRecord) + static_cast<size_t>(ws.bandRows) * 8);
+    OPSCV_DISPATCH_DT(dt, T, {
+        auto launch = [&](auto columns) {
+            constexpr int K = decltype(columns)::value;
+            auto kernel = nhwc ? Bicubic2dBwdWalkKernel<T, true, K> : Bicubic2dBwdWalkKernel<T, false, K>;
+            if (smem > 48 * 1024) {
+                err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            }
+            if (err == cudaSuccess) {
+                kernel<<<static_cast<unsigned>(blocks), kWalkThreads, smem, s>>>(static_cast<const T*>(go), static_cast<T*>(gi),
+                                                                                 g, ws);
+            }
+        };
+        if (walk <= 8) {
+            launch(std::integral_constant<int, 8>{});
+        } else if (walk <= 10) {
+            launch(std::integral_constant<int, 10>{});
+        } else if (walk <= 12) {
+            launch(std::integral_constant<int, 12>{});
+        } else if (walk <= 14) {
+            launch(std::integral_constant<int, 14>{});
+        } else {
+            launch(std::integral_constant<int, 18>{});
+        }
+    });
+    CountLaunch();
     return err != cudaSuccess ? err : cudaGetLastError();
 }
 

@@ -265,3 +265,35 @@ def test_bicubic_2x_random_extents(ops, oracle, dev):
         gi = ops.upsample_bicubic2d_backward(g.to(dev), (2 * hi, 2 * wi), (n, c, hi, wi), False)
         assert np.array_equal(gi.cpu().numpy(),
                               oracle.bicubic2d_bwd(g.numpy(), (hi, wi), False, definition="gather")), (n, c, hi, wi)
+
+
+# The walk kernel at every register count (scales 1.2 to 4), rows that end in a partly used block, extents of three,
+# down-scales, and a user scale whose last row takes every remaining grads row (the list kernel)
+WALK_SHAPES = [(1, 2, 3, 3, 4, 4), (2, 3, 11, 13, 14, 17), (1, 3, 20, 30, 50, 67), (3, 1, 9, 140, 27, 300),
+               (1, 2, 17, 19, 66, 75), (1, 1, 40, 33, 21, 15), (1, 1, 300, 3, 700, 9), (5, 7, 6, 5, 21, 19)]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("fmt", ["NCHW", "NHWC"])
+@pytest.mark.parametrize("align", [False, True])
+@pytest.mark.parametrize("shape", WALK_SHAPES)
+def test_bicubic_backward_walk(ops, oracle, dev, dtype, fmt, align, shape):
+    n, c, hi, wi, ho, wo = shape
+    g, g32 = quant(torch.randn((n, c, ho, wo), generator=gen(120)), dtype)
+    gl = torch.from_numpy(_layout(g32, fmt)).to(dtype)
+    size = (n, hi, wi, c) if fmt == "NHWC" else (n, c, hi, wi)
+    gi = ops.upsample_bicubic2d_backward(gl.to(dev), (ho, wo), size, align, fmt)
+    ofmt = oracle.NHWC if fmt == "NHWC" else oracle.NCHW
+    check(gi, oracle.bicubic2d_bwd(_layout(g32, fmt), (hi, wi), align, fmt=ofmt, definition="gather"), dtype, exact=True)
+
+
+def test_bicubic_backward_walk_user_scale_and_non_finite(ops, oracle, dev):
+    g = torch.randn((1, 2, 60, 50), generator=gen(121))
+    for scales in ((2.3, 2.1), (1.5, 2.5), (4.0, 3.0)):
+        gi = ops.upsample_bicubic2d_backward(g.to(dev), (60, 50), (1, 2, 24, 20), False, scales=scales)
+        check(gi, oracle.bicubic2d_bwd(g.numpy(), (24, 20), False, scales, definition="gather"), torch.float32, exact=True)
+    g[0, 0, 31, 7], g[0, 1, 0, 49], g[0, 1, 59, 20] = float("inf"), float("nan"), -float("inf")
+    gi = ops.upsample_bicubic2d_backward(g.to(dev), (60, 50), (1, 2, 24, 20), False).cpu().numpy()
+    ref = oracle.bicubic2d_bwd(g.numpy(), (24, 20), False, definition="gather")
+    assert np.array_equal(gi.view(np.uint32)[~np.isnan(ref)], ref.view(np.uint32)[~np.isnan(ref)])
+    assert np.isnan(gi[np.isnan(ref)]).all()
