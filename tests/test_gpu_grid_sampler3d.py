@@ -145,3 +145,22 @@ def test_grid_sampler3d_ncdhw_through_channels_last(ops, oracle, dev, dtype, cha
     keep = torch.full_like(x, 7.0).to(dev)
     ops.grid_sampler3d_backward(go.to(dev), x.to(dev), grid.to(dev), interp, 0, False, mask=(False, True), input_grad=keep)
     assert torch.equal(keep.cpu(), torch.full_like(x, 7.0))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("c", [16, 20, 36])
+@pytest.mark.parametrize("vol", [((4, 5, 6), (2, 3, 4)), ((3, 7, 43), (5, 3, 9)), ((1, 2, 2), (8, 16, 17)), ((5, 1, 3), (1, 1, 2))])
+def test_channels_last_copies_at_ragged_volumes(ops, oracle, dev, dtype, c, vol):
+    """NCDHW tensors that go through channels-last copies in the workspace: extents that are no multiple of a tile, a word or
+    either side of it (fp32 forward and grad_grid: the oracle's bits)."""
+    (d, h, w), (do, ho, wo) = vol
+    x, x32 = quant(torch.randn((2, c, d, h, w), generator=gen(130)), dtype)
+    grid, g32 = quant(make_grid(2, do, ho, wo, 131), dtype)
+    go, go32 = quant(torch.randn((2, c, do, ho, wo), generator=gen(132)), dtype)
+    y = ops.grid_sampler3d(x.to(dev), grid.to(dev), 0, 0, False)
+    check(y, oracle.grid_sampler3d_fwd(x32, g32, 0, False), dtype, exact=(dtype == torch.float32))
+    if dtype == torch.float32:
+        gi, gg = ops.grid_sampler3d_backward(go.to(dev), x.to(dev), grid.to(dev), 0, 0, False)
+        ri, rg = oracle.grid_sampler3d_bwd(go32, x32, g32, 0, 0, False)
+        np.testing.assert_allclose(gi.cpu().numpy(), ri, rtol=1e-5, atol=1e-6 * max(1.0, float(np.abs(ri).max())))
+        assert np.array_equal(gg.cpu().numpy(), rg)
