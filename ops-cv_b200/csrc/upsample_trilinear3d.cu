@@ -23,6 +23,7 @@
 // axis, zero padded to the longest) are built on the device by BuildTrilinearBwdTables.
 #include <algorithm>
 
+#include "cp_async.cuh"
 #include "launch_util.cuh"
 
 namespace opscv {
@@ -461,6 +462,199 @@ void LaunchAxis(const T* x, T* y, const Trilinear3dGeom& g, const RowLaunch& rl,
     }
 }
 
+// The W and the H stage of the backward in one kernel, NCDHW: a block takes one grad_output slice (plane, d), or a band
+// of grad_input rows of it, copies the slice's rows into shared memory as they are (asynchronous 16-byte copies), forms
+// the W sums of those rows there and the H sums from them: the sums of the two stage kernels in the same order, so the
+// bits are theirs. The W stage's buffer, the largest of the operator (fp16 2x32 planes 32x56x56 <- 64x112x112: 103 MB
+// written and read again, more than the L2 keeps), is gone, and a tap is a shared-memory read instead of a 2-byte global
+// load. What bounds it is instruction issue on the taps (76 % of the slots). At those sizes: 95 us in two kernels -> 59 us.
+struct PlaneShape {
+    int64_t slices;
+    int32_t ho, wo, hi, wi;
+    int32_t bandRows, bands; // grad_input rows per block, blocks per slice
+    int32_t capRows;         // most grad_output rows a band reads
+    int32_t tapsH, tapsW;
+};
+
+__host__ __device__ __forceinline__ int32_t PlaneRawBytes(int32_t rows, int32_t wo, int32_t es)
+{
+    return (rows * wo * es + 16 + 15) & ~15; // the copy keeps the phase of its global address within 16 bytes
+}
+
+template <typename T, int KW, int V>
+__global__ void __launch_bounds__(kThreads, 4)
+    TrilinearBwdPlaneKernel(const T* __restrict__ go, float* __restrict__ out, PlaneShape sh,
+                            const int32_t* __restrict__ startH, const int32_t* __restrict__ countH,
+                            const float* __restrict__ wH, const int32_t* __restrict__ startW,
+                            const int32_t* __restrict__ countW, const float* __restrict__ wW)
+{
+    extern __shared__ __align__(16) unsigned char planeSmem[];
+    __shared__ int32_t sLo, sHi;
+    float* t1 = reinterpret_cast<float*>(planeSmem + PlaneRawBytes(sh.capRows, sh.wo, sizeof(T))); // [capRows][wi]
+    float* sW = t1 + ((sh.capRows * sh.wi + 3) & ~3);                                            // [bandRows][tapsH]
+    int32_t* sStart = reinterpret_cast<int32_t*>(sW + sh.bandRows * sh.tapsH);                   // [bandRows]
+    int32_t* sCount = sStart + sh.bandRows;
+    const int64_t slice = blockIdx.x / sh.bands;
+    const int32_t band = static_cast<int32_t>(blockIdx.x - slice * sh.bands);
+    const int32_t y0 = band * sh.bandRows, y1 = min(y0 + sh.bandRows, sh.hi), rows = y1 - y0;
+    const int32_t tid = threadIdx.x;
+    if (rows <= 0) {
+        return;
+    }
+    if (tid == 0) {
+        sLo = sh.ho;
+        sHi = 0;
+    }
+    __syncthreads();
+    for (int32_t r = tid; r < rows; r += kThreads) {
+        const int32_t a = __ldg(startH + y0 + r), n = __ldg(countH + y0 + r);
+        sStart[r] = a;
+        sCount[r] = n;
+        if (n > 0) {
+            atomicMin(&sLo, a);
+            atomicMax(&sHi, a + n);
+        }
+    }
+    for (int32_t e = tid; e < rows * sh.tapsH; e += kThreads) {
+        sW[e] = __ldg(wH + static_cast<int64_t>(y0) * sh.tapsH + e);
+    }
+    __syncthreads();
+    const int32_t lo = sLo, n = max(0, min(min(sHi, sh.ho) - lo, sh.capRows));
+    const T* src = go + (slice * sh.ho + lo) * static_cast<int64_t>(sh.wo);
+    const int32_t total = n * sh.wo;
+    const int32_t phase = static_cast<int32_t>(reinterpret_cast<uintptr_t>(src) & 15) / static_cast<int32_t>(sizeof(T));
+    constexpr int kVec = 16 / sizeof(T);
+    T* raw = reinterpret_cast<T*>(planeSmem) + phase;
+    const int32_t head = min(total, phase == 0 ? 0 : kVec - phase); // elements before the first 16-byte boundary
+    const int32_t words = (total - head) / kVec;
+    for (int32_t q = tid; q < words; q += kThreads) {
+        CpAsync16(raw + head + q * kVec, src + head + q * kVec);
+    }
+    CpAsyncCommit();
+    for (int32_t e = tid; e < head; e += kThreads) {
+        raw[e] = __ldg(src + e);
+    }
+    for (int32_t e = head + words * kVec + tid; e < total; e += kThreads) {
+        raw[e] = __ldg(src + e);
+    }
+    CpAsyncWait<0>();
+    __syncthreads();
+    // W sums: a thread keeps the weights of its column for all the rows that it visits
+    const int32_t ct = min(sh.wi, kThreads), rt = kThreads / ct;
+    const int32_t ty = tid / ct;
+    if (ty < rt) {
+        for (int32_t col = tid - ty * ct; col < sh.wi; col += ct) {
+            const int32_t first = __ldg(startW + col), cnt = __ldg(countW + col);
+            float wr[KW];
+#pragma unroll
+            for (int e = 0; e < KW; ++e) {
+                wr[e] = e < sh.tapsW ? __ldg(wW + static_cast<int64_t>(col) * sh.tapsW + e) : 0.0f;
+            }
+            const T* p = raw + ty * sh.wo + first;
+            float* q = t1 + ty * sh.wi + col;
+            for (int32_t r = ty; r < n; r += rt, p += rt * sh.wo, q += rt * sh.wi) {
+                float acc = 0.0f;
+#pragma unroll
+                for (int e = 0; e < KW; ++e) {
+                    if (e < cnt) {
+                        acc = Add(acc, Mul(wr[e], DType<T>::ToF(p[e])));
+                    }
+                }
+                *q = acc;
+            }
+        }
+    }
+    __syncthreads();
+    // H sums, V adjacent columns per thread
+    const int32_t packs = sh.wi / V;
+    const int32_t hc = min(packs, kThreads), hr = kThreads / hc;
+    const int32_t hy = tid / hc;
+    float* po = out + (slice * sh.hi + y0) * static_cast<int64_t>(sh.wi);
+    if (hy < hr) {
+        for (int32_t c = tid - hy * hc; c < packs; c += hc) {
+            for (int32_t r = hy; r < rows; r += hr) {
+                const int32_t taps = sCount[r];
+                const int32_t rel = sStart[r] - lo;
+                const float* p = t1 + rel * sh.wi + c * V;
+                const float* w = sW + r * sh.tapsH;
+                float acc[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    acc[v] = 0.0f;
+                }
+                for (int32_t k = 0; k < taps && rel + k < n; ++k, p += sh.wi) {
+                    float t[V];
+                    LoadPack<float, V>(p, t);
+                    const float wk = w[k];
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        acc[v] = Add(acc[v], Mul(wk, t[v]));
+                    }
+                }
+                StorePack<float, V>(po + static_cast<int64_t>(r) * sh.wi + c * V, acc);
+            }
+        }
+    }
+}
+
+// Shape and shared memory of the plane kernel; false where a band of at least eight rows (or all of them) does not fit
+// 56 KB (four blocks per SM). More bands than that asks for where slices alone leave SMs idle.
+bool PlanPlane(const Trilinear3dGeom& g, const TrilinearBwdTables& t, int es, int64_t slices, PlaneShape* out, size_t* smem)
+{
+    if (g.chan != 1 || t.taps[2] > 10 || t.taps[1] > 64) {
+        return false;
+    }
+    PlaneShape p{slices, g.ho, g.wo, g.hi, g.wi, 0, 0, 0, t.taps[1], t.taps[2]};
+    // grad_output rows of a band: source positions are scale apart
+    const double perRow = g.sh > 0.0f ? 1.0 / static_cast<double>(g.sh) : static_cast<double>(g.ho);
+    for (int32_t nb = 1; nb <= g.hi; ++nb) {
+        const int32_t band = (g.hi + nb - 1) / nb;
+        if (nb > 1 && band < 8) {
+            return p.bands > 0;
+        }
+        const int32_t cap = static_cast<int32_t>(std::min<double>(g.ho, std::ceil((band + 2) * perRow) + t.taps[1] + 4));
+        const size_t need = static_cast<size_t>(PlaneRawBytes(cap, g.wo, es)) +
+                            (static_cast<size_t>((cap * g.wi + 3) & ~3) + static_cast<size_t>(band) * (t.taps[1] + 2)) * 4;
+        if (static_cast<int64_t>(cap) * (static_cast<int64_t>(g.wo) * es + static_cast<int64_t>(g.wi) * 4) > 56 * 1024 ||
+            need > 60 * 1024) {
+            continue;
+        }
+        p.bandRows = band;
+        p.bands = (g.hi + band - 1) / band;
+        p.capRows = cap;
+        *out = p;
+        *smem = need;
+        if (slices * p.bands >= static_cast<int64_t>(NumSMs()) * 4) {
+            break;
+        }
+    }
+    return p.bands > 0 && slices * p.bands <= INT32_MAX;
+}
+
+template <typename T, int V>
+cudaError_t LaunchPlane(const T* go, float* out, const PlaneShape& p, const TrilinearBwdTables& t, size_t smem, cudaStream_t s)
+{
+    auto launch = [&](auto kernel) {
+        if (smem > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            if (e != cudaSuccess) {
+                return e;
+            }
+        }
+        kernel<<<static_cast<unsigned>(p.slices * p.bands), kThreads, smem, s>>>(go, out, p, t.start[1], t.count[1], t.w[1],
+                                                                                t.start[2], t.count[2], t.w[2]);
+        CountLaunch();
+        return cudaGetLastError();
+    };
+    if (p.tapsW <= 4) {
+        return launch(TrilinearBwdPlaneKernel<T, 4, V>);
+    }
+    if (p.tapsW <= 5) {
+        return launch(TrilinearBwdPlaneKernel<T, 5, V>);
+    }
+    return launch(TrilinearBwdPlaneKernel<T, 10, V>);
+}
+
 } // namespace
 
 uint64_t Trilinear3dFwdWorkspace(const Trilinear3dGeom& g, int64_t planes)
@@ -569,6 +763,18 @@ cudaError_t Trilinear3dBwd(Dt dt, const void* go, void* gi, float* stage, Trilin
     OPSCV_DISPATCH_DT(dt, T, {
         // W: (planes * dout * ho) x wo x chan -> wi;  H: (planes * dout) x ho x (wi * chan) -> hi;  D: planes x dout x
         // (hi * wi * chan) -> di
+        PlaneShape ps;
+        size_t smem = 0;
+        if (PlanPlane(g, t, static_cast<int>(sizeof(T)), planes * g.dout, &ps, &smem)) {
+            const T* pg = static_cast<const T*>(go);
+            const cudaError_t e = g.wi % 4 == 0 ? LaunchPlane<T, 4>(pg, t2, ps, t, smem, s) : LaunchPlane<T, 1>(pg, t2, ps, t, smem, s);
+            if (e != cudaSuccess) {
+                return e;
+            }
+            LaunchBwdStage<float, T>(t2, static_cast<T*>(gi), planes, g.dout, g.di,
+                                     static_cast<int64_t>(g.hi) * g.wi * g.chan, t.start[0], t.count[0], t.w[0], t.taps[0], s);
+            return cudaGetLastError();
+        }
         if (g.chan <= 4) {
             const int64_t rowsW = planes * g.dout * g.ho;
             const RowLaunch rl = RowTiling(rowsW, static_cast<int64_t>(g.wi) * g.chan, kThreads);

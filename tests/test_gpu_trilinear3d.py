@@ -141,3 +141,17 @@ def test_trilinear3d_larger_case_is_bit_exact(ops, oracle, dev):
     g = torch.randn((6, 8, 24, 48, 48), generator=gen(119))
     gi = ops.upsample_trilinear3d_backward(g.to(dev), (24, 48, 48), (6, 8, 12, 24, 24), False)
     assert np.array_equal(gi.cpu().numpy(), oracle.trilinear3d_bwd(g.numpy(), (12, 24, 24), False))
+
+
+# The plane kernel of the backward: whole slices and bands of them, slices that start at every offset within 16 bytes, rows
+# wider than a block, every register count of the W taps, an extent that takes the stage kernels (taps past ten)
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("align", [False, True])
+@pytest.mark.parametrize("shape", [(1, 2, 2, 5, 3, 3, 9, 5), (1, 1, 2, 60, 70, 2, 119, 139), (1, 1, 1, 3, 300, 2, 5, 599),
+                                   (1, 1, 2, 150, 5, 2, 300, 11), (1, 2, 2, 9, 8, 2, 38, 33), (1, 1, 2, 4, 3, 2, 40, 31),
+                                   (3, 1, 1, 33, 20, 1, 17, 9)])
+def test_trilinear3d_backward_planes(ops, oracle, dev, dtype, align, shape):
+    n, c, di, hi, wi, do, ho, wo = shape
+    g, g32 = quant(torch.randn((n, c, do, ho, wo), generator=gen(140)), dtype)
+    gi = ops.upsample_trilinear3d_backward(g.to(dev), (do, ho, wo), (n, c, di, hi, wi), align)
+    check(gi, oracle.trilinear3d_bwd(g32, (di, hi, wi), align), dtype, exact=(dtype == torch.float32))
