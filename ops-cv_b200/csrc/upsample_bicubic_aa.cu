@@ -404,13 +404,35 @@ __global__ void __launch_bounds__(MAXT, BULK ? 1 : 2)
                         }
                     }
                 }
+                // Slots past the run are not touched (an Inf / NaN input must not leak in). Away from the first and last
+                // rows the run fills all slots but the last, which one test then covers: photographs 487 -> 463 us against a test
+                // per slot. With three slots the tests are few and the other form's registers cost more (87 -> 92 us).
+                F2 xp[VC / 2];
 #pragma unroll
-                for (int a = 0; a < NS; ++a) {
-                    const F2 w = a == NS - 1 ? F2{mLast.x} : (a % 2 == 0 ? F2{m[a / 2].x} : F2{m[a / 2].y});
-                    if (a < cnt) { // slots past the run are not touched (an Inf / NaN input must not leak in)
+                for (int k = 0; k < VC / 2; ++k) {
+                    xp[k] = MakeF2(xv[2 * k], xv[2 * k + 1]);
+                }
+                auto slot = [&](int a, F2 w) {
 #pragma unroll
-                        for (int k = 0; k < VC / 2; ++k) {
-                            acc[a][k] = Fma2(w, MakeF2(xv[2 * k], xv[2 * k + 1]), acc[a][k]);
+                    for (int k = 0; k < VC / 2; ++k) {
+                        acc[a][k] = Fma2(w, xp[k], acc[a][k]);
+                    }
+                };
+                if (NS > 3 && cnt >= NS - 1) {
+#pragma unroll
+                    for (int a = 0; a + 1 < NS; a += 2) {
+                        const ulonglong2 w = m[a / 2];
+                        slot(a, F2{w.x});
+                        slot(a + 1, F2{w.y});
+                    }
+                    if (cnt == NS) {
+                        slot(NS - 1, F2{mLast.x});
+                    }
+                } else {
+#pragma unroll
+                    for (int a = 0; a < NS; ++a) {
+                        if (a < cnt) {
+                            slot(a, a == NS - 1 ? F2{mLast.x} : F2{a % 2 == 0 ? m[a / 2].x : m[a / 2].y});
                         }
                     }
                 }
@@ -490,7 +512,7 @@ __global__ void __launch_bounds__(kThreads)
 // with the column weights it keeps in registers as packed pairs. Weights come from the slot records of both axes; a
 // weight that does not exist is 0 and its product changes nothing while the grads are finite.
 // What bounds it is instruction issue: 125 instructions per warp and row (photographs, fp32) while every row walked its
-// own grads rows and sums were single, 68 % of the issue slots busy. 64x3x1024x1024 <-> 224x224 fp32, both directions: 529 -> 487 us.
+// own grads rows and sums were single, 68 % of the issue slots busy. 64x3x1024x1024 <-> 224x224 fp32, both directions: 529 -> 463 us.
 constexpr int kBwdRows = 4;     // grad_input rows per synchronisation
 constexpr int kBwdRowSlots = 8; // grads rows that reach four consecutive grad_input rows (4 + ceil(3 / scale) + 1)
 constexpr int kBwdGroupBytes = (kBwdRowSlots + 1) * 16; // weights of a step, its first grads row and their count
