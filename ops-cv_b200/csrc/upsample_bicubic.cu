@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(kListThreads) Bicubic2dBwdListKernel(const T* 
 // once per block into shared-memory records. First and last rows take up to four taps per grads row: they ride along
 // in the blocks whose band holds them. The first and the last column are list blocks, the first blocks of the same grid,
 // so that their long chains run under the walk. fp32 8x64 planes 60x80 <- 150x199: 230 us as two launches that loaded
-// every term -> 82 us.
+// every term -> 80 us.
 constexpr int kOpen = 5;
 constexpr int kWalkThreads = 128;
 constexpr int kWalkMaxRows = 448; // grads rows that a band may read (their records stay below 48 KB)
@@ -1821,13 +1821,18 @@ cudaError_t Bicubic2dBwd(Dt dt, Layout lay, const void* go, void* gi, Shape4 sh,
                                                                                  g, ws);
             }
         };
-        if (walk <= 8) {
+        // A walk spans four source pixels: at most ceil(4 / scale) columns, with a margin for rounding (a column whose walk is
+        // longer all the same takes the uncached walk).
+        const int64_t columns = static_cast<int64_t>(std::ceil(4.0 * perScale + 0.02));
+        if (columns <= 6) {
+            launch(std::integral_constant<int, 6>{});
+        } else if (columns <= 8) {
             launch(std::integral_constant<int, 8>{});
-        } else if (walk <= 10) {
+        } else if (columns <= 10) {
             launch(std::integral_constant<int, 10>{});
-        } else if (walk <= 12) {
+        } else if (columns <= 12) {
             launch(std::integral_constant<int, 12>{});
-        } else if (walk <= 14) {
+        } else if (columns <= 14) {
             launch(std::integral_constant<int, 14>{});
         } else {
             launch(std::integral_constant<int, 18>{});
