@@ -244,6 +244,101 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
+// The same tile for rows that allow no store wider than two elements (odd widths). A thread owns NC column groups of V
+// elements, a block width apart, so the stores of a warp stay contiguous, and looks a row up once for all of them: with
+// one group per walk three table reads and the comparisons went with every output, and a width just above a multiple of
+// the block (513) walked the tile once more for its last column. Same expressions, same bits.
+// fp32 168 planes 65x65 -> 513x513: 53 -> 44 us, 40.3 M -> 28.8 M warp instructions.
+template <typename T, int V, int NC>
+__global__ void __launch_bounds__(kThreads)
+    BilinearFwdColumnsKernel(const T* __restrict__ x, T* __restrict__ y, int64_t planes, int32_t hin, int32_t win,
+                             int32_t hout, int32_t wout, LerpAxis th, LerpAxis tw, int32_t tileRows, int32_t stageStride)
+{
+    extern __shared__ __align__(16) unsigned char smemRaw[];
+    const int64_t pBase = static_cast<int64_t>(blockIdx.x) * blockDim.y;
+    const int32_t np = static_cast<int32_t>(min(static_cast<int64_t>(blockDim.y), planes - pBase));
+    const int32_t ha = blockIdx.y * tileRows, hb = min(hout, ha + tileRows);
+    const int32_t r0 = __ldg(th.lo + ha), r1 = __ldg(th.hi + hb - 1) + 1;
+    const int64_t planeElems = hin * static_cast<int64_t>(win);
+    const T* src = nullptr;
+    for (int32_t pl = 0; pl < np; ++pl) {
+        const T* staged = StageSpan<T>(x + (pBase + pl) * planeElems + static_cast<int64_t>(r0) * win,
+                                       static_cast<int64_t>(r1 - r0) * win, smemRaw + pl * stageStride);
+        if (pl == static_cast<int32_t>(threadIdx.y)) {
+            src = staged;
+        }
+    }
+    __syncthreads();
+    if (static_cast<int32_t>(threadIdx.y) >= np) {
+        return;
+    }
+    const int32_t groups = wout / V, ct = blockDim.x;
+    T* yp = y + (pBase + threadIdx.y) * hout * static_cast<int64_t>(wout);
+    for (int32_t g0 = threadIdx.x; g0 < groups; g0 += NC * ct) {
+        int32_t wl[NC][V], wh[NC][V];
+        float dx[NC][V], dx1[NC][V], top[NC][V], bot[NC][V];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            const int32_t g = min(g0 + j * ct, groups - 1); // a group past the row is computed and not stored
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                wl[j][k] = __ldg(tw.lo + g * V + k);
+                wh[j][k] = __ldg(tw.hi + g * V + k);
+                dx[j][k] = __ldg(tw.delta + g * V + k);
+                dx1[j][k] = Sub(1.0f, dx[j][k]);
+            }
+        }
+        auto blendRow = [&](int32_t row, float (&out)[NC][V]) {
+            const T* xr = src + (row - r0) * win;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+#pragma unroll
+                for (int k = 0; k < V; ++k) {
+                    out[j][k] = Add(Mul(dx1[j][k], DType<T>::ToF(xr[wl[j][k]])), Mul(dx[j][k], DType<T>::ToF(xr[wh[j][k]])));
+                }
+            }
+        };
+        auto copyRow = [&](const float (&from)[NC][V], float (&to)[NC][V]) {
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+#pragma unroll
+                for (int k = 0; k < V; ++k) {
+                    to[j][k] = from[j][k];
+                }
+            }
+        };
+        int32_t curTop = -1, curBot = -1;
+        T* dst = yp + static_cast<int64_t>(ha) * wout + g0 * V;
+        for (int32_t h = ha; h < hb; ++h) {
+            const int32_t lo = __ldg(th.lo + h), hi = __ldg(th.hi + h);
+            const float dy = __ldg(th.delta + h);
+            if (lo != curTop) {
+                if (lo == curBot) {
+                    copyRow(bot, top);
+                } else {
+                    blendRow(lo, top);
+                }
+                curTop = lo;
+            }
+            if (hi != curBot) {
+                if (hi == curTop) {
+                    copyRow(top, bot);
+                } else {
+                    blendRow(hi, bot);
+                }
+                curBot = hi;
+            }
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                if (g0 + j * ct < groups) {
+                    BlendStore<T, V>(dst + j * ct * V, top[j], bot[j], dy);
+                }
+            }
+            dst += wout;
+        }
+    }
+}
+
 // ---- per-thread asynchronous row queues ------------------------------------------------------------------------
 // The row walks below are serial chains per thread, so what bounds them is the number of bytes a thread has in
 // flight. cp.async copies a thread's own piece of the next rows into a private shared-memory queue (one commit
@@ -2026,15 +2121,33 @@ cudaError_t BilinearFwd(Dt dt, Layout lay, const void* x, void* y, Shape4 sh, Le
                 const int32_t tiles = static_cast<int32_t>(CeilDiv(sh.hout, plan.tileRows));
                 const int32_t stride = static_cast<int32_t>(
                     (StageBytes(static_cast<int64_t>(plan.bandRows) * sh.win, sizeof(T)) + 15) & ~size_t(15));
+                // Several column groups per thread where that leaves every SM its threads: three or four of one element,
+                // whichever leaves fewer lanes of the row's warps idle. With fewer threads than that a walk per group is as
+                // long and has more of them (bf16 800 planes 24x26 -> 48x51, a pyramid step: 53 us, 59 us with four groups).
                 const int vv = std::min(v, 4);
-                OPSCV_DISPATCH_VEC(vv, V, {
-                    if constexpr (V <= 4) {
-                        const dim3 block = PlaneBlock(sh.wout / V, planes, plan.planesPerBlock);
-                        const dim3 grid(static_cast<unsigned>(CeilDiv(planes, block.y)), static_cast<unsigned>(tiles));
-                        BilinearFwdTileKernel<T, V><<<grid, block, static_cast<size_t>(stride) * block.y, s>>>(
-                            px, py, planes, sh.hin, sh.win, sh.hout, sh.wout, th, tw, plan.tileRows, stride);
-                    }
-                });
+                const int32_t groups = sh.wout / vv;
+                const int64_t walks = planes * groups * tiles, full = static_cast<int64_t>(NumSMs()) * 2048;
+                auto threads = [&](int32_t nc) { return static_cast<int32_t>(CeilDiv(groups, nc)); };
+                auto lanes = [&](int32_t nc) { return nc * ((threads(nc) + 31) & ~31); };
+                auto launchTile = [&](auto kernel, int32_t nc) {
+                    const dim3 block = PlaneBlock(threads(nc), planes, plan.planesPerBlock);
+                    const dim3 grid(static_cast<unsigned>(CeilDiv(planes, block.y)), static_cast<unsigned>(tiles));
+                    kernel<<<grid, block, static_cast<size_t>(stride) * block.y, s>>>(
+                        px, py, planes, sh.hin, sh.win, sh.hout, sh.wout, th, tw, plan.tileRows, stride);
+                };
+                if (vv == 4) {
+                    launchTile(BilinearFwdTileKernel<T, 4>, 1);
+                } else if (vv == 2 && walks >= 2 * full) {
+                    launchTile(BilinearFwdColumnsKernel<T, 2, 2>, 2);
+                } else if (vv == 2) {
+                    launchTile(BilinearFwdTileKernel<T, 2>, 1);
+                } else if (walks < 4 * full) {
+                    launchTile(BilinearFwdTileKernel<T, 1>, 1);
+                } else if (threads(3) > 128 && lanes(3) < lanes(4)) {
+                    launchTile(BilinearFwdColumnsKernel<T, 1, 3>, 3);
+                } else {
+                    launchTile(BilinearFwdColumnsKernel<T, 1, 4>, 4);
+                }
             } else {
                 OPSCV_DISPATCH_VEC(v, V, {
                     if constexpr (V * sizeof(T) <= 16) {
