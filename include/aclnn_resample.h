@@ -353,6 +353,16 @@ ACLNN_API aclnnStatus aclnnGridSampler2DBackward(void* workspace, uint64_t works
 ACLNN_API aclnnStatus opscvDebugAxisTable(int32_t kind, int64_t inSize, int64_t outSize, int32_t alignCorners,
                                           float userScale, int32_t* i0, int32_t* i1, float* f0, int32_t* tapsOut);
 
+/* The launch shape that an operator takes for contiguous, aligned tensors of the given sizes, evaluated on the host alone (no
+ * GPU is needed), so that tests can hold the bounds it was sized by against a restatement of the index arithmetic and can
+ * tell which kernel a call reaches. sizes = {N, C, forward-input H, W, forward-output H, W}; `scales` as at the operator's
+ * entry point. *taken is 0 where the kernel does not take the call, else 1 and `values` is filled:
+ * kind 0, UpsampleBilinear2dBackward by row walks: {grad_input rows per band, most grads rows of a band, groups per stage
+ *   (NCHW) or columns per tile (NHWC), most grads rows of a stage (NCHW) or grads columns of a tile (NHWC), columns per
+ *   thread (NCHW) or channel slices (NHWC), planes or images per block, bands, shared-memory bytes}. */
+ACLNN_API aclnnStatus opscvDebugPlan(int32_t kind, int32_t elemSize, aclFormat format, const int64_t sizes[6],
+                                     int32_t alignCorners, const double scales[2], int32_t* taken, int64_t values[8]);
+
 /* ---- allocation-free bilinear forward ------------------------------------------------------------------------
  * No counterpart in the reference (its entry points all take a workspace). For callers that can neither allocate
  * device memory nor pass a workspace at the point of the call: the per-axis tap tables live in a fixed 192 KiB

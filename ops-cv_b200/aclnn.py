@@ -9,7 +9,7 @@ from . import (ACL_BF16, ACL_DOUBLE, ACL_FLOAT, ACL_FLOAT16, ACL_FORMAT_NCDHW, A
 
 __all__ = [
     "AclnnError", "acl_tensor", "int_array", "bool_array", "float_array", "resize", "two_phase", "set_deterministic", "set_backward_algo",
-    "launch_count", "reset_launch_count", "async_copy_timeouts", "last_error", "debug_axis_table", "upsample_nearest2d",
+    "launch_count", "reset_launch_count", "async_copy_timeouts", "last_error", "debug_axis_table", "debug_plan", "upsample_nearest2d",
     "upsample_nearest2d_backward", "upsample_bilinear2d", "upsample_bilinear2d_no_alloc",
     "upsample_bilinear2d_backward", "upsample_bicubic2d", "upsample_bicubic2d_backward", "upsample_bilinear2d_aa",
     "upsample_bilinear2d_aa_backward", "upsample_nearest_exact2d", "upsample_nearest_exact2d_backward",
@@ -173,6 +173,18 @@ def debug_axis_table(kind, in_size, out_size, align=False, user_scale=0.0):
     if status != 0:
         raise AclnnError("opscvDebugAxisTable", status)
     return i0, i1, f0
+
+
+def debug_plan(kind, elem_size, sizes, fmt="NCHW", align=False, scales=(0.0, 0.0)):
+    """The launch shape of a kernel for these sizes (see opscvDebugPlan), or None where it does not take the call."""
+    taken = ctypes.c_int32(0)
+    values = (ctypes.c_int64 * 8)()
+    kinds = {"bilinear_backward_walk": 0}
+    status = lib().opscvDebugPlan(kinds[kind], elem_size, _FORMATS[fmt], (ctypes.c_int64 * 6)(*sizes), int(align),
+                                  (ctypes.c_double * 2)(*scales), ctypes.byref(taken), values)
+    if status != 0:
+        raise AclnnError("opscvDebugPlan", status)
+    return list(values) if taken.value else None
 
 
 def _out_shape(x, out_hw, fmt):

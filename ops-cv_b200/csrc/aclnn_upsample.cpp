@@ -1972,4 +1972,34 @@ aclnnStatus opscvDebugAxisTable(int32_t kind, int64_t inSize, int64_t outSize, i
     return ACLNN_SUCCESS;
 }
 
+aclnnStatus opscvDebugPlan(int32_t kind, int32_t elemSize, aclFormat format, const int64_t sizes[6], int32_t alignCorners,
+                           const double scales[2], int32_t* taken, int64_t values[8])
+{
+    static const char* api = "opscvDebugPlan";
+    if (sizes == nullptr || scales == nullptr || taken == nullptr || values == nullptr) {
+        return Fail(ACLNN_ERR_PARAM_NULLPTR, "%s: null argument", api);
+    }
+    for (int i = 0; i < 6; ++i) {
+        if (sizes[i] <= 0 || sizes[i] > INT32_MAX) {
+            return Fail(ACLNN_ERR_PARAM_INVALID, "%s: sizes must be in [1, INT32_MAX]", api);
+        }
+    }
+    if (elemSize != 2 && elemSize != 4) {
+        return Fail(ACLNN_ERR_PARAM_INVALID, "%s: elemSize must be 2 or 4", api);
+    }
+    const bool align = alignCorners != 0;
+    const Layout lay = format == ACL_FORMAT_NHWC ? kNHWC : kNCHW;
+    Geom in{sizes[0], sizes[1], sizes[2], sizes[3]}, out{sizes[0], sizes[1], sizes[4], sizes[5]};
+    const Shape4 sh = MakeShape(in, out);
+    switch (kind) {
+        case 0: {
+            const AxisGeom gh{sh.hin, sh.hout, BilinearGradScale(in.h, out.h, align, static_cast<float>(scales[0]))};
+            const AxisGeom gw{sh.win, sh.wout, BilinearGradScale(in.w, out.w, align, static_cast<float>(scales[1]))};
+            *taken = DebugBilinearBwdWalk(elemSize, lay, sh, gh, gw, !align, values) ? 1 : 0;
+            return ACLNN_SUCCESS;
+        }
+        default: return Fail(ACLNN_ERR_PARAM_INVALID, "%s: unknown kind %d", api, kind);
+    }
+}
+
 } // extern "C"

@@ -697,11 +697,15 @@ bool Overshoots(const BwdAxis& a)
 }
 
 // Most grads indices that `groups` adjacent groups hold: the ends of the axis, where indices are clamped, exactly;
-// elsewhere the integers in an interval of groups / scale (and one more for the rounding of the positions).
+// elsewhere the integers in an interval of groups / scale, widened at both ends by the rounding of the positions.
+// In units of an index, index + offset is off by nothing below 2^23 and by 1/2 below 2^24, the product and the difference by
+// index * 2^-24 each: together at most 1/2 below 2^22, 5/2 below 2^24. From there on indices share a position and no such
+// bound holds.
+constexpr int32_t kMostExtent = 1 << 24;
 int32_t MostRows(const BwdAxis& a, int32_t groups)
 {
-    const float inner = static_cast<float>(groups) / a.scale + 2.0f;
-    const int32_t most = inner < static_cast<float>(a.out) ? static_cast<int32_t>(inner) : a.out;
+    const double inner = groups / static_cast<double>(a.scale) + (a.out <= kMostExtent / 4 ? 2.0 : 6.0);
+    const int32_t most = inner < a.out ? static_cast<int32_t>(inner) : a.out;
     return std::max({most, GroupStart(a, groups), a.out - GroupStart(a, a.last - groups + 1)});
 }
 
@@ -722,12 +726,20 @@ int32_t PickBandRows(int32_t rows, int64_t blocksPerBand, int64_t slots)
     return static_cast<int32_t>(std::max<int64_t>(best, CeilDiv(rows, 65535)));
 }
 
-template <typename TIn, typename TOut>
-bool LaunchColumns(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, cudaStream_t s)
+// Launch shape of the column kernel; false where it does not take the call.
+struct ColumnsPlan {
+    ColumnsShape q;
+    int32_t k, threads, bands; // columns per thread
+    int64_t planeGroups;
+    size_t smem;
+};
+bool PlanColumns(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, ColumnsPlan* plan)
 {
     constexpr int32_t kTarget = 256; // threads per block to aim for
+    constexpr size_t kMostSmem = 96 * 1024;
     const int64_t planes = sh.n * sh.c;
-    ColumnsShape q{};
+    ColumnsShape& q = plan->q;
+    q = ColumnsShape{};
     q.hin = sh.hin;
     q.win = sh.win;
     q.hout = sh.hout;
@@ -746,11 +758,15 @@ bool LaunchColumns(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah
     const int32_t threads = static_cast<int32_t>(CeilDiv(q.planesPerBlock * q.team, 32)) * 32 + 32; // and the copying warp
     const int64_t planeGroups = CeilDiv(planes, q.planesPerBlock);
     // about eight grads rows per stage, no more than some twelve kilobytes of them; three stages unless they are large
-    const int32_t rowBytes = sh.wout * static_cast<int32_t>(sizeof(TIn));
+    const int32_t rowBytes = sh.wout * es;
     const float perGroup = std::max(1.0f / ah.scale, 1.0f);
     q.stageGroups = static_cast<int32_t>(std::min(8.0f, 12288.0f / (static_cast<float>(rowBytes) * q.planesPerBlock)) / perGroup);
     q.stageGroups = std::max(1, std::min(q.stageGroups, kColumnsBatch));
-    q.slotBytes = (MostRows(ah, q.stageGroups) * rowBytes + 30) / 16 * 16;
+    const int64_t slotBytes = (static_cast<int64_t>(MostRows(ah, q.stageGroups)) * rowBytes + 30) / 16 * 16;
+    if (slotBytes * q.planesPerBlock > static_cast<int64_t>(kMostSmem)) {
+        return false;
+    }
+    q.slotBytes = static_cast<int32_t>(slotBytes);
     q.stages = q.slotBytes * q.planesPerBlock <= 14 * 1024 ? 3 : 2;
     const int64_t resident = std::max<int64_t>(1, std::min<int64_t>(1024 / threads + 1, (200 << 10) / (ColumnsSmem(q) + 2048)));
     q.bandRows = PickBandRows(sh.hin, planeGroups, static_cast<int64_t>(NumSMs()) * resident);
@@ -761,21 +777,33 @@ bool LaunchColumns(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah
     while (q.lanesLog < 3 && (2 << q.lanesLog) <= perOutput) {
         ++q.lanesLog;
     }
-    const size_t smem = ColumnsSmem(q);
-    if (smem > 96 * 1024 || planeGroups > 0x7fffffff || bands > 65535) {
+    plan->k = k;
+    plan->threads = threads;
+    plan->bands = bands;
+    plan->planeGroups = planeGroups;
+    plan->smem = ColumnsSmem(q);
+    return plan->smem <= kMostSmem && planeGroups <= 0x7fffffff && bands <= 65535;
+}
+
+template <typename TIn, typename TOut>
+bool LaunchColumns(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, cudaStream_t s)
+{
+    ColumnsPlan plan;
+    if (!PlanColumns(static_cast<int>(sizeof(TIn)), sh, ah, aw, &plan)) {
         return false;
     }
-    const dim3 grid(static_cast<unsigned>(planeGroups), static_cast<unsigned>(bands));
+    const dim3 grid(static_cast<unsigned>(plan.planeGroups), static_cast<unsigned>(plan.bands));
     auto launch = [&](auto kernel) {
-        if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(smem)) != cudaSuccess) {
+        if (plan.smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                          static_cast<int>(plan.smem)) != cudaSuccess) {
             (void)cudaGetLastError();
             return false;
         }
-        kernel<<<grid, threads, smem, s>>>(static_cast<const TIn*>(go), static_cast<TOut*>(gi), planes, q, ah, aw);
+        kernel<<<grid, plan.threads, plan.smem, s>>>(static_cast<const TIn*>(go), static_cast<TOut*>(gi), sh.n * sh.c, plan.q,
+                                                     ah, aw);
         return true;
     };
-    switch (k) {
+    switch (plan.k) {
         case 1: return launch(BilinearBwdColumnsKernel<TIn, TOut, 1>);
         case 2: return launch(BilinearBwdColumnsKernel<TIn, TOut, 2>);
         case 4: return launch(BilinearBwdColumnsKernel<TIn, TOut, 4>);
@@ -805,15 +833,22 @@ int AxisBits(const BwdAxis& a)
     return bits;
 }
 
-template <typename T, typename TOut>
-bool LaunchNHWC(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, cudaStream_t s)
+// Launch shape of the NHWC kernel; false where it does not take the call.
+struct WalkPlan {
+    WalkShape q;
+    int32_t tiles, slices, bands;
+    int64_t imageGroups;
+    size_t smem;
+};
+bool PlanNHWC(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, WalkPlan* plan)
 {
-    constexpr int V = 16 / sizeof(T);
-    if (sh.c % V != 0 || !Aligned(go, 16) || !Aligned(gi, V * sizeof(TOut))) {
+    const int v = 16 / es;
+    if (sh.c % v != 0) {
         return false;
     }
-    WalkShape q{};
-    q.groups = static_cast<int32_t>(sh.c / V);
+    WalkShape& q = plan->q;
+    q = WalkShape{};
+    q.groups = static_cast<int32_t>(sh.c / v);
     q.hin = sh.hin;
     q.win = sh.win;
     q.hout = sh.hout;
@@ -826,21 +861,36 @@ bool LaunchNHWC(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah, c
     const int32_t tiles = static_cast<int32_t>(CeilDiv(sh.win, q.tileX));
     q.segPixels = MostRows(aw, q.tileX + 1);
     // a whole group per stage where that is some eighteen kilobytes at most
-    const int32_t rowBytes = std::max(1, q.images * q.segPixels * q.slice * 16);
+    const int64_t rowBytes = std::max<int64_t>(1, static_cast<int64_t>(q.images) * q.segPixels * q.slice * 16);
     const int32_t groupRows = static_cast<int32_t>(std::min(std::ceil(1.0f / ah.scale), static_cast<float>(sh.hout)));
-    q.stageRows = std::max(1, std::min(groupRows, 18 * 1024 / rowBytes));
+    q.stageRows = std::max(1, static_cast<int32_t>(std::min<int64_t>(groupRows, 18 * 1024 / rowBytes)));
     const int64_t imageGroups = CeilDiv(sh.n, q.images);
     const int64_t resident = std::max<int64_t>(1, std::min<int64_t>(4, (220 << 10) / (WalkSmem(q) + 2048)));
     q.bandRows = PickBandRows(sh.hin, imageGroups * tiles * slices, static_cast<int64_t>(NumSMs()) * resident);
     const int32_t bands = static_cast<int32_t>(CeilDiv(sh.hin, q.bandRows));
     q.dRowCap = MostRows(ah, q.bandRows + 1);
-    const size_t smem = WalkSmem(q);
-    if (smem > 112 * 1024 || imageGroups > 65535 || bands > 65535) {
+    plan->tiles = tiles;
+    plan->slices = slices;
+    plan->bands = bands;
+    plan->imageGroups = imageGroups;
+    plan->smem = WalkSmem(q);
+    return plan->smem <= 112 * 1024 && imageGroups <= 65535 && bands <= 65535;
+}
+
+template <typename T, typename TOut>
+bool LaunchNHWC(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, cudaStream_t s)
+{
+    constexpr int V = 16 / sizeof(T);
+    WalkPlan plan;
+    if (!Aligned(go, 16) || !Aligned(gi, V * sizeof(TOut)) || !PlanNHWC(static_cast<int>(sizeof(T)), sh, ah, aw, &plan)) {
         return false;
     }
+    const WalkShape& q = plan.q;
+    const size_t smem = plan.smem;
     const int mant = std::is_same<T, __half>::value ? 11 : 8; // significand bits of T
     const bool fuse = sizeof(T) == 2 && AxisBits(ah) + AxisBits(aw) + mant <= 24;
-    const dim3 grid(static_cast<unsigned>(tiles * slices), static_cast<unsigned>(imageGroups), static_cast<unsigned>(bands));
+    const dim3 grid(static_cast<unsigned>(plan.tiles * plan.slices), static_cast<unsigned>(plan.imageGroups),
+                    static_cast<unsigned>(plan.bands));
     const int32_t threads = static_cast<int32_t>(CeilDiv(q.images * q.tileX * q.slice, 32)) * 32 + 32;
     auto launch = [&](auto kernel) {
         if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -865,14 +915,46 @@ bool Launch(Layout lay, const void* go, void* gi, const Shape4& sh, const BwdAxi
     return lay == kNCHW ? LaunchColumns<TIn, TOut>(go, gi, sh, ah, aw, s) : LaunchNHWC<TIn, TOut>(go, gi, sh, ah, aw, s);
 }
 
+// An up-scale whose groups follow from the scale, at extents for which MostRows holds.
+bool Walkable(const BwdAxis& a)
+{
+    return a.scale > 0.0f && a.scale <= 1.0f && a.out <= kMostExtent && a.last < kMostExtent && !Overshoots(a);
+}
+
 } // namespace
+
+bool DebugBilinearBwdWalk(int es, Layout lay, Shape4 sh, AxisGeom gh, AxisGeom gw, bool halfPixel, int64_t values[8])
+{
+    const BwdAxis ah = MakeAxis(gh, halfPixel), aw = MakeAxis(gw, halfPixel);
+    if (!Walkable(ah) || !Walkable(aw)) {
+        return false;
+    }
+    if (lay == kNCHW) {
+        ColumnsPlan p;
+        if (!PlanColumns(es, sh, ah, aw, &p)) {
+            return false;
+        }
+        const int64_t stage = (p.q.slotBytes - 15) / (sh.wout * static_cast<int64_t>(es));
+        const int64_t v[8] = {p.q.bandRows, p.q.dRowCap, p.q.stageGroups, stage, p.k, p.q.planesPerBlock, p.bands,
+                              static_cast<int64_t>(p.smem)};
+        std::copy(v, v + 8, values);
+        return true;
+    }
+    WalkPlan p;
+    if (!PlanNHWC(es, sh, ah, aw, &p)) {
+        return false;
+    }
+    const int64_t v[8] = {p.q.bandRows, p.q.dRowCap, p.q.tileX, p.q.segPixels, p.slices, p.q.images, p.bands,
+                          static_cast<int64_t>(p.smem)};
+    std::copy(v, v + 8, values);
+    return true;
+}
 
 bool BilinearBwdWalk(Dt dtIn, Dt dtOut, Layout lay, const void* go, void* gi, Shape4 sh, AxisGeom gh, AxisGeom gw,
                      bool halfPixel, cudaStream_t s)
 {
     const BwdAxis ah = MakeAxis(gh, halfPixel), aw = MakeAxis(gw, halfPixel);
-    if (!(gh.scale > 0.0f && gh.scale <= 1.0f && gw.scale > 0.0f && gw.scale <= 1.0f) || Overshoots(ah) ||
-        Overshoots(aw)) {
+    if (!Walkable(ah) || !Walkable(aw)) {
         return false;
     }
     if (dtIn == dtOut) {

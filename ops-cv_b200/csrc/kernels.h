@@ -155,6 +155,8 @@ cudaError_t BilinearBwdGather(Dt dtIn, Dt dtOut, Layout lay, const void* go, voi
 // without a launch (down-scales, user scales that run past the input, rows too long for a block).
 bool BilinearBwdWalk(Dt dtIn, Dt dtOut, Layout lay, const void* go, void* gi, Shape4 sh, AxisGeom gh, AxisGeom gw,
                      bool halfPixel, cudaStream_t s);
+// The launch shape behind it (values as documented at opscvDebugPlan); false where it does not take the call.
+bool DebugBilinearBwdWalk(int elemSize, Layout lay, Shape4 sh, AxisGeom gh, AxisGeom gw, bool halfPixel, int64_t values[8]);
 bool BilinearBwdTakesPitch(Dt dtIn, Dt dtOut, Layout lay, const void* go, const void* gi, Shape4 sh,
                            const BilinearPlan& plan, const ViewStrides& grads);
 // Scatter backward with fp32 atomics into `acc` (fp32, N*C*hin*win, zeroed by this call). If dtOut is fp32 the

@@ -1,0 +1,72 @@
+"""The bounds that launch shapes are sized by, against a restatement of the kernels' index arithmetic: a block's shared memory
+holds what its rows, columns or windows can ask for. Host arithmetic only (opscvDebugPlan), no GPU."""
+import random
+
+import numpy as np
+import pytest
+
+F = np.float32
+
+
+def bilinear_backward_scale(n_in, n_out, align, user):
+    if align:
+        return F(n_in - 1) / F(n_out - 1) if n_out > 1 else F(0)
+    return F(1) / F(user) if user > 0 else F(n_in) / F(n_out)
+
+
+def group_starts(n_in, n_out, align, user=0.0):
+    """starts[y] = first grads index whose lower tap is y or more, for y = 0 .. n_in (fp32, each operation rounded)."""
+    off = F(0) if align else F(0.5)
+    scale = bilinear_backward_scale(n_in, n_out, align, user)
+    src = (np.arange(n_out, dtype=np.int64).astype(F) + off) * scale - off
+    lo = np.minimum(np.floor(np.maximum(src, F(0))).astype(np.int64), n_in - 1)
+    return np.searchsorted(lo, np.arange(n_in + 1))
+
+
+def most(starts, first, count):
+    """Most grads indices in the groups first .. first + count - 1, over the given first groups (negative ones are empty)."""
+    n_in = len(starts) - 1
+    lo = starts[np.clip(first, 0, n_in)]
+    hi = starts[np.clip(np.asarray(first) + count, 0, n_in)]
+    return int((hi - lo).max())
+
+
+def check_walk(ops, fmt, elem, n, c, hi, wi, ho, wo, align):
+    plan = ops.debug_plan("bilinear_backward_walk", elem, (n, c, hi, wi, ho, wo), fmt, align)
+    if plan is None:
+        return False
+    band, band_cap, group, group_cap, _, _, _, smem = plan
+    assert 0 < smem <= 112 * 1024
+    rows = group_starts(hi, ho, align)
+    assert most(rows, np.arange(0, hi, band) - 1, band + 1) <= band_cap
+    if fmt == "NCHW":  # a stage: any run of groups that starts a multiple of them from a band's first
+        assert most(rows, np.arange(-1, hi), group) <= group_cap
+    else:
+        assert most(group_starts(wi, wo, align), np.arange(0, wi, group) - 1, group + 1) <= group_cap
+    return True
+
+
+# long rows and columns: from 2^22 on an index and its half are no longer exact, from 2^24 on indices share a position
+LONG = [("NHWC", 4, 4, 1, 11358413, 1, 27879496), ("NHWC", 2, 8, 1, 9000001, 1, 16777216), ("NHWC", 4, 8, 1, 3000001, 1, 8388607),
+        ("NHWC", 4, 4, 4000003, 1, 16777215, 2), ("NHWC", 4, 4, 5000000, 1, 20000001, 2), ("NCHW", 4, 1, 5000000, 1, 16777216, 2),
+        ("NCHW", 4, 1, 4000001, 2, 33000001, 3), ("NCHW", 2, 1, 8000000, 2, 16777215, 3)]
+
+
+@pytest.mark.parametrize("fmt,elem,c,hi,wi,ho,wo", LONG)
+@pytest.mark.parametrize("align", [False, True])
+def test_bilinear_walk_of_long_axes(ops, fmt, elem, c, hi, wi, ho, wo, align):
+    taken = check_walk(ops, fmt, elem, 1, c, hi, wi, ho, wo, align)
+    if max(ho, wo) > 2 ** 24:
+        assert not taken
+
+
+def test_bilinear_walk_of_random_sizes(ops):
+    rng = random.Random(5)
+    taken = 0
+    for _ in range(1500):
+        fmt, elem = rng.choice(["NCHW", "NHWC"]), rng.choice([2, 4])
+        hi, wi = int(2 ** rng.uniform(0, 10)), int(2 ** rng.uniform(0, 10))
+        ho, wo = int(hi * 2 ** rng.uniform(0, 4)), int(wi * 2 ** rng.uniform(0, 4))
+        n, c = rng.randint(1, 20), rng.choice([1, 3, 8, 48, 264])
+        taken += check_walk(ops, fmt, elem, n, c, hi, wi, ho, wo, rng.random() < 0.5)
+    assert taken > 500
