@@ -811,26 +811,19 @@ bool LaunchColumns(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah
     }
 }
 
-// Significant bits of a weight (0 for zero).
-int WeightBits(float w)
-{
-    int exponent = 0;
-    const float m = std::frexp(std::fabs(w), &exponent); // m in [0.5, 1)
-    uint32_t digits = static_cast<uint32_t>(std::ldexp(m, 24));
-    int bits = w == 0.0f ? 0 : 24;
-    for (; bits > 0 && (digits & 1u) == 0; digits >>= 1) {
-        --bits;
-    }
-    return bits;
-}
+// Most significant bits that a weight of this axis can have. With scale = odd * 2^e a position is a multiple of 2^e, or of
+// 2^(e - 1) with the half-pixel offset (rounding moves it to a coarser multiple), and so are a weight and its complement.
+// From the scale alone: a look at every index took 193 us per axis and call at 4096 indices and a scale of two.
 int AxisBits(const BwdAxis& a)
 {
-    int bits = 0;
-    for (int32_t d = 0; d < a.out && bits < 24; ++d) {
-        const float delta = std::fmin(std::fmax(BwdPosition(a, d) - static_cast<float>(BwdLower(a, d)), 0.0f), 1.0f);
-        bits = std::max({bits, WeightBits(delta), WeightBits(1.0f - delta)});
+    int exponent = 0;
+    const float m = std::frexp(a.scale, &exponent); // scale = m * 2^exponent, m in [0.5, 1)
+    uint32_t digits = static_cast<uint32_t>(std::ldexp(m, 24));
+    int e = exponent - 24;
+    for (; (digits & 1u) == 0; digits >>= 1) { // scale is not zero
+        ++e;
     }
-    return bits;
+    return std::max(1, std::min(24, (a.offset > 0.0f ? 1 : 0) - e));
 }
 
 // Launch shape of the NHWC kernel; false where it does not take the call.
@@ -944,7 +937,7 @@ bool DebugBilinearBwdWalk(int es, Layout lay, Shape4 sh, AxisGeom gh, AxisGeom g
     if (!PlanNHWC(es, sh, ah, aw, &p)) {
         return false;
     }
-    const int64_t v[8] = {p.q.bandRows, p.q.dRowCap, p.q.tileX, p.q.segPixels, p.slices, p.q.images, p.bands,
+    const int64_t v[8] = {p.q.bandRows, p.q.dRowCap, p.q.tileX, p.q.segPixels, p.slices, p.q.images, AxisBits(ah) + AxisBits(aw),
                           static_cast<int64_t>(p.smem)};
     std::copy(v, v + 8, values);
     return true;

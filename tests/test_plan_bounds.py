@@ -1,6 +1,7 @@
 """The bounds that launch shapes are sized by, against a restatement of the kernels' index arithmetic: a block's shared memory
 holds what its rows, columns or windows can ask for. Host arithmetic only (opscvDebugPlan), no GPU."""
 import random
+import time
 
 import numpy as np
 import pytest
@@ -70,3 +71,40 @@ def test_bilinear_walk_of_random_sizes(ops):
         n, c = rng.randint(1, 20), rng.choice([1, 3, 8, 48, 264])
         taken += check_walk(ops, fmt, elem, n, c, hi, wi, ho, wo, rng.random() < 0.5)
     assert taken > 500
+
+
+def weight_bits(n_in, n_out, align):
+    """Significant bits of the widest weight of an axis, looked up index by index."""
+    off = F(0) if align else F(0.5)
+    scale = bilinear_backward_scale(n_in, n_out, align, 0.0)
+    src = np.maximum((np.arange(n_out).astype(F) + off) * scale - off, F(0))
+    delta = src - np.minimum(np.floor(src), F(n_in - 1))
+    bits = 0
+    for w in np.unique(np.concatenate([delta, F(1) - delta])):
+        digits = int(float(w) * 2 ** 60)
+        bits = max(bits, digits.bit_length() - (digits & -digits).bit_length() + 1 if digits else 0)
+    return bits
+
+
+def test_weight_bits_of_the_nhwc_walk(ops):
+    """Products with weights of few bits are added with one rounding, which is exact only if the bits are not underrated."""
+    rng = random.Random(6)
+    for k in range(300):
+        align = rng.random() < 0.5
+        hi, wi = rng.randint(1, 90), rng.randint(1, 90)
+        ho, wo = (hi * 2, wi * 4) if k % 3 == 0 else (rng.randint(hi, 4 * hi), rng.randint(wi, 4 * wi))
+        plan = ops.debug_plan("bilinear_backward_walk", 2, (1, 8, hi, wi, ho, wo), "NHWC", align)
+        if plan is not None:
+            assert weight_bits(hi, ho, align) + weight_bits(wi, wo, align) <= plan[6]
+    for size, bits in (((1, 8, 64, 64, 128, 128), 4), ((1, 8, 64, 48, 256, 96), 5), ((1, 8, 30, 30, 80, 80), 8)):
+        assert ops.debug_plan("bilinear_backward_walk", 2, size, "NHWC")[6] == bits
+
+
+def test_planning_does_not_grow_with_the_extent(ops):
+    """A launch shape is found on the host in every call: microseconds, not one look at every index."""
+    best = 1.0
+    for _ in range(20):
+        start = time.perf_counter()
+        ops.debug_plan("bilinear_backward_walk", 2, (1, 8, 4096, 4096, 8192, 8192), "NHWC")
+        best = min(best, time.perf_counter() - start)
+    assert best < 3e-4
