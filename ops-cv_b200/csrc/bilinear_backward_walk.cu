@@ -710,12 +710,14 @@ int32_t MostRows(const BwdAxis& a, int32_t groups)
 }
 
 // Rows of a band: the blocks of all bands run in waves of `slots` resident blocks, and a band costs its own rows, one
-// more group of grads rows and its start (about two rows).
+// more group of grads rows and its start (about two rows). Tall planes are cut into more than 64 bands while a band keeps
+// eight rows: a few images of one would leave most SMs idle and each block a long walk (fp32 NHWC 1x100000x4x8 <- 250000x9:
+// 2663 us in 64 bands).
 int32_t PickBandRows(int32_t rows, int64_t blocksPerBand, int64_t slots)
 {
     int32_t best = rows;
     double bestCost = 1e30;
-    for (int32_t bands = 1; bands <= std::min(rows, 64); ++bands) {
+    for (int32_t bands = 1; bands <= rows && (bands <= 64 || rows / bands >= 8); bands += bands < 64 ? 1 : bands / 16) {
         const int32_t r = static_cast<int32_t>(CeilDiv(rows, bands));
         const double cost = static_cast<double>(CeilDiv(blocksPerBand * CeilDiv(rows, r), slots)) * (r + 3);
         if (cost < bestCost) {
@@ -829,7 +831,7 @@ int AxisBits(const BwdAxis& a)
 // Launch shape of the NHWC kernel; false where it does not take the call.
 struct WalkPlan {
     WalkShape q;
-    int32_t tiles, slices, bands;
+    int32_t tiles, slices, threads, bands;
     int64_t imageGroups;
     size_t smem;
 };
@@ -851,6 +853,11 @@ bool PlanNHWC(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, Wa
     q.tileX = std::min(sh.win, kWalkThreads / q.slice);
     q.tileX = static_cast<int32_t>(CeilDiv(sh.win, CeilDiv(sh.win, q.tileX))); // equal tiles
     q.images = static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(sh.n, kWalkThreads / (q.tileX * q.slice))));
+    // A single narrow image leaves a block a warp: on a tall one the gather kernel, with a thread per element, is faster
+    // (fp32 1x100000x4x8 <- 250000x9: 104 us against 239, 10000 rows: 25 against 34 us, 500 rows: 21 us both).
+    if (q.images * q.tileX * q.slice <= 32 && sh.hin > 1024) {
+        return false;
+    }
     const int32_t tiles = static_cast<int32_t>(CeilDiv(sh.win, q.tileX));
     q.segPixels = MostRows(aw, q.tileX + 1);
     // a whole group per stage where that is some eighteen kilobytes at most
@@ -858,12 +865,14 @@ bool PlanNHWC(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, Wa
     const int32_t groupRows = static_cast<int32_t>(std::min(std::ceil(1.0f / ah.scale), static_cast<float>(sh.hout)));
     q.stageRows = std::max(1, static_cast<int32_t>(std::min<int64_t>(groupRows, 18 * 1024 / rowBytes)));
     const int64_t imageGroups = CeilDiv(sh.n, q.images);
-    const int64_t resident = std::max<int64_t>(1, std::min<int64_t>(4, (220 << 10) / (WalkSmem(q) + 2048)));
+    const int32_t threads = static_cast<int32_t>(CeilDiv(q.images * q.tileX * q.slice, 32)) * 32 + 32; // and the copying warp
+    const int64_t resident = std::max<int64_t>(1, std::min<int64_t>(1024 / threads, (220 << 10) / (WalkSmem(q) + 2048)));
     q.bandRows = PickBandRows(sh.hin, imageGroups * tiles * slices, static_cast<int64_t>(NumSMs()) * resident);
     const int32_t bands = static_cast<int32_t>(CeilDiv(sh.hin, q.bandRows));
     q.dRowCap = MostRows(ah, q.bandRows + 1);
     plan->tiles = tiles;
     plan->slices = slices;
+    plan->threads = threads;
     plan->bands = bands;
     plan->imageGroups = imageGroups;
     plan->smem = WalkSmem(q);
@@ -884,7 +893,7 @@ bool LaunchNHWC(const void* go, void* gi, const Shape4& sh, const BwdAxis& ah, c
     const bool fuse = sizeof(T) == 2 && AxisBits(ah) + AxisBits(aw) + mant <= 24;
     const dim3 grid(static_cast<unsigned>(plan.tiles * plan.slices), static_cast<unsigned>(plan.imageGroups),
                     static_cast<unsigned>(plan.bands));
-    const int32_t threads = static_cast<int32_t>(CeilDiv(q.images * q.tileX * q.slice, 32)) * 32 + 32;
+    const int32_t threads = plan.threads;
     auto launch = [&](auto kernel) {
         if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      static_cast<int>(smem)) != cudaSuccess) {

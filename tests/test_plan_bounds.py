@@ -108,3 +108,11 @@ def test_planning_does_not_grow_with_the_extent(ops):
         ops.debug_plan("bilinear_backward_walk", 2, (1, 8, 4096, 4096, 8192, 8192), "NHWC")
         best = min(best, time.perf_counter() - start)
     assert best < 3e-4
+
+
+@pytest.mark.parametrize("fmt,c,hi,wi,ho,wo", [("NHWC", 64, 100000, 4, 250000, 9), ("NCHW", 1, 100000, 16, 250000, 40),
+                                               ("NHWC", 48, 16000, 16, 32000, 32)])
+def test_bilinear_walk_of_one_tall_plane_fills_the_device(ops, fmt, c, hi, wi, ho, wo):
+    plan = ops.debug_plan("bilinear_backward_walk", 4, (1, c, hi, wi, ho, wo), fmt)
+    assert plan is not None and -(-hi // plan[0]) >= 148  # bands; B200 has 148 SMs
+    assert check_walk(ops, fmt, 4, 1, c, hi, wi, ho, wo, False)
