@@ -360,7 +360,9 @@ ACLNN_API aclnnStatus opscvDebugAxisTable(int32_t kind, int64_t inSize, int64_t 
  * kind 0, UpsampleBilinear2dBackward by row walks: {grad_input rows per band, most grads rows of a band, groups per stage
  *   (NCHW) or columns per tile (NHWC), most grads rows of a stage (NCHW) or grads columns of a tile (NHWC), columns per
  *   thread (NCHW) or channel slices (NHWC), planes or images per block, bands (NCHW) or most significant bits of a product
- *   of two weights (NHWC), shared-memory bytes}. */
+ *   of two weights (NHWC), shared-memory bytes};
+ * kind 1, UpsampleBicubic2dBackward by row walks: {grad_input rows per band, most grads rows of a band, most grad_input rows
+ *   that one grads row feeds, 0, 0, 0, bands, shared-memory bytes}. */
 ACLNN_API aclnnStatus opscvDebugPlan(int32_t kind, int32_t elemSize, aclFormat format, const int64_t sizes[6],
                                      int32_t alignCorners, const double scales[2], int32_t* taken, int64_t values[8]);
 

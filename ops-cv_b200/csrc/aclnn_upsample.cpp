@@ -1998,6 +1998,12 @@ aclnnStatus opscvDebugPlan(int32_t kind, int32_t elemSize, aclFormat format, con
             *taken = DebugBilinearBwdWalk(elemSize, lay, sh, gh, gw, !align, values) ? 1 : 0;
             return ACLNN_SUCCESS;
         }
+        case 1: {
+            const BicubicGradScale bh = MakeBicubicGradScale(in.h, out.h, align, static_cast<float>(scales[0]));
+            const BicubicGradScale bw = MakeBicubicGradScale(in.w, out.w, align, static_cast<float>(scales[1]));
+            *taken = DebugBicubic2dBwd(lay, sh, bh.scale, bw.scale, bh.inverse, bw.inverse, align, values) ? 1 : 0;
+            return ACLNN_SUCCESS;
+        }
         default: return Fail(ACLNN_ERR_PARAM_INVALID, "%s: unknown kind %d", api, kind);
     }
 }

@@ -201,6 +201,8 @@ cudaError_t BicubicAABwdAtomic(Dt dt, const void* go, void* gi, float* acc, Shap
 // source positions (equal extents are a copy made by the host layer). The backward is a gather in a fixed order.
 cudaError_t Bicubic2dFwd(Dt dt, Layout lay, const void* x, void* y, Shape4 sh, float scaleH, float scaleW,
                          bool halfPixel, int32_t schedule, cudaStream_t s);
+// The row walk's launch shape (values as documented at opscvDebugPlan); false where another kernel serves the call.
+bool DebugBicubic2dBwd(Layout lay, Shape4 sh, float scaleH, float scaleW, float invH, float invW, bool align, int64_t values[8]);
 cudaError_t Bicubic2dBwd(Dt dt, Layout lay, const void* go, void* gi, Shape4 sh, float scaleH, float scaleW,
                          float invH, float invW, bool align, cudaStream_t s);
 

@@ -773,18 +773,19 @@ __global__ void __launch_bounds__(kWalkThreads, (NHWC && K > 14) ? 3 : ((NHWC ||
         rowEnd[r] = h;
     }
     __syncthreads();
-    int32_t hLo = rowStart[0], hHi = rowEnd[0];
-    for (int32_t r = 1; r < y1 - y0; ++r) {
-        hLo = min(hLo, rowStart[r]);
-        hHi = max(hHi, rowEnd[r]);
-    }
-    hHi = min(hHi, hLo + ws.maxRows);
+    // starts and ends grow with the row
+    const int32_t hLo = rowStart[0], hHi = min(rowEnd[y1 - 1 - y0], hLo + ws.maxRows);
     for (int32_t h = hLo + threadIdx.x; h < hHi; h += blockDim.x) {
         const float rh = BwdSrc(g.scaleH, h, g.align);
         WalkRecord w{};
-        int32_t y = yi0;
-        while (y < yi1 && rowEnd[y - y0] <= h) {
-            ++y;
+        int32_t y = yi0, yEnd = yi1; // the first interior row whose walk has not ended
+        while (y < yEnd) {
+            const int32_t mid = (y + yEnd) >> 1;
+            if (rowEnd[mid - y0] <= h) {
+                y = mid + 1;
+            } else {
+                yEnd = mid;
+            }
         }
         w.first = y;
 #pragma unroll
@@ -1510,6 +1511,122 @@ dim3 RowGrid(int64_t rows, int64_t inner)
     return dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy), 1);
 }
 
+// ---- launch shapes of the general backward ------------------------------------------------------------------------
+struct ListLaunch {
+    int32_t colsPB, entries, x, y;
+    size_t smem;
+};
+ListLaunch PlanBwdList(const BicubicGeom& g, bool borderOnly)
+{
+    const int64_t inner = static_cast<int64_t>(g.win) * g.chan;
+    const double perScale = g.invW > 0.0f ? static_cast<double>(g.invW) : 1.0;
+    // Columns of one list: the grads columns of an interior walk; a first or last column takes those within two and a
+    // half source pixels. Lists that would not fit make their thread fall back to the uncached walk, so the bound only
+    // has to be good, not safe; a single-column image (every grads column is a tap) always falls back.
+    const int64_t maxW = static_cast<int64_t>(std::ceil(4.0 * perScale)) + 4;
+    const int64_t positions = borderOnly ? 2LL * g.chan : inner;
+    ListLaunch l;
+    l.colsPB = static_cast<int32_t>(std::min<int64_t>(kListThreads, positions));
+    const int rowsPB = kListThreads / l.colsPB;
+    const int64_t cap = 96 * 1024 / (kListBytes * kListThreads);
+    l.entries = static_cast<int32_t>(std::max<int64_t>(4, std::min<int64_t>(maxW, cap)));
+    l.smem = static_cast<size_t>(l.entries) * kListThreads * kListBytes;
+    l.x = static_cast<int32_t>(CeilDiv(positions, l.colsPB));
+    const int64_t gyCap = std::max<int64_t>(static_cast<int64_t>(NumSMs()) * 32 / l.x, 1);
+    l.y = static_cast<int32_t>(std::min<int64_t>(std::min<int64_t>(CeilDiv(g.rows, rowsPB), gyCap), 65535));
+    return l;
+}
+
+// Interior columns by the row walk, the two border columns apart; false where the list kernel serves the call.
+struct BwdWalkPlan {
+    WalkShape ws;
+    int64_t bands, blocks;
+    size_t smem;
+};
+bool PlanBwdWalk(const BicubicGeom& g, BwdWalkPlan* plan)
+{
+    constexpr size_t kMostSmem = 48 * 1024; // four blocks per SM
+    const int64_t inner = static_cast<int64_t>(g.win) * g.chan;
+    const double perScale = g.invW > 0.0f ? static_cast<double>(g.invW) : 1.0;
+    // columns of the longest interior walk: 4 / scale within two source pixels either side, one more for rounding
+    const int64_t walk = static_cast<int64_t>(std::ceil(4.0 * perScale)) + 1;
+    // The bound on open rows holds while the start of a walk (from the inverse scale) and its end (from the scale) speak of
+    // the same positions: a quarter of a source pixel for the two scales, another quarter for the rounding of positions up to
+    // 2^20 rows and 2^22 grads rows. The last row's walk runs to the end of the grads, which a user scale can put anywhere.
+    const double rowsPerRow = g.invH;
+    const double drift = g.invH > 0.0f && g.scaleH > 0.0f ? std::fabs(static_cast<double>(g.scaleH) * g.invH - 1.0) *
+                                                                (static_cast<double>(g.hin) + 2.0 * rowsPerRow + 4.0)
+                                                          : 1.0;
+    if (walk > 17 || g.win <= 2 || g.hin <= 2 || g.hin > (1 << 20) || g.hout > (1 << 22) || !(drift < 0.25) ||
+        !(8.0 * rowsPerRow + 8.0 < kWalkMaxRows) ||
+        !(static_cast<double>(g.hout) <= (static_cast<double>(g.hin) + 2.0) * rowsPerRow + 2.0)) {
+        return false;
+    }
+    const int64_t planes = g.rows / g.hin;
+    const ListLaunch l = PlanBwdList(g, true);
+    WalkShape& ws = plan->ws;
+    ws = WalkShape{};
+    ws.positions = planes * (inner - 2LL * g.chan);
+    const int64_t gx = CeilDiv(ws.positions, kWalkThreads);
+    // grads rows of a band: four source pixels beyond it, and the rounding of its ends
+    auto bandReads = [&](int64_t band) { return static_cast<int64_t>((static_cast<double>(band) + 5.0) * rowsPerRow) + 4; };
+    // shared memory: a record per grads row, start and end of every row of the band (which are what fills it where a band
+    // reads few rows, in a strong vertical down-scale)
+    auto bandSmem = [&](int64_t band) { return static_cast<size_t>(bandReads(band)) * sizeof(WalkRecord) + static_cast<size_t>(band) * 8; };
+    // Bands: every band re-reads four source pixels' worth of grads rows; fewer than five blocks per SM leave each of them
+    // waiting on its own loads (about 0.25 us a row), more share the issue slots (about 0.06 us a row). A tall plane needs
+    // more than 256 of them for its records to fit (fp32 1x40000x64 <- 160000x256: 247 us, by lists 1352).
+    double bestTime = 0.0;
+    for (int64_t b = 1; b <= g.hin && (b <= 256 || g.hin / b >= 16); b += b < 256 ? 1 : b / 16) {
+        const int64_t band = CeilDiv(g.hin, b);
+        const int64_t reads = bandReads(band);
+        if (reads > kWalkMaxRows || bandSmem(band) > kMostSmem) {
+            continue;
+        }
+        const double k = static_cast<double>(CeilDiv(gx * CeilDiv(g.hin, band), NumSMs()));
+        const double time = (static_cast<double>(reads) + 8.0) * std::max(0.25 * std::ceil(k / 5.0), 0.06 * k);
+        if (ws.bandRows == 0 || time < bestTime * 0.98) {
+            ws.bandRows = static_cast<int32_t>(band);
+            bestTime = time;
+        }
+    }
+    if (ws.bandRows == 0) {
+        return false;
+    }
+    plan->bands = CeilDiv(g.hin, ws.bandRows);
+    plan->blocks = gx * plan->bands + static_cast<int64_t>(l.x) * l.y;
+    if (plan->blocks > INT32_MAX) {
+        return false;
+    }
+    ws.maxRows = static_cast<int32_t>(bandReads(ws.bandRows));
+    ws.walkX = static_cast<int32_t>(gx);
+    ws.listX = l.x;
+    ws.listY = l.y;
+    ws.listCols = l.colsPB;
+    ws.listMax = l.entries;
+    plan->smem = std::max(l.smem, bandSmem(ws.bandRows));
+    return true;
+}
+
+BicubicGeom BwdGeom(Layout lay, const Shape4& sh, float scaleH, float scaleW, float invH, float invW, bool align)
+{
+    const bool nhwc = lay == kNHWC;
+    BicubicGeom g;
+    g.rows = (nhwc ? sh.n : sh.n * sh.c) * sh.hin;
+    g.hin = sh.hin;
+    g.win = sh.win;
+    g.hout = sh.hout;
+    g.wout = sh.wout;
+    g.chan = nhwc ? static_cast<int32_t>(sh.c) : 1;
+    g.scaleH = scaleH;
+    g.scaleW = scaleW;
+    g.invH = invH;
+    g.invW = invW;
+    g.align = align ? 1 : 0;
+    g.schedule = 0;
+    return g;
+}
+
 } // namespace
 
 cudaError_t Bicubic2dFwd(Dt dt, Layout lay, const void* x, void* y, Shape4 sh, float scaleH, float scaleW,
@@ -1680,56 +1797,11 @@ cudaError_t Bicubic2dBwd(Dt dt, Layout lay, const void* go, void* gi, Shape4 sh,
                          float invH, float invW, bool align, cudaStream_t s)
 {
     const bool nhwc = lay == kNHWC;
-    BicubicGeom g;
-    g.rows = (nhwc ? sh.n : sh.n * sh.c) * sh.hin;
-    g.hin = sh.hin;
-    g.win = sh.win;
-    g.hout = sh.hout;
-    g.wout = sh.wout;
-    g.chan = nhwc ? static_cast<int32_t>(sh.c) : 1;
-    g.scaleH = scaleH;
-    g.scaleW = scaleW;
-    g.invH = invH;
-    g.invW = invW;
-    g.align = align ? 1 : 0;
-    g.schedule = 0;
-    const int64_t inner = static_cast<int64_t>(g.win) * g.chan;
+    const BicubicGeom g = BwdGeom(lay, sh, scaleH, scaleW, invH, invW, align);
     const double perScale = invW > 0.0f ? static_cast<double>(invW) : 1.0;
-    // columns of the longest interior walk: 4 / scale within two source pixels either side, one more for rounding
-    const int64_t walk = static_cast<int64_t>(std::ceil(4.0 * perScale)) + 1;
-    // Interior columns by the row walk, the two border columns apart. The walk's bound on open rows holds while the
-    // start of a walk (from the inverse scale) and its end (from the scale) speak of the same positions; the last row's
-    // walk runs to the end of the grads, which a user scale can put anywhere.
-    const double rowsPerRow = invH;
-    const double drift = invH > 0.0f && scaleH > 0.0f ? std::fabs(static_cast<double>(scaleH) * invH - 1.0) *
-                                                            (static_cast<double>(sh.hin) + 2.0 * rowsPerRow + 4.0)
-                                                      : 1.0;
-    const bool split = walk <= 17 && sh.win > 2 && sh.hin > 2 && drift < 0.25 && 8.0 * rowsPerRow + 8.0 < kWalkMaxRows &&
-                       static_cast<double>(sh.hout) <= (static_cast<double>(sh.hin) + 2.0) * rowsPerRow + 2.0;
-    // Columns of one list: the grads columns of an interior walk; a first or last column takes those within two and a
-    // half source pixels. Lists that would not fit make their thread fall back to the uncached walk, so the bound only
-    // has to be good, not safe; a single-column image (every grads column is a tap) always falls back.
-    const int64_t maxW = static_cast<int64_t>(std::ceil(4.0 * perScale)) + 4;
     cudaError_t err = cudaSuccess;
-    struct ListLaunch {
-        int32_t colsPB, entries, x, y;
-        size_t smem;
-    };
-    auto planList = [&](bool borderOnly) {
-        const int64_t positions = borderOnly ? 2LL * g.chan : inner;
-        ListLaunch l;
-        l.colsPB = static_cast<int32_t>(std::min<int64_t>(kListThreads, positions));
-        const int rowsPB = kListThreads / l.colsPB;
-        const int64_t cap = 96 * 1024 / (kListBytes * kListThreads);
-        l.entries = static_cast<int32_t>(std::max<int64_t>(4, std::min<int64_t>(maxW, cap)));
-        l.smem = static_cast<size_t>(l.entries) * kListThreads * kListBytes;
-        l.x = static_cast<int32_t>(CeilDiv(positions, l.colsPB));
-        const int64_t gyCap = std::max<int64_t>(static_cast<int64_t>(NumSMs()) * 32 / l.x, 1);
-        l.y = static_cast<int32_t>(std::min<int64_t>(std::min<int64_t>(CeilDiv(g.rows, rowsPB), gyCap), 65535));
-        return l;
-    };
     auto launchList = [&]() {
-        const ListLaunch l = planList(false);
+        const ListLaunch l = PlanBwdList(g, false);
         OPSCV_DISPATCH_DT(dt, T, {
             auto kernel = nhwc ? Bicubic2dBwdListKernel<T, true> : Bicubic2dBwdListKernel<T, false>;
             if (l.smem > 48 * 1024) {
@@ -1769,56 +1841,21 @@ cudaError_t Bicubic2dBwd(Dt dt, Layout lay, const void* go, void* gi, Shape4 sh,
         CountLaunch();
         return cudaGetLastError();
     }
-    if (!split) {
+    BwdWalkPlan plan;
+    if (!PlanBwdWalk(g, &plan)) {
         launchList();
         return err != cudaSuccess ? err : cudaGetLastError();
     }
-    const int64_t planes = g.rows / g.hin;
-    const ListLaunch l = planList(true);
-    WalkShape ws{};
-    ws.positions = planes * (inner - 2LL * g.chan);
-    const int64_t gx = CeilDiv(ws.positions, kWalkThreads);
-    // grads rows of a band: four source pixels beyond it, and the rounding of its ends
-    auto bandReads = [&](int64_t band) { return static_cast<int64_t>((static_cast<double>(band) + 5.0) * rowsPerRow) + 4; };
-    // Bands: every band re-reads four source pixels' worth of grads rows; fewer than five blocks per SM leave each of them
-    // waiting on its own loads (about 0.25 us a row), more share the issue slots (about 0.06 us a row).
-    double bestTime = 0.0;
-    for (int64_t b = 1; b <= sh.hin && b <= 256; ++b) {
-        const int64_t band = CeilDiv(sh.hin, b);
-        const int64_t reads = bandReads(band);
-        if (reads > kWalkMaxRows) {
-            continue;
-        }
-        const double k = static_cast<double>(CeilDiv(gx * CeilDiv(sh.hin, band), NumSMs()));
-        const double time = (static_cast<double>(reads) + 8.0) * std::max(0.25 * std::ceil(k / 5.0), 0.06 * k);
-        if (ws.bandRows == 0 || time < bestTime * 0.98) {
-            ws.bandRows = static_cast<int32_t>(band);
-            bestTime = time;
-        }
-    }
-    const int64_t bands = ws.bandRows > 0 ? CeilDiv(sh.hin, ws.bandRows) : 0;
-    const int64_t blocks = gx * bands + static_cast<int64_t>(l.x) * l.y;
-    if (ws.bandRows == 0 || blocks > INT32_MAX) {
-        launchList();
-        return err != cudaSuccess ? err : cudaGetLastError();
-    }
-    ws.maxRows = static_cast<int32_t>(bandReads(ws.bandRows));
-    ws.walkX = static_cast<int32_t>(gx);
-    ws.listX = l.x;
-    ws.listY = l.y;
-    ws.listCols = l.colsPB;
-    ws.listMax = l.entries;
-    const size_t smem = std::max(l.smem, static_cast<size_t>(ws.maxRows) * sizeof(WalkRecord) + static_cast<size_t>(ws.bandRows) * 8);
     OPSCV_DISPATCH_DT(dt, T, {
         auto launch = [&](auto columns) {
             constexpr int K = decltype(columns)::value;
             auto kernel = nhwc ? Bicubic2dBwdWalkKernel<T, true, K> : Bicubic2dBwdWalkKernel<T, false, K>;
-            if (smem > 48 * 1024) {
-                err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            if (plan.smem > 48 * 1024) {
+                err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.smem));
             }
             if (err == cudaSuccess) {
-                kernel<<<static_cast<unsigned>(blocks), kWalkThreads, smem, s>>>(static_cast<const T*>(go), static_cast<T*>(gi),
-                                                                                 g, ws);
+                kernel<<<static_cast<unsigned>(plan.blocks), kWalkThreads, plan.smem, s>>>(
+                    static_cast<const T*>(go), static_cast<T*>(gi), g, plan.ws);
             }
         };
         // A walk spans four source pixels: at most ceil(4 / scale) columns, with a margin for rounding (a column whose walk is
@@ -1840,6 +1877,19 @@ cudaError_t Bicubic2dBwd(Dt dt, Layout lay, const void* go, void* gi, Shape4 sh,
     });
     CountLaunch();
     return err != cudaSuccess ? err : cudaGetLastError();
+}
+
+bool DebugBicubic2dBwd(Layout lay, Shape4 sh, float scaleH, float scaleW, float invH, float invW, bool align, int64_t values[8])
+{
+    const BicubicGeom g = BwdGeom(lay, sh, scaleH, scaleW, invH, invW, align);
+    X2Launch x2;
+    BwdWalkPlan p;
+    if (PlanBwdX2(g, lay == kNHWC, &x2) || !PlanBwdWalk(g, &p)) {
+        return false;
+    }
+    const int64_t v[8] = {p.ws.bandRows, p.ws.maxRows, kOpen, 0, 0, 0, p.bands, static_cast<int64_t>(p.smem)};
+    std::copy(v, v + 8, values);
+    return true;
 }
 
 } // namespace opscv

@@ -297,3 +297,13 @@ def test_bicubic_backward_walk_user_scale_and_non_finite(ops, oracle, dev):
     ref = oracle.bicubic2d_bwd(g.numpy(), (24, 20), False, definition="gather")
     assert np.array_equal(gi.view(np.uint32)[~np.isnan(ref)], ref.view(np.uint32)[~np.isnan(ref)])
     assert np.isnan(gi[np.isnan(ref)]).all()
+
+
+# Tall planes: bands whose rows, not the grads rows that they read, fill the shared memory, and more than 256 bands
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hi,ho", [(60000, 1), (100000, 2), (30000, 120000), (1 << 20, (1 << 20) + 5)])
+def test_bicubic_backward_of_tall_planes(ops, oracle, dev, dtype, hi, ho):
+    assert ops.debug_plan("bicubic_backward_walk", 4, (1, 2, hi, 4, ho, 4)) is not None
+    g, g32 = quant(torch.randn((1, 2, ho, 4), generator=gen(122)), dtype)
+    gi = ops.upsample_bicubic2d_backward(g.to(dev), (ho, 4), (1, 2, hi, 4), False)
+    check(gi, oracle.bicubic2d_bwd(g32, (hi, 4), False, definition="gather"), dtype, exact=True)

@@ -116,3 +116,62 @@ def test_bilinear_walk_of_one_tall_plane_fills_the_device(ops, fmt, c, hi, wi, h
     plan = ops.debug_plan("bilinear_backward_walk", 4, (1, c, hi, wi, ho, wo), fmt)
     assert plan is not None and -(-hi // plan[0]) >= 148  # bands; B200 has 148 SMs
     assert check_walk(ops, fmt, 4, 1, c, hi, wi, ho, wo, False)
+
+
+def bicubic_rows(n_in, n_out, align, user):
+    """First and one past the last grads row of the walk of every grad_input row."""
+    off = F(0) if align else F(0.5)
+    if align and n_in > 1 and n_out > 1:
+        scale, inv = F(n_in - 1) / F(n_out - 1), F(n_out - 1) / F(n_in - 1)
+    elif not align and user > 0:
+        scale, inv = F(1) / F(user), F(user)
+    else:
+        scale, inv = F(n_in) / F(n_out), F(n_out) / F(n_in)
+    y = np.arange(n_in).astype(F)
+    start = np.ceil((y - F(2) + off) * inv - off)
+    start = np.clip(start.astype(np.float64), 0, n_out).astype(np.int64)
+    h = np.arange(n_out).astype(F)
+    src = h * scale if align else (h + off) * scale - off
+    end = np.searchsorted(src, y + F(2))
+    end[0] = np.searchsorted(np.floor(src), 1, side="right")
+    end[-1] = n_out
+    return start, np.maximum(end, start)
+
+
+def check_bicubic(ops, elem, n, c, hi, wi, ho, wo, align, user=0.0, fmt="NCHW"):
+    plan = ops.debug_plan("bicubic_backward_walk", elem, (n, c, hi, wi, ho, wo), fmt, align, (user, user))
+    if plan is None:
+        return False
+    band, most_rows, most_open, smem = plan[0], plan[1], plan[2], plan[7]
+    assert 0 < smem <= 48 * 1024
+    start, end = bicubic_rows(hi, ho, align, user)
+    for y0 in range(0, hi, band):
+        y1 = min(y0 + band, hi)
+        assert end[y0:y1].max() - start[y0:y1].min() <= most_rows
+    if hi > 2:  # interior rows whose walks include a grads row
+        diff = np.zeros(ho + 1, np.int64)
+        np.add.at(diff, start[1:-1], 1)
+        np.add.at(diff, end[1:-1], -1)
+        assert np.cumsum(diff).max() <= most_open
+    return True
+
+
+@pytest.mark.parametrize("hi,ho", [(60000, 1), (60000, 2), (100000, 2), (20000, 100), (40000, 160000), (200000, 200000),
+                                   (1 << 20, 1 << 20), (1 << 20, 1 << 22), ((1 << 20) - 1, 3000001)])
+@pytest.mark.parametrize("align", [False, True])
+def test_bicubic_walk_of_tall_planes(ops, hi, ho, align):
+    taken = check_bicubic(ops, 4, 1, 3, hi, 8, ho, 9, align)
+    if not align:
+        assert taken
+
+
+def test_bicubic_walk_of_random_sizes(ops):
+    rng = random.Random(8)
+    taken = 0
+    for _ in range(600):
+        hi, wi = int(2 ** rng.uniform(1, 12)), int(2 ** rng.uniform(1, 8))
+        ho, wo = max(1, int(hi * 2 ** rng.uniform(-8, 4))), max(1, int(wi * 2 ** rng.uniform(-3, 2)))
+        user = rng.choice([0.0, 0.0, ho / hi * rng.uniform(0.97, 1.03)])
+        taken += check_bicubic(ops, rng.choice([2, 4]), rng.randint(1, 3), rng.choice([1, 3, 8]), hi, wi, ho, wo,
+                               rng.random() < 0.4, user, rng.choice(["NCHW", "NHWC"]))
+    assert taken > 200
