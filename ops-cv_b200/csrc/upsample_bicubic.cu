@@ -538,30 +538,36 @@ __device__ float BwdElementDirect(const T* __restrict__ pg, const BicubicGeom& g
 // so the sum has the same bits. The additions of a thread are one chain; what it must not wait for one by one are the
 // loads, so the grads values of kListBatch columns are fetched before the first of them is used (border columns of
 // fp32 8x64 planes 60x80 <- 150x199: 58 us with one load at a time, 38 us in batches).
-// colsPB: element positions of a row that a block covers (its threads beyond that take further rows);
-// borderOnly: the block's positions are those of the first and the last column only.
+// The blocks of a launch divide its element positions (of all columns, or of the first and the last, or of those between)
+// by x and its rows by y; colsPB positions per block, further threads take further rows.
+// TAPS: most taps of a list's column, one where the border columns are not among them.
 constexpr int kListBatch = 8;
-constexpr int kListTaps = 3;                       // a fourth needs an extent of 1
-constexpr int kListBytes = 4 + 4 * kListTaps;      // per column and thread
+constexpr int kListTaps = 3; // a fourth needs an extent of 1
 constexpr int kListThreads = 128;
+constexpr int ListBytes(int taps) { return 4 + 4 * taps; } // per column and thread
+enum ListColumns { kAllColumns, kBorderColumns, kInteriorColumns };
+struct ListShape {
+    int32_t colsPB, entries, x, y;
+};
 
-template <typename T, bool NHWC>
-__device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __restrict__ gi, const BicubicGeom& g, int32_t maxW,
-                                             int32_t colsPB, bool borderOnly, float* sList, int32_t blockX, int64_t blockY,
-                                             int64_t blocksY)
+template <typename T, bool NHWC, int TAPS>
+__device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __restrict__ gi, const BicubicGeom& g,
+                                             int32_t maxW, int32_t colsPB, ListColumns columns, float* sList, int32_t blockX,
+                                             int64_t blockY, int64_t blocksY)
 {
     const int32_t nt = blockDim.x, tid = threadIdx.x;
-    float* sCoef = sList; // [maxW][kListTaps][nt]
-    int32_t* sCol = reinterpret_cast<int32_t*>(sList + static_cast<size_t>(maxW) * kListTaps * nt); // column << 2 | taps
+    float* sCoef = sList; // [maxW][TAPS][nt]
+    int32_t* sCol = reinterpret_cast<int32_t*>(sList + static_cast<size_t>(maxW) * TAPS * nt); // column << 2 | taps
     const int32_t inner = g.win * g.chan;
     const int32_t rowsPB = nt / colsPB;
     const int32_t rowLane = tid / colsPB;
     const int32_t pos = blockX * colsPB + (tid - rowLane * colsPB);
-    if (rowLane >= rowsPB || pos >= (borderOnly ? 2 * g.chan : inner)) {
+    const int32_t positions = columns == kAllColumns ? inner : (columns == kBorderColumns ? 2 * g.chan : inner - 2 * g.chan);
+    if (rowLane >= rowsPB || pos >= positions) {
         return;
     }
-    int32_t t = pos;
-    if (borderOnly) {
+    int32_t t = columns == kInteriorColumns ? pos + g.chan : pos;
+    if (columns == kBorderColumns) {
         const int32_t side = NHWC ? pos / g.chan : pos;
         t = side == 0 ? pos : inner - 2 * g.chan + pos; // column 0 or column win - 1, same channel
     }
@@ -570,7 +576,7 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
     const int64_t planeGo = static_cast<int64_t>(g.hout) * g.wout * g.chan;
     const int64_t rowGo = static_cast<int64_t>(g.wout) * g.chan;
     const float offset = g.align ? 0.0f : 0.5f;
-    const bool borderW = yw == 0 || yw == g.win - 1;
+    const bool borderW = columns != kInteriorColumns && (yw == 0 || yw == g.win - 1);
 
     // the column walk, once
     int32_t cnt = 0;
@@ -591,8 +597,8 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (!overflow && ClampIdx(fw - 1 + j, g.win - 1) == yw) {
-                        if (n < kListTaps) {
-                            sCoef[(cnt * kListTaps + n) * nt + tid] = cwTap[j];
+                        if (n < TAPS) {
+                            sCoef[(cnt * TAPS + n) * nt + tid] = cwTap[j];
                             ++n;
                         } else {
                             overflow = true;
@@ -609,7 +615,7 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
                 }
                 overflow = cnt >= maxW || w >= (1 << 29);
                 if (!overflow) {
-                    sCoef[cnt * kListTaps * nt + tid] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
+                    sCoef[cnt * TAPS * nt + tid] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
                     sCol[cnt * nt + tid] = w << 2 | 1;
                     ++cnt;
                 }
@@ -677,12 +683,12 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
                     if (taps[u] == 0) {
                         break;
                     }
-                    const float* cu = sCoef + (k0 + u) * kListTaps * nt + tid;
+                    const float* cu = sCoef + (k0 + u) * TAPS * nt + tid;
                     for (int i = 0; i < nH; ++i) {
                         const float gc = Mul(gv[u], i == 0 ? chv[0] : (i == 1 ? chv[1] : (i == 2 ? chv[2] : chv[3])));
 #pragma unroll
-                        for (int j = 0; j < kListTaps; ++j) {
-                            if (j < taps[u]) {
+                        for (int j = 0; j < TAPS; ++j) {
+                            if (TAPS == 1 || j < taps[u]) {
                                 add = Add(add, Mul(gc, cu[j * nt]));
                             }
                         }
@@ -694,12 +700,25 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
     }
 }
 
+// All columns by lists (scales beyond four, user scales that contradict the extents, extents of two): the border columns in
+// the first blocks, whose chains are the longest, the interior ones behind them with one coefficient per column. With room
+// for three in every list fewer of them fit (fp32 4x16 planes 32x64 <- 512x1024: 4223 us; so 2072 us).
 template <typename T, bool NHWC>
 __global__ void __launch_bounds__(kListThreads) Bicubic2dBwdListKernel(const T* __restrict__ go, T* __restrict__ gi, BicubicGeom g,
-                                                                        int32_t maxW, int32_t colsPB)
+                                                                        ListShape border, ListShape interior)
 {
     extern __shared__ __align__(16) float sList[];
-    BwdListBlock<T, NHWC>(go, gi, g, maxW, colsPB, false, sList, blockIdx.x, blockIdx.y, gridDim.y);
+    const int32_t block = blockIdx.x, borders = border.x * border.y;
+    if (g.win <= 2) {
+        BwdListBlock<T, NHWC, kListTaps>(go, gi, g, border.entries, border.colsPB, kAllColumns, sList, block % border.x,
+                                         block / border.x, border.y);
+    } else if (block < borders) {
+        BwdListBlock<T, NHWC, kListTaps>(go, gi, g, border.entries, border.colsPB, kBorderColumns, sList, block % border.x,
+                                         block / border.x, border.y);
+    } else {
+        BwdListBlock<T, NHWC, 1>(go, gi, g, interior.entries, interior.colsPB, kInteriorColumns, sList,
+                                 (block - borders) % interior.x, (block - borders) / interior.x, interior.y);
+    }
 }
 
 // ---- the same gather for the interior columns (1 .. win - 2): a walk down the grads rows --------------------------
@@ -729,10 +748,11 @@ struct WalkRecord {
 static_assert(sizeof(WalkRecord) == 64, "records are read as 16-byte words");
 static_assert(kListThreads == kWalkThreads, "list blocks and walk blocks share a grid");
 
-// walkX: blocks of one band; the first listX * listY blocks of the grid are list blocks.
+// walkX: blocks of one band; the first list.x * list.y blocks of the grid are list blocks.
 struct WalkShape {
     int64_t positions; // planes * interior element positions of a row
-    int32_t bandRows, maxRows, walkX, listX, listY, listCols, listMax;
+    int32_t bandRows, maxRows, walkX;
+    ListShape list;
 };
 
 template <typename T, bool NHWC, int K>
@@ -740,10 +760,11 @@ __global__ void __launch_bounds__(kWalkThreads, (NHWC && K > 14) ? 3 : ((NHWC ||
     Bicubic2dBwdWalkKernel(const T* __restrict__ go, T* __restrict__ gi, BicubicGeom g, WalkShape ws)
 {
     extern __shared__ __align__(16) float sWalk[];
-    const int32_t lists = ws.listX * ws.listY;
+    const int32_t lists = ws.list.x * ws.list.y;
     if (static_cast<int32_t>(blockIdx.x) < lists) {
-        BwdListBlock<T, NHWC>(go, gi, g, ws.listMax, ws.listCols, true, sWalk, static_cast<int32_t>(blockIdx.x) % ws.listX,
-                              static_cast<int32_t>(blockIdx.x) / ws.listX, ws.listY);
+        BwdListBlock<T, NHWC, kListTaps>(go, gi, g, ws.list.entries, ws.list.colsPB, kBorderColumns, sWalk,
+                                         static_cast<int32_t>(blockIdx.x) % ws.list.x,
+                                         static_cast<int32_t>(blockIdx.x) / ws.list.x, ws.list.y);
         return;
     }
     const int32_t walkBlock = static_cast<int32_t>(blockIdx.x) - lists;
@@ -1512,29 +1533,56 @@ dim3 RowGrid(int64_t rows, int64_t inner)
 }
 
 // ---- launch shapes of the general backward ------------------------------------------------------------------------
-struct ListLaunch {
-    int32_t colsPB, entries, x, y;
-    size_t smem;
-};
-ListLaunch PlanBwdList(const BicubicGeom& g, bool borderOnly)
+// A launch of `positions` element positions per row, columns of up to `taps` taps, `threads` threads per block. Columns of one
+// list: four source pixels for an interior column, two and a half for a first or last one (three, for user scales). Lists that
+// would not fit make their thread fall back to the uncached walk, so the bound only has to be good, not safe; a
+// single-column image (every grads column is a tap) always falls back.
+ListShape PlanBwdList(const BicubicGeom& g, int64_t positions, int taps, int threads, double span)
 {
-    const int64_t inner = static_cast<int64_t>(g.win) * g.chan;
     const double perScale = g.invW > 0.0f ? static_cast<double>(g.invW) : 1.0;
-    // Columns of one list: the grads columns of an interior walk; a first or last column takes those within two and a
-    // half source pixels. Lists that would not fit make their thread fall back to the uncached walk, so the bound only
-    // has to be good, not safe; a single-column image (every grads column is a tap) always falls back.
-    const int64_t maxW = static_cast<int64_t>(std::ceil(4.0 * perScale)) + 4;
-    const int64_t positions = borderOnly ? 2LL * g.chan : inner;
-    ListLaunch l;
-    l.colsPB = static_cast<int32_t>(std::min<int64_t>(kListThreads, positions));
-    const int rowsPB = kListThreads / l.colsPB;
-    const int64_t cap = 96 * 1024 / (kListBytes * kListThreads);
+    const int64_t maxW = static_cast<int64_t>(std::ceil(span * perScale)) + 4;
+    const int64_t cap = (taps == 1 ? 96 : 192) * 1024 / (ListBytes(taps) * threads);
+    ListShape l;
+    l.colsPB = static_cast<int32_t>(std::min<int64_t>(threads, positions));
+    const int rowsPB = threads / l.colsPB;
     l.entries = static_cast<int32_t>(std::max<int64_t>(4, std::min<int64_t>(maxW, cap)));
-    l.smem = static_cast<size_t>(l.entries) * kListThreads * kListBytes;
     l.x = static_cast<int32_t>(CeilDiv(positions, l.colsPB));
     const int64_t gyCap = std::max<int64_t>(static_cast<int64_t>(NumSMs()) * 32 / l.x, 1);
     l.y = static_cast<int32_t>(std::min<int64_t>(std::min<int64_t>(CeilDiv(g.rows, rowsPB), gyCap), 65535));
     return l;
+}
+size_t ListSmem(const ListShape& l, int taps, int threads)
+{
+    return static_cast<size_t>(l.entries) * threads * ListBytes(taps);
+}
+
+// The list kernel alone.
+struct BwdListPlan {
+    ListShape border, interior;
+    int32_t threads;
+    int64_t blocks;
+    size_t smem;
+};
+BwdListPlan PlanBwdLists(const BicubicGeom& g)
+{
+    const int64_t inner = static_cast<int64_t>(g.win) * g.chan;
+    BwdListPlan p{};
+    if (g.win <= 2) {
+        p.threads = kListThreads;
+        p.border = PlanBwdList(g, inner, kListTaps, p.threads, 4.0);
+    } else {
+        // equal shares of a row for its blocks, so that none of them is nearly empty, and no more threads than that needs:
+        // fewer threads leave room for longer lists
+        const int64_t positions = inner - 2LL * g.chan, share = CeilDiv(positions, CeilDiv(positions, kListThreads));
+        p.threads = static_cast<int32_t>(std::max<int64_t>(64, (share + 31) / 32 * 32));
+        p.border = PlanBwdList(g, 2LL * g.chan, kListTaps, p.threads, 3.0);
+        p.interior = PlanBwdList(g, positions, 1, p.threads, 4.0);
+        p.blocks = static_cast<int64_t>(p.interior.x) * p.interior.y;
+        p.smem = ListSmem(p.interior, 1, p.threads);
+    }
+    p.blocks += static_cast<int64_t>(p.border.x) * p.border.y;
+    p.smem = std::max(p.smem, ListSmem(p.border, kListTaps, p.threads));
+    return p;
 }
 
 // Interior columns by the row walk, the two border columns apart; false where the list kernel serves the call.
@@ -1563,7 +1611,7 @@ bool PlanBwdWalk(const BicubicGeom& g, BwdWalkPlan* plan)
         return false;
     }
     const int64_t planes = g.rows / g.hin;
-    const ListLaunch l = PlanBwdList(g, true);
+    const ListShape l = PlanBwdList(g, 2LL * g.chan, kListTaps, kListThreads, 4.0);
     WalkShape& ws = plan->ws;
     ws = WalkShape{};
     ws.positions = planes * (inner - 2LL * g.chan);
@@ -1600,11 +1648,8 @@ bool PlanBwdWalk(const BicubicGeom& g, BwdWalkPlan* plan)
     }
     ws.maxRows = static_cast<int32_t>(bandReads(ws.bandRows));
     ws.walkX = static_cast<int32_t>(gx);
-    ws.listX = l.x;
-    ws.listY = l.y;
-    ws.listCols = l.colsPB;
-    ws.listMax = l.entries;
-    plan->smem = std::max(l.smem, bandSmem(ws.bandRows));
+    ws.list = l;
+    plan->smem = std::max(ListSmem(l, kListTaps, kListThreads), bandSmem(ws.bandRows));
     return true;
 }
 
@@ -1801,15 +1846,15 @@ cudaError_t Bicubic2dBwd(Dt dt, Layout lay, const void* go, void* gi, Shape4 sh,
     const double perScale = invW > 0.0f ? static_cast<double>(invW) : 1.0;
     cudaError_t err = cudaSuccess;
     auto launchList = [&]() {
-        const ListLaunch l = PlanBwdList(g, false);
+        const BwdListPlan l = PlanBwdLists(g);
         OPSCV_DISPATCH_DT(dt, T, {
             auto kernel = nhwc ? Bicubic2dBwdListKernel<T, true> : Bicubic2dBwdListKernel<T, false>;
             if (l.smem > 48 * 1024) {
                 err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(l.smem));
             }
             if (err == cudaSuccess) {
-                kernel<<<dim3(l.x, l.y), kListThreads, l.smem, s>>>(static_cast<const T*>(go), static_cast<T*>(gi), g, l.entries,
-                                                                    l.colsPB);
+                kernel<<<static_cast<unsigned>(l.blocks), l.threads, l.smem, s>>>(
+                    static_cast<const T*>(go), static_cast<T*>(gi), g, l.border, l.interior);
             }
         });
         CountLaunch();

@@ -307,3 +307,24 @@ def test_bicubic_backward_of_tall_planes(ops, oracle, dev, dtype, hi, ho):
     g, g32 = quant(torch.randn((1, 2, ho, 4), generator=gen(122)), dtype)
     gi = ops.upsample_bicubic2d_backward(g.to(dev), (ho, 4), (1, 2, hi, 4), False)
     check(gi, oracle.bicubic2d_bwd(g32, (hi, 4), False, definition="gather"), dtype, exact=True)
+
+
+# The list kernel: scales beyond four and strongly beyond (lists that just fit and that do not), rows of several equal blocks, of
+# a few elements, extents of one and two
+LIST_SHAPES = [(1, 2, 5, 7, 81, 140), (2, 1, 6, 300, 31, 1400), (1, 3, 4, 3, 50, 150), (3, 2, 2, 2, 9, 13), (1, 2, 4, 1, 50, 9),
+               (1, 1, 3, 130, 20, 2600), (2, 3, 2, 40, 5, 100)]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("fmt", ["NCHW", "NHWC"])
+@pytest.mark.parametrize("align", [False, True])
+@pytest.mark.parametrize("shape", LIST_SHAPES)
+def test_bicubic_backward_lists(ops, oracle, dev, dtype, fmt, align, shape):
+    n, c, hi, wi, ho, wo = shape
+    assert ops.debug_plan("bicubic_backward_walk", 4, shape[:2] + (hi, wi, ho, wo), fmt, align) is None
+    g, g32 = quant(torch.randn((n, c, ho, wo), generator=gen(123)), dtype)
+    gl = torch.from_numpy(_layout(g32, fmt)).to(dtype)
+    size = (n, hi, wi, c) if fmt == "NHWC" else (n, c, hi, wi)
+    gi = ops.upsample_bicubic2d_backward(gl.to(dev), (ho, wo), size, align, fmt)
+    ofmt = oracle.NHWC if fmt == "NHWC" else oracle.NCHW
+    check(gi, oracle.bicubic2d_bwd(_layout(g32, fmt), (hi, wi), align, fmt=ofmt, definition="gather"), dtype, exact=True)
