@@ -354,13 +354,15 @@ __global__ void __launch_bounds__(kThreads) Bicubic2dFwdTileKernel(const T* __re
         }
         __syncthreads();
         T* py = y + (plane * g.hout + h0) * static_cast<int64_t>(g.wout);
-        if constexpr (V <= 2) {
+        const int32_t segs = (nOut + kFwdWalk - 1) / kFwdWalk;
+        if (V <= 2 && g.scaleH < 1.0f && packs * segs >= kThreads) {
             // Rows that allow no wider store than two elements: a thread walks kFwdWalk output rows down its columns with
             // the four sums in registers. An up-scale moves the window on by at most one source row per output row, so
             // most rows load one sum or none; with four loads and four row offsets per output the pass was bound by
             // instruction issue (fp32 8x64 planes 60x80 -> 150x199: 80 instructions per output, 81 % of the issue slots; 46 -> 37 us).
-            // Columns and segments of rows share one index, so that no thread is idle at any width.
-            const int32_t segs = (nOut + kFwdWalk - 1) / kFwdWalk;
+            // Columns and segments of rows share one index, so that no thread is idle at any width. A down-scale loads four
+            // sums per row all the same, and a tile with fewer walks than threads leaves some idle: both take a thread per
+            // output (bf16 4x50 planes 45x44 -> 26x27: 8.3 us by walks, 6.4).
             for (int32_t i = tid; i < packs * segs; i += kThreads) {
                 const int32_t seg = i / packs, p = i - seg * packs;
                 const int32_t r1 = min(nOut, (seg + 1) * kFwdWalk);
