@@ -5,6 +5,7 @@
 //
 // The functions take positional arguments in the order of the wrappers in aclnn.py, which document them.
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <ATen/Functions.h>
@@ -567,6 +568,9 @@ PyObject* GridSamplerBackward(Args a)
         }, aclnnGridSampler2DBackward, x.device(), a[10]);
     }
     PyObject* pair = PyTuple_New(2);
+    if (pair == nullptr) {
+        throw Raised{};
+    }
     PyTuple_SET_ITEM(pair, 0, Give(gx));
     PyTuple_SET_ITEM(pair, 1, Give(gg));
     return pair;
@@ -584,8 +588,8 @@ PyObject* Entry(PyObject*, PyObject* const* args, Py_ssize_t n)
         return F(args);
     } catch (const Raised&) {
         return nullptr;
-    } catch (const std::exception& e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
+    } catch (...) { // by torch's own table: a full device is torch.OutOfMemoryError, and so on
+        torch::translate_exception_to_python(std::current_exception());
         return nullptr;
     }
 }
