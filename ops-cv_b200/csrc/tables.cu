@@ -217,6 +217,9 @@ __device__ __forceinline__ float FilterAA(int filter, float m)
 
 // upsample_bicubic2d_aa_simt_base.h:70-124 and upsample_bilinear2d_aa_simt_base.h:52-88: window
 // [xmin, xmin+xsize), weights normalised by their sum. filter: 0 Keys cubic, 1 triangle.
+// HOLD: a weight waits in its table entry for the sum instead of being evaluated again: a shorter chain for the few threads of a
+// cluster, more memory traffic for a thread per index (4x2^20 -> 2x2^18, the whole forward: 85 us, 65 without).
+template <bool HOLD>
 __device__ __forceinline__ void AATableEntry(const AxisGeom& g, const AAAxis& t, float inv, float support, int backward,
                                              int filter, int32_t i)
 {
@@ -244,12 +247,17 @@ __device__ __forceinline__ void AATableEntry(const AxisGeom& g, const AAAxis& t,
     for (int32_t j = 0; j < size; ++j) {
         const float dist = Mul(Add(Sub(static_cast<float>(lo + j), center), 0.5f), inv);
         const float wj = FilterAA(filter, dist);
-        w[j] = wj;
+        if (HOLD) {
+            w[j] = wj;
+        }
         total = Add(total, wj);
     }
     for (int32_t j = 0; j < t.taps; ++j) {
         if (j >= size) {
             w[j] = 0.0f;
+        } else if (!HOLD) {
+            const float wj = FilterAA(filter, Mul(Add(Sub(static_cast<float>(lo + j), center), 0.5f), inv));
+            w[j] = total != 0.0f ? Div(wj, total) : wj;
         } else if (total != 0.0f) {
             w[j] = Div(w[j], total);
         }
@@ -263,7 +271,7 @@ __global__ void AATableKernel(AxisGeom gh, AxisGeom gw, float invH, float invW, 
     const AxisGeom g = isH ? gh : gw;
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < g.out) {
-        AATableEntry(g, isH ? th : tw, isH ? invH : invW, isH ? supH : supW, backward, filter, i);
+        AATableEntry<false>(g, isH ? th : tw, isH ? invH : invW, isH ? supH : supW, backward, filter, i);
     }
 }
 
@@ -293,14 +301,55 @@ __device__ __forceinline__ void AARangeEntry(const AxisGeom& g, const AAAxis& t,
     end = a > first ? a : first;
 }
 
+// Range of input index y and, where there is one, its slot record (kAASlotStride floats): weight at y of output start + a for
+// a < kAASlots (0 past the run), then start and the run length as integer bit patterns.
+__device__ __forceinline__ void AARangeAndRecord(const AxisGeom& g, const AAAxis& t, const RangeAxis& r, float* rec, int32_t y)
+{
+    int32_t s, e;
+    AARangeEntry(g, t, y, s, e);
+    r.start[y] = s;
+    r.end[y] = e;
+    if (rec == nullptr) {
+        return;
+    }
+    float slot[kAASlotStride];
+#pragma unroll
+    for (int a = 0; a < kAASlots; ++a) {
+        slot[a] = 0.0f;
+        if (s + a < e) {
+            const int32_t k = y - t.xmin[s + a];
+            if (k >= 0 && k < t.xsize[s + a]) {
+                slot[a] = t.w[static_cast<int64_t>(s + a) * t.taps + k];
+            }
+        }
+    }
+    slot[kAASlots] = __int_as_float(s);
+    slot[kAASlots + 1] = __int_as_float(min(e - s, kAASlots));
+    float4* out = reinterpret_cast<float4*>(rec + static_cast<int64_t>(y) * kAASlotStride);
+    out[0] = make_float4(slot[0], slot[1], slot[2], slot[3]);
+    out[1] = make_float4(slot[4], slot[5], slot[6], slot[7]);
+}
+
+__global__ void AARangesKernel(AxisGeom gh, AxisGeom gw, AAAxis th, AAAxis tw, RangeAxis rh, RangeAxis rw,
+                               float* __restrict__ recH, float* __restrict__ recW)
+{
+    const bool isH = blockIdx.y == 0;
+    const AxisGeom g = isH ? gh : gw;
+    const int32_t y = blockIdx.x * blockDim.x + threadIdx.x;
+    if (y < g.in) {
+        AARangeAndRecord(g, isH ? th : tw, isH ? rh : rw, isH ? recH : recW, y);
+    }
+}
+
 // Tables, ranges and slot records of both axes in one launch: one cluster per axis, whose blocks meet at the cluster
 // barrier between the entries per output index and the entries per input index that are searched from them (the
 // barrier orders the global writes before the reads of the other blocks). As three or four dependent launches this
-// preparation took 12 to 18 us of a call, most of it launch latency; in one launch 5 to 10 us.
-// Record of input index y (kAASlotStride floats): weight at y of output start + a for a < kAASlots (0 past the run),
-// then start and the run length as integer bit patterns.
+// preparation took 12 to 18 us of a call, most of it launch latency; in one launch 5 to 10 us. Its eight blocks take 2048
+// indices at a time, some five microseconds each time, so axes of more than kAAClusterMost indices are better off with a
+// thread per index and two launches (4x2^20 <- 2x2^18: 3053 us by clusters).
 constexpr int kAAClusterBlocks = 8;
 constexpr int kAAClusterThreads = 256;
+constexpr int kAAClusterMost = 4 * kAAClusterBlocks * kAAClusterThreads;
 
 __global__ void __cluster_dims__(kAAClusterBlocks, 1, 1) __launch_bounds__(kAAClusterThreads)
     AATablesAndRangesKernel(AxisGeom gh, AxisGeom gw, float invH, float invW, float supH, float supW, AAAxis th, AAAxis tw,
@@ -313,35 +362,13 @@ __global__ void __cluster_dims__(kAAClusterBlocks, 1, 1) __launch_bounds__(kAACl
     // consecutive indices go to different blocks: a short axis keeps all eight SMs busy
     const int32_t first = threadIdx.x * kAAClusterBlocks + blockIdx.x, step = kAAClusterBlocks * kAAClusterThreads;
     for (int32_t i = first; i < g.out; i += step) {
-        AATableEntry(g, t, isH ? invH : invW, isH ? supH : supW, backward, filter, i);
+        AATableEntry<true>(g, t, isH ? invH : invW, isH ? supH : supW, backward, filter, i);
     }
     cooperative_groups::this_cluster().sync();
     const RangeAxis r = isH ? rh : rw;
     float* rec = isH ? recH : recW;
     for (int32_t y = first; y < g.in; y += step) {
-        int32_t s, e;
-        AARangeEntry(g, t, y, s, e);
-        r.start[y] = s;
-        r.end[y] = e;
-        if (rec == nullptr) {
-            continue;
-        }
-        float slot[kAASlotStride];
-#pragma unroll
-        for (int a = 0; a < kAASlots; ++a) {
-            slot[a] = 0.0f;
-            if (s + a < e) {
-                const int32_t k = y - t.xmin[s + a];
-                if (k >= 0 && k < t.xsize[s + a]) {
-                    slot[a] = t.w[static_cast<int64_t>(s + a) * t.taps + k];
-                }
-            }
-        }
-        slot[kAASlots] = __int_as_float(s);
-        slot[kAASlots + 1] = __int_as_float(min(e - s, kAASlots));
-        float4* out = reinterpret_cast<float4*>(rec + static_cast<int64_t>(y) * kAASlotStride);
-        out[0] = make_float4(slot[0], slot[1], slot[2], slot[3]);
-        out[1] = make_float4(slot[4], slot[5], slot[6], slot[7]);
+        AARangeAndRecord(g, t, r, rec, y);
     }
 }
 
@@ -400,6 +427,15 @@ cudaError_t BuildAATablesAndRanges(AxisGeom h, AxisGeom w, float invH, float inv
                                    AAAxis tw, bool backward, int filter, RangeAxis rh, RangeAxis rw, float* recH,
                                    float* recW, cudaStream_t s)
 {
+    if (std::max({h.in, h.out, w.in, w.out}) > kAAClusterMost) {
+        const cudaError_t e = BuildAATables(h, w, invH, invW, supH, supW, th, tw, backward, filter, s);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        AARangesKernel<<<TableGrid(h.in, w.in), kTableThreads, 0, s>>>(h, w, th, tw, rh, rw, recH, recW);
+        CountLaunch();
+        return cudaGetLastError();
+    }
     AATablesAndRangesKernel<<<dim3(kAAClusterBlocks, 2), kAAClusterThreads, 0, s>>>(
         h, w, invH, invW, supH, supW, th, tw, backward ? 1 : 0, filter, rh, rw, recH, recW);
     CountLaunch();

@@ -84,3 +84,25 @@ def test_non_finite_values_at_odd_widths(ops, oracle, dev):
     g = _poison(torch.rand((1, 2, 13, 19), generator=gen(96)), rng, 4)
     _same_nonfinite(ops.upsample_bicubic2d_aa_grad(g.to(dev), (13, 19), (1, 2, 41, 57), False),
                     oracle.bicubic_aa_bwd(g.numpy(), (41, 57), False, definition="gather"), "backward")
+
+
+# one long axis: its tables come from a thread per index (two launches), short ones from a cluster (one)
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("filt", ["bicubic", "bilinear"])
+@pytest.mark.parametrize("shape", [(1, 1, 8193, 40, 2731, 20), (1, 1, 20011, 33, 5003, 11), (1, 1, 6, 8193, 3, 4001),
+                                   (1, 2, 3, 5000, 5, 9000), (1, 1, 8192, 36, 4096, 18)])
+def test_long_axes(ops, oracle, dev, dtype, filt, shape):
+    n, c, h, w, oh, ow = shape
+    fwd, bwd, ofwd, obwd = {
+        "bicubic": (ops.upsample_bicubic2d_aa, ops.upsample_bicubic2d_aa_grad, oracle.bicubic_aa_fwd,
+                    oracle.bicubic_aa_bwd),
+        "bilinear": (ops.upsample_bilinear2d_aa, ops.upsample_bilinear2d_aa_backward, oracle.bilinear_aa_fwd,
+                     oracle.bilinear_aa_bwd)}[filt]
+    x, x32 = quant(torch.rand((n, c, h, w), generator=gen(98)), dtype)
+    close(fwd(x.to(dev), (oh, ow), False), ofwd(x32, (oh, ow), False), dtype)
+    g, g32 = quant(torch.rand((n, c, oh, ow), generator=gen(99)), dtype)
+    g = g.to(dev)
+    ops.reset_launch_count()
+    gi = bwd(g, (oh, ow), (n, c, h, w), False)
+    assert ops.launch_count() == (3 if max(shape) > 8192 else 2)
+    close(gi, obwd(g32, (h, w), False, definition="gather"), dtype)
