@@ -362,7 +362,11 @@ ACLNN_API aclnnStatus opscvDebugAxisTable(int32_t kind, int64_t inSize, int64_t 
  *   thread (NCHW) or channel slices (NHWC), planes or images per block, bands (NCHW) or most significant bits of a product
  *   of two weights (NHWC), shared-memory bytes};
  * kind 1, UpsampleBicubic2dBackward by row walks: {grad_input rows per band, most grads rows of a band, most grad_input rows
- *   that one grads row feeds, 0, 0, 0, bands, shared-memory bytes}. */
+ *   that one grads row feeds, 0, 0, 0, bands, shared-memory bytes};
+ * kinds 2 and 4, the streaming forward of UpsampleBicubic2dAA and UpsampleBilinear2dAA: {output rows per band, most input rows of
+ *   a band, most output rows that one input row feeds, 0, horizontal weights in shared memory, 0, 0, 0};
+ * kinds 3 and 5, the band backward of the two: {grad_input rows per band, most grads rows of a band, most grads rows that feed
+ *   four grad_input rows, most grads columns that feed four grad_input columns, 0, 0, 0, 0}. */
 ACLNN_API aclnnStatus opscvDebugPlan(int32_t kind, int32_t elemSize, aclFormat format, const int64_t sizes[6],
                                      int32_t alignCorners, const double scales[2], int32_t* taken, int64_t values[8]);
 

@@ -179,7 +179,8 @@ def debug_plan(kind, elem_size, sizes, fmt="NCHW", align=False, scales=(0.0, 0.0
     """The launch shape of a kernel for these sizes (see opscvDebugPlan), or None where it does not take the call."""
     taken = ctypes.c_int32(0)
     values = (ctypes.c_int64 * 8)()
-    kinds = {"bilinear_backward_walk": 0, "bicubic_backward_walk": 1}
+    kinds = {"bilinear_backward_walk": 0, "bicubic_backward_walk": 1, "bicubic_aa_forward_stream": 2,
+             "bicubic_aa_backward_band": 3, "bilinear_aa_forward_stream": 4, "bilinear_aa_backward_band": 5}
     status = lib().opscvDebugPlan(kinds[kind], elem_size, _FORMATS[fmt], (ctypes.c_int64 * 6)(*sizes), int(align),
                                   (ctypes.c_double * 2)(*scales), ctypes.byref(taken), values)
     if status != 0:

@@ -2004,6 +2004,28 @@ aclnnStatus opscvDebugPlan(int32_t kind, int32_t elemSize, aclFormat format, con
             *taken = DebugBicubic2dBwd(lay, sh, bh.scale, bw.scale, bh.inverse, bw.inverse, align, values) ? 1 : 0;
             return ACLNN_SUCCESS;
         }
+        case 2:
+        case 3:
+        case 4:
+        case 5: {
+            const bool forward = kind % 2 == 0;
+            const int filter = kind >= 4 ? 1 : 0;
+            const Dt dt = elemSize == 4 ? Dt::F32 : Dt::F16;
+            const AAGeom ah = MakeAAGeom(in.h, out.h, align, scales[0], filter == 1 || !forward, filter);
+            const AAGeom aw = MakeAAGeom(in.w, out.w, align, scales[1], filter == 1 || !forward, filter);
+            if (forward) {
+                const AAFwdPlan p = MakeAAFwdPlan(dt, sh, ah.scale, aw.taps, filter);
+                const int64_t v[8] = {p.bandRows, p.metaRows, p.slots, 0, p.regWeights ? 1 : 0, 0, 0, 0};
+                std::copy(v, v + 8, values);
+                *taken = p.stream ? 1 : 0;
+            } else {
+                const AABwdPlan p = MakeAABwdPlan(dt, sh, ah.scale, aw.scale, filter);
+                const int64_t v[8] = {p.bandRows, p.stageRows, kAABwdRowSlots, p.colSlots, 0, 0, 0, 0};
+                std::copy(v, v + 8, values);
+                *taken = p.band ? 1 : 0;
+            }
+            return ACLNN_SUCCESS;
+        }
         default: return Fail(ACLNN_ERR_PARAM_INVALID, "%s: unknown kind %d", api, kind);
     }
 }

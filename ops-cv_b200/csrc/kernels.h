@@ -182,6 +182,7 @@ cudaError_t BicubicAAFwd(Dt dt, const void* x, void* y, Shape4 sh, AAAxis th, AA
 // Bounded waits on asynchronous copies that ran out since the library was loaded (0 in a healthy run).
 uint32_t AsyncCopyTimeouts();
 
+constexpr int kAABwdRowSlots = 8; // grads rows that reach four consecutive grad_input rows (4 + ceil(3 / scale) + 1)
 struct AABwdPlan {
     bool band;         // band-tiled separable kernel (else one thread per grad_input element)
     int32_t threads;   // block size

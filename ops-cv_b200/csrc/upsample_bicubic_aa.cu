@@ -65,8 +65,10 @@ __global__ void __launch_bounds__(kThreads)
 // ---- forward, streaming (down-scaling) -----------------------------------------------------------------------
 // Per input row r, the outputs whose vertical window covers r form a short run: an output covers r iff its centre lies in
 // [r + 0.5 - support, r + 0.5 + support). Centres are `scale` apart and support is 2 * scale (cubic) or scale (triangle),
-// so for scale >= 1 that is 4 or 2 outputs, one more through rounding: NS = 5 or 3 open sums. The table launch writes, once
+// so for scale >= 1 that is 4 or 2 outputs, one more through rounding (up to kAAMostRows rows: centres and window ends are off
+// by 3/8 at most there, past 2^23 rows by more than one): NS = 5 or 3 open sums. The table launch writes, once
 // per call, one 32-byte record per input row (AATablesAndRangesKernel): the weights of the run, its start and its length.
+constexpr int32_t kAAMostRows = 1 << 22;
 constexpr int kSlots = kAASlots;
 constexpr int kSlotStride = kAASlotStride;
 constexpr int kFlushBatch = 4;        // output rows per horizontal pass of the streaming forward kernel
@@ -514,7 +516,7 @@ __global__ void __launch_bounds__(kThreads)
 // What bounds it is instruction issue: 125 instructions per warp and row (photographs, fp32) while every row walked its
 // own grads rows and sums were single, 68 % of the issue slots busy. 64x3x1024x1024 <-> 224x224 fp32, both directions: 529 -> 463 us.
 constexpr int kBwdRows = 4;     // grad_input rows per synchronisation
-constexpr int kBwdRowSlots = 8; // grads rows that reach four consecutive grad_input rows (4 + ceil(3 / scale) + 1)
+constexpr int kBwdRowSlots = kAABwdRowSlots;
 constexpr int kBwdGroupBytes = (kBwdRowSlots + 1) * 16; // weights of a step, its first grads row and their count
 
 // Rows parked by the VEC = false variant: [kBwdRows][OutPitch] of T.
@@ -759,8 +761,7 @@ AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW, int filte
     // Streaming needs every input row covered by at most NS outputs (true for scale >= 1) and rows that one block can own
     // (four columns per thread). Wider rows and up-scales take a thread per output element.
     const int es = DtSize(dt);
-    plan.stream = scaleH >= 1.0f && sh.win <= 4 * kStreamThreads;
-    if (!plan.stream) {
+    if (!(scaleH >= 1.0f) || sh.win > 4 * kStreamThreads || sh.hin > kAAMostRows) {
         return plan;
     }
     plan.slots = filter == 0 ? 5 : 3;
@@ -772,7 +773,9 @@ AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW, int filte
         return static_cast<int32_t>(std::min<double>(
             sh.hin, std::ceil(static_cast<double>(bandRows) * scaleH + 4.0 * scaleH + 4.0)));
     };
-    // Bands per plane: least time by a model of the walk. A block alone takes a load latency per step (about 0.3 us a
+    constexpr size_t kMostSmem = 96 * 1024; // row buffers and records, beside the horizontal weights where those fit too
+    auto restBytes = [&](int64_t bandRows) { return rowBufs + static_cast<size_t>(metaRows(bandRows)) * recBytes + 32; };
+    // Bands per plane, of those whose records fit: least time by a model of the walk. A block alone takes a load latency per step (about 0.3 us a
     // row with the rows in flight that its registers hold); the blocks of an SM share its issue slots (about 50
     // instructions per warp and row). Every band re-reads the rows of its first window and pays a fixed start.
     const int64_t planes = std::max<int64_t>(sh.n * sh.c, 1);
@@ -780,25 +783,30 @@ AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW, int filte
     double bestTime = 0.0;
     for (int64_t b = 1; b == 1 || (b <= 256 && sh.hout / b >= 4); ++b) {
         const int64_t band = CeilDiv(sh.hout, b);
-        const size_t smem = rowBufs + static_cast<size_t>(metaRows(band)) * recBytes + 64 + (wBytes <= 48 * 1024 ? wBytes : 0);
+        if (restBytes(band) > kMostSmem) {
+            continue;
+        }
+        const size_t smem = restBytes(band) + 32 + (wBytes <= 48 * 1024 ? wBytes : 0);
         const int64_t perSm = std::max<int64_t>(
             1, std::min<int64_t>(1024 / plan.threads, static_cast<int64_t>((225 * 1024) / (smem + 1024))));
         const int64_t blocks = planes * CeilDiv(sh.hout, band);
         const double k = static_cast<double>(CeilDiv(blocks, NumSMs()));
         const double rows = static_cast<double>(metaRows(band)) + 10.0;
         const double time = rows * std::max(0.3 * std::ceil(k / static_cast<double>(perSm)), 0.0065 * k * warps);
-        if (b == 1 || time < bestTime * 0.98) {
+        if (plan.bandRows == 0 || time < bestTime * 0.98) {
             bestTime = time;
             plan.bandRows = static_cast<int32_t>(band);
         }
     }
-    plan.metaRows = metaRows(plan.bandRows);
-    // horizontal weights in shared memory if they fit beside the row buffer and the records
-    const size_t rest = rowBufs + static_cast<size_t>(plan.metaRows) * recBytes + 32;
-    plan.regWeights = wBytes + rest <= 96 * 1024;
-    if (rest > 96 * 1024) {
-        plan.stream = false;
+    if (plan.bandRows == 0) {
+        return plan;
     }
+    plan.stream = true;
+    plan.metaRows = metaRows(plan.bandRows);
+    // Horizontal weights in shared memory if they fit beside the row buffer and the records, of which 32 bytes each count: that
+    // is what a record takes without its weights twice, and 48 bytes must not drive the weights out.
+    const size_t rest = restBytes(plan.bandRows);
+    plan.regWeights = wBytes + rest - static_cast<size_t>(plan.metaRows) * (recBytes - 32) <= kMostSmem;
     plan.wrowBytes = static_cast<uint64_t>(sh.hin) * kSlotStride * sizeof(float);
     // The bulk-copy row ring is off by default: on B200 it measured 15-25 % slower than register prefetch for this
     // kernel (the limiter is the shared-memory data pipe of the horizontal pass, not load latency, and the ring adds
@@ -909,7 +917,7 @@ AABwdPlan MakeAABwdPlan(Dt dt, Shape4 sh, float scaleH, float scaleW, int filter
     AABwdPlan plan{};
     const int es = DtSize(dt);
     // Same covering bound as the forward streaming kernel, on both axes; one block owns whole grad_input rows.
-    plan.band = scaleH >= 1.0f && scaleW >= 1.0f && sh.win <= 4096;
+    plan.band = scaleH >= 1.0f && scaleW >= 1.0f && sh.win <= 4096 && sh.hin <= kAAMostRows;
     if (!plan.band) {
         return plan;
     }

@@ -175,3 +175,65 @@ def test_bicubic_walk_of_random_sizes(ops):
         taken += check_bicubic(ops, rng.choice([2, 4]), rng.randint(1, 3), rng.choice([1, 3, 8]), hi, wi, ho, wo,
                                rng.random() < 0.4, user, rng.choice(["NCHW", "NHWC"]))
     assert taken > 200
+
+
+def aa_windows(n_in, n_out, cubic, align):
+    """Per output index: first input index of its window and one past the last."""
+    scale = (F(n_in - 1) / F(n_out - 1) if n_out > 1 else F(0)) if align else F(n_in) / F(n_out)
+    support = (F(2) if cubic else F(1)) * max(scale, F(1))
+    centre = scale * (np.arange(n_out).astype(F) + F(0.5))
+    lo = np.maximum(np.floor((centre - support) + F(0.5)).astype(np.int64), 0)
+    hi = np.minimum(np.floor((centre + support) + F(0.5)).astype(np.int64), n_in)
+    return lo, np.maximum(hi, lo)
+
+
+def covering(lo, hi, n_in, span):
+    """Most windows that reach `span` adjacent input indices, over all places."""
+    y = np.arange(n_in)
+    start, end = np.searchsorted(hi, y, side="right"), np.searchsorted(lo, y, side="right")
+    last = np.minimum(y + span - 1, n_in - 1)
+    return int((end[last] - start).max())
+
+
+def check_aa(ops, cubic, n, c, hi, wi, ho, wo, align):
+    name = "bicubic" if cubic else "bilinear"
+    lo, top = aa_windows(hi, ho, cubic, align)
+    forward = ops.debug_plan(name + "_aa_forward_stream", 4, (n, c, hi, wi, ho, wo), "NCHW", align)
+    if forward is not None:
+        band, rows, slots = forward[:3]
+        assert covering(lo, top, hi, 1) <= slots
+        first = np.arange(0, ho, band)
+        assert int((top[np.minimum(first + band, ho) - 1] - lo[first]).max()) <= rows
+    backward = ops.debug_plan(name + "_aa_backward_band", 4, (n, c, hi, wi, ho, wo), "NCHW", align)
+    if backward is not None:
+        band, rows, row_slots, col_slots = backward[:4]
+        assert covering(lo, top, hi, 4) <= row_slots
+        assert covering(lo, top, hi, band) <= rows
+        assert covering(*aa_windows(wi, wo, cubic, align), wi, 4) <= col_slots
+        assert covering(*aa_windows(wi, wo, cubic, align), wi, 1) <= 5
+    return forward is not None, backward is not None
+
+
+@pytest.mark.parametrize("cubic", [True, False])
+@pytest.mark.parametrize("hi,ho", [(1 << 22, 1 << 22), ((1 << 22) - 3, 4100001), (4000000, 1300000), (1 << 23, 8388605),
+                                   (16700001, 16690007), ((1 << 24) - 1, 9000001), (25000000, 20000000)])
+def test_aa_kernels_of_long_axes(ops, cubic, hi, ho):
+    """Past 2^23 rows centres round by so much that an input row can feed more outputs than the kernels keep open."""
+    for align in (False, True):
+        check_aa(ops, cubic, 1, 1, hi, 8, ho, 2, align)
+
+
+def test_aa_kernels_of_random_sizes(ops):
+    rng = random.Random(9)
+    for _ in range(400):
+        hi, wi = int(2 ** rng.uniform(0, 12)), int(2 ** rng.uniform(0, 12))
+        s = 2 ** rng.uniform(0, 4)
+        check_aa(ops, rng.random() < 0.5, rng.randint(1, 64), rng.choice([1, 3, 8]), hi, wi, max(1, int(hi / s)),
+                 max(1, int(wi / (s * rng.uniform(0.9, 1.1)))), rng.random() < 0.3)
+
+
+def test_aa_stream_takes_bands_that_fit(ops):
+    """The band that the model of the walk likes best may need more shared memory than there is: another one is taken."""
+    assert ops.debug_plan("bilinear_aa_forward_stream", 4, (33, 8, 2397, 1331, 508, 282)) is not None
+    wide = ops.debug_plan("bicubic_aa_forward_stream", 4, (62, 3, 2110, 1864, 875, 773))
+    assert wide is not None and wide[4] == 1  # and the horizontal weights stay in shared memory
