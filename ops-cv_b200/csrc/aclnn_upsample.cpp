@@ -1345,7 +1345,7 @@ static aclnnStatus PlanAAForward(const char* api, int filter, const aclTensor* x
     const Dt dt = ToDt(x->dtype);
     const AxisGeom gh{sh.hin, sh.hout, ah.scale}, gw{sh.win, sh.wout, aw.scale};
     const AAOffsets oh = AllocAA(ws, sh.hout, ah.taps), ow = AllocAA(ws, sh.wout, aw.taps);
-    const AAFwdPlan plan = MakeAAFwdPlan(dt, sh, ah.scale, aw.taps, filter);
+    const AAFwdPlan plan = MakeAAFwdPlan(dt, sh, ah.scale, ah.taps, aw.taps, filter);
     const RangeOffsets rh = AllocRange(ws, sh.hin), rw = AllocRange(ws, sh.win);
     const uint64_t wrowOff = ws.Alloc(plan.wrowBytes);
     ex->steps.push_back([=](char* w, cudaStream_t s) {
@@ -2014,7 +2014,7 @@ aclnnStatus opscvDebugPlan(int32_t kind, int32_t elemSize, aclFormat format, con
             const AAGeom ah = MakeAAGeom(in.h, out.h, align, scales[0], filter == 1 || !forward, filter);
             const AAGeom aw = MakeAAGeom(in.w, out.w, align, scales[1], filter == 1 || !forward, filter);
             if (forward) {
-                const AAFwdPlan p = MakeAAFwdPlan(dt, sh, ah.scale, aw.taps, filter);
+                const AAFwdPlan p = MakeAAFwdPlan(dt, sh, ah.scale, ah.taps, aw.taps, filter);
                 const int64_t v[8] = {p.bandRows, p.metaRows, p.slots, 0, p.regWeights ? 1 : 0, 0, 0, 0};
                 std::copy(v, v + 8, values);
                 *taken = p.stream ? 1 : 0;

@@ -175,7 +175,7 @@ struct AAFwdPlan {
     int32_t bandRows;   // output rows per block
     uint64_t wrowBytes; // workspace for the per-input-row vertical weights
 };
-AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW, int filter);
+AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsH, int32_t tapsW, int filter);
 // wrow (records of the input rows) is only used by the streaming kernel.
 cudaError_t BicubicAAFwd(Dt dt, const void* x, void* y, Shape4 sh, AAAxis th, AAAxis tw, const float* wrow,
                          const AAFwdPlan& plan, cudaStream_t s);

@@ -755,13 +755,36 @@ __global__ void __launch_bounds__(kThreads)
 
 } // namespace
 
-AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW, int filter)
+// The streaming and the band kernel own whole rows with 64 or 128 threads at least: little work and narrow rows (planes of a few
+// columns) are done sooner by a thread per element. Both sides beyond the fixed part of a call (tables, launches), in
+// microseconds, from sweeps of 2 to 63 columns by 256 rows, 3 to 300 planes, scales of 1.4 and 4, both filters:
+//   forward, thread per output: 0.6 to 1 ns per thousand taps, and the chain of one window; streaming: its start, and its rows.
+//   300 planes of 3 columns 256 -> 182 rows, cubic: 10 us against 45; 31 columns 43 against 47; 63 columns 79 against 49.
+//   48 planes 240x248 -> 72x77, triangle: 27 us against 17.
+static bool StreamPays(const Shape4& sh, int32_t tapsH, int32_t tapsW, int filter)
+{
+    const double planes = static_cast<double>(sh.n) * sh.c, taps = static_cast<double>(tapsH) * tapsW;
+    const double outputs = planes * sh.hout * sh.wout;
+    const double elements = std::max(1e-6 * outputs * taps * (0.6 + 0.0012 * taps) * (filter == 0 ? 1.0 : 1.4), 0.06 * taps);
+    return elements > 4.5 + 3.0 * std::min(1.0, sh.hin / 256.0) + 0.3e-3 * planes * sh.hin;
+}
+//   backward, thread per grad_input element: 40 (cubic) or 16 ns per thousand elements and the chain of its taps; band: as above.
+//   300 planes of 3 columns: 19 us against 47 (cubic); 13 columns 62 against 49; triangle 25 columns 41 against 39.
+static bool BandPays(const Shape4& sh, int filter)
+{
+    const double planes = static_cast<double>(sh.n) * sh.c;
+    const double inputs = planes * sh.hin * sh.win;
+    const double elements = std::max(1e-6 * inputs * (filter == 0 ? 40.0 : 16.0), filter == 0 ? std::min(5.0, 1.0 * sh.wout) : 1.0);
+    return elements > 3.0 + 0.3e-3 * planes * sh.hin;
+}
+
+AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsH, int32_t tapsW, int filter)
 {
     AAFwdPlan plan{};
     // Streaming needs every input row covered by at most NS outputs (true for scale >= 1) and rows that one block can own
     // (four columns per thread). Wider rows and up-scales take a thread per output element.
     const int es = DtSize(dt);
-    if (!(scaleH >= 1.0f) || sh.win > 4 * kStreamThreads || sh.hin > kAAMostRows) {
+    if (!(scaleH >= 1.0f) || sh.win > 4 * kStreamThreads || sh.hin > kAAMostRows || !StreamPays(sh, tapsH, tapsW, filter)) {
         return plan;
     }
     plan.slots = filter == 0 ? 5 : 3;
@@ -781,7 +804,7 @@ AAFwdPlan MakeAAFwdPlan(Dt dt, Shape4 sh, float scaleH, int32_t tapsW, int filte
     const int64_t planes = std::max<int64_t>(sh.n * sh.c, 1);
     const double warps = plan.threads / 32;
     double bestTime = 0.0;
-    for (int64_t b = 1; b == 1 || (b <= 256 && sh.hout / b >= 4); ++b) {
+    for (int64_t b = 1; b == 1 || sh.hout / b >= 4; b += b < 256 ? 1 : b / 16) {
         const int64_t band = CeilDiv(sh.hout, b);
         if (restBytes(band) > kMostSmem) {
             continue;
@@ -917,7 +940,7 @@ AABwdPlan MakeAABwdPlan(Dt dt, Shape4 sh, float scaleH, float scaleW, int filter
     AABwdPlan plan{};
     const int es = DtSize(dt);
     // Same covering bound as the forward streaming kernel, on both axes; one block owns whole grad_input rows.
-    plan.band = scaleH >= 1.0f && scaleW >= 1.0f && sh.win <= 4096 && sh.hin <= kAAMostRows;
+    plan.band = scaleH >= 1.0f && scaleW >= 1.0f && sh.win <= 4096 && sh.hin <= kAAMostRows && BandPays(sh, filter);
     if (!plan.band) {
         return plan;
     }

@@ -106,3 +106,38 @@ def test_long_axes(ops, oracle, dev, dtype, filt, shape):
     gi = bwd(g, (oh, ow), (n, c, h, w), False)
     assert ops.launch_count() == (3 if max(shape) > 8192 else 2)
     close(gi, obwd(g32, (h, w), False, definition="gather"), dtype)
+
+
+# Sizes at which the streaming forward and the band backward take the call (small calls go to a thread per element): every load
+# width, a block's last thread partly used, the widest rows, scales just above one
+REACHED = [("bicubic", "forward", (1, 2, 33, 63, 5, 9)), ("bicubic", "forward", (1, 2, 40, 62, 8, 12)),
+           ("bicubic", "forward", (1, 3, 37, 64, 11, 17)), ("bicubic", "forward", (1, 1, 7, 2047, 2, 341)),
+           ("bicubic", "forward", (1, 1, 9, 2048, 3, 400)), ("bicubic", "forward", (64, 1, 100, 96, 99, 95)),
+           ("bicubic", "forward", (64, 1, 64, 130, 31, 129)), ("bicubic", "forward", (3, 1, 700, 5, 30, 1)),
+           ("bilinear", "forward", (1, 3, 64, 130, 11, 23)), ("bilinear", "forward", (1, 2, 60, 61, 10, 10)),
+           ("bilinear", "forward", (2, 2, 36, 64, 6, 12)), ("bilinear", "forward", (1, 1, 40, 2047, 6, 341)),
+           ("bilinear", "forward", (256, 1, 100, 96, 99, 95)), ("bicubic", "backward", (1, 2, 33, 63, 5, 9)),
+           ("bicubic", "backward", (1, 1, 12, 4095, 4, 1365)), ("bicubic", "backward", (1, 1, 100, 96, 99, 95)),
+           ("bilinear", "backward", (64, 1, 100, 96, 99, 95)), ("bilinear", "backward", (64, 1, 20, 513, 3, 100)),
+           ("bilinear", "backward", (16, 1, 12, 4095, 4, 1365)), ("bilinear", "backward", (128, 2, 37, 62, 11, 17))]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("filt,way,shape", REACHED)
+def test_streaming_and_band_kernels(ops, oracle, dev, dtype, filt, way, shape):
+    n, c, h, w, oh, ow = shape
+    kernel = f"{filt}_aa_forward_stream" if way == "forward" else f"{filt}_aa_backward_band"
+    assert ops.debug_plan(kernel, 4 if dtype == torch.float32 else 2, shape) is not None
+    if way == "forward":
+        x, x32 = quant(torch.rand((n, c, h, w), generator=gen(100)), dtype)
+        ref = getattr(oracle, f"{filt}_aa_fwd")(x32, (oh, ow), False)
+        for shift in (0, 1, 2):
+            close(getattr(ops, f"upsample_{filt}2d_aa")(off_by(x, dev, shift), (oh, ow), False), ref, dtype)
+        return
+    bwd = ops.upsample_bicubic2d_aa_grad if filt == "bicubic" else ops.upsample_bilinear2d_aa_backward
+    g, g32 = quant(torch.rand((n, c, oh, ow), generator=gen(101)), dtype)
+    ref = getattr(oracle, f"{filt}_aa_bwd")(g32, (h, w), False, definition="gather")
+    for shift in (0, 1, 3):
+        out = off_by(torch.full((n, c, h, w), 7.0, dtype=dtype), dev, shift)
+        bwd(g.to(dev), (oh, ow), (n, c, h, w), False, out=out)
+        close(out, ref, dtype)
