@@ -7,7 +7,7 @@
 // Backward: image/grid_sampler3_d_grad/op_kernel/arch35/grid_sampler3_d_grad_simt.h:43-300 with the coordinate
 // helpers of grid_sampler3_d_grad_simt_base.h:46-168 (the ones the 2-D backward uses). grad_input is accumulated
 // with fp32 atomics (in place for fp32 tensors, in a workspace that is cast afterwards for 16-bit ones); grad_grid
-// is one thread's sum over the channels in the reference's corner and channel order. Channels-last tensors of sixteen or more
+// is one thread's sum over the channels in the reference's corner and channel order. Channels-last tensors of many
 // channels take grad_input in a launch of its own with a point's channel vectors on adjacent lanes.
 #include <algorithm>
 
@@ -434,9 +434,13 @@ cudaError_t GridSampler3dBwd(Dt dt, const void* go, const void* x, const void* g
         const unsigned grid1 = GridFor(total, kThreads);
         int32_t wi = wantInput ? 1 : 0;
         const int32_t wg = wantGrid ? 1 : 0;
-        // Four or more vectors per point: grad_input by lanes, grad_grid by points. With fewer, adjacent points share the
-        // lines of a tap about as well as adjacent lanes do, and grad_output would be read twice for nothing.
-        if (g.cl && v == 4 && wantInput && g.c >= 16) {
+        // Many vectors per point: grad_input by lanes, grad_grid by points. With few, adjacent points share the lines of a tap
+        // about as well as adjacent lanes do, and the second launch and the second look at grad_output cost more than that
+        // gives; so do small volumes, whose reductions are few, and more so in 16-bit types. Backward of NDHWC, us, one launch
+        // and two: fp32 12x24x24, 16 channels 17.5 / 18.6, 24 21.7 / 23.9, 32 28.5 / 26.7; 32x64x64, 16 channels 44.8 / 43.2;
+        // fp16 16x40x40, 32 channels 32.8 / 34.9, 64 53.5 / 51.4; 32x64x64, 24 channels 59.6 / 61.7, 32 81.3 / 75.0.
+        const int32_t fewest = (sizeof(T) == 4 ? 16 : 32) << (total < 65536 ? 1 : 0);
+        if (g.cl && v == 4 && wantInput && g.c >= fewest) {
             const int32_t groups = static_cast<int32_t>(g.c / 4);
             GridSampler3dScatterLanesKernel<T><<<GridFor(total * groups, kThreads), kThreads, 0, s>>>(pgo, pg, acc, g, groups);
             if (wg != 0) {

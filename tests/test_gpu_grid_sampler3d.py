@@ -164,3 +164,33 @@ def test_channels_last_copies_at_ragged_volumes(ops, oracle, dev, dtype, c, vol)
         ri, rg = oracle.grid_sampler3d_bwd(go32, x32, g32, 0, 0, False)
         np.testing.assert_allclose(gi.cpu().numpy(), ri, rtol=1e-5, atol=1e-6 * max(1.0, float(np.abs(ri).max())))
         assert np.array_equal(gg.cpu().numpy(), rg)
+
+
+# (dtype, channels, output volume): on either side of the lines at which grad_input gets a launch of its own
+@pytest.mark.parametrize("dtype,c,vol,lanes", [(torch.float32, 28, (3, 7, 9), False), (torch.float32, 32, (3, 7, 9), True),
+                                               (torch.float32, 16, (16, 64, 65), True), (torch.float32, 12, (16, 64, 65), False),
+                                               (torch.float16, 60, (3, 7, 9), False), (torch.float16, 64, (3, 7, 9), True),
+                                               (torch.float16, 32, (16, 64, 65), True), (torch.bfloat16, 28, (16, 64, 65), False)])
+def test_backward_by_lanes_or_by_points(ops, oracle, dev, dtype, c, vol, lanes):
+    do, ho, wo = vol
+    x, x32 = quant(torch.randn((1, 16, 20, 22, c), generator=gen(133)), dtype)
+    grid, g32 = quant(make_grid(1, do, ho, wo, 134), dtype)
+    go, go32 = quant(torch.randn((1, do, ho, wo, c), generator=gen(135)), dtype)
+    xd, gd, god = x.to(dev), grid.to(dev), go.to(dev)
+
+    def launches(mask):
+        ops.reset_launch_count()
+        out = ops.grid_sampler3d_backward(god, xd, gd, 0, 0, False, mask=mask, fmt="NDHWC")
+        return out, ops.launch_count()
+
+    (gi, gg), both = launches((True, True))
+    (_, gg_alone), grid_alone = launches((False, True))
+    casts = 0 if dtype == torch.float32 else 1
+    assert both - grid_alone == 1 + casts + (1 if lanes else 0)  # zeroing, the cast, the launch by lanes
+    assert torch.equal(gg, gg_alone)
+    ncdhw = (0, 4, 1, 2, 3)
+    ri, rg = oracle.grid_sampler3d_bwd(go32.transpose(ncdhw), x32.transpose(ncdhw), g32, 0, 0, False)
+    ulp = {torch.float32: 0.0, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+    for got, ref in ((gi.float().cpu().numpy().transpose(ncdhw), ri), (gg.float().cpu().numpy(), rg)):
+        bar = (1e-5 + ulp) * np.abs(ref) + 4e-6 * max(1.0, float(np.abs(ref).max())) + (2.0 ** -25 if ulp else 0.0)
+        assert (np.abs(got - ref) <= bar).all(), float((np.abs(got - ref) - bar).max())
