@@ -39,7 +39,7 @@ def native():
     global _native
     if _native is None:
         module = native_module()
-        module.set_error_class(AclnnError)
+        module.set_classes(AclnnError, Workspace)
         _native = module
     return _native
 
@@ -311,20 +311,20 @@ def resize(x, scales, mode="bilinear", fmt="NCHW", out=None, workspace=None):
 
 
 def grid_sampler2d(x, grid, interpolation=0, padding=0, align_corners=False, out=None, workspace=None):
-    return native().grid_sampler(x, grid, interpolation, padding, align_corners, None, out, workspace)
+    return native().grid_sampler(x, grid, int(interpolation), int(padding), align_corners, None, out, workspace)
 
 
 def grid_sampler2d_backward(grad_out, x, grid, interpolation=0, padding=0, align_corners=False, mask=(True, True),
                             input_grad=None, grid_grad=None, workspace=None):
-    return native().grid_sampler_backward(grad_out, x, grid, interpolation, padding, align_corners, mask, None,
+    return native().grid_sampler_backward(grad_out, x, grid, int(interpolation), int(padding), align_corners, mask, None,
                                           input_grad, grid_grad, workspace)
 
 
 def grid_sampler3d(x, grid, interpolation=0, padding=0, align_corners=False, fmt="NCDHW", out=None, workspace=None):
-    return native().grid_sampler(x, grid, interpolation, padding, align_corners, fmt, out, workspace)
+    return native().grid_sampler(x, grid, int(interpolation), int(padding), align_corners, fmt, out, workspace)
 
 
 def grid_sampler3d_backward(grad_out, x, grid, interpolation=0, padding=0, align_corners=False, mask=(True, True),
                             fmt="NCDHW", input_grad=None, grid_grad=None, workspace=None):
-    return native().grid_sampler_backward(grad_out, x, grid, interpolation, padding, align_corners, mask, fmt,
+    return native().grid_sampler_backward(grad_out, x, grid, int(interpolation), int(padding), align_corners, mask, fmt,
                                           input_grad, grid_grad, workspace)

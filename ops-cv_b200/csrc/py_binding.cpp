@@ -19,6 +19,7 @@
 namespace {
 
 PyObject* g_error = nullptr; // AclnnError(api, status)
+PyObject* g_workspace = nullptr; // aclnn.Workspace
 PyObject* g_bufName = nullptr;
 
 // Thrown after a Python exception has been set.
@@ -50,12 +51,17 @@ int64_t IntOf(PyObject* o)
     }
     return v;
 }
-double DoubleOf(PyObject* o)
+double DoubleOf(PyObject* o) // float(o)
 {
-    const double v = PyFloat_AsDouble(o);
-    if (v == -1.0 && PyErr_Occurred()) {
+    if (PyFloat_CheckExact(o)) {
+        return PyFloat_AS_DOUBLE(o);
+    }
+    PyObject* f = PyNumber_Float(o);
+    if (f == nullptr) {
         throw Raised{};
     }
+    const double v = PyFloat_AS_DOUBLE(f);
+    Py_DECREF(f);
     return v;
 }
 bool BoolOf(PyObject* o)
@@ -171,8 +177,53 @@ struct NoGil {
     ~NoGil() { PyEval_RestoreThread(state); }
 };
 
-// Both phases: `first` runs the first phase, `second` is the entry point of the second. The workspace is the caller's
-// (an object with `buf` and `get`, see aclnn.Workspace) or a fresh allocation.
+// The caller's workspace for `size` bytes: the buffer of an aclnn.Workspace as it is where it is large enough, else the first
+// item of what `get(size)` of any object returns: a tensor, another object with data_ptr(), or None. *keep owns it.
+struct Held {
+    PyObject* o = nullptr;
+    ~Held() { Py_XDECREF(o); }
+};
+void* CallersBuffer(PyObject* workspace, uint64_t size, Held* keep)
+{
+    if (reinterpret_cast<PyObject*>(Py_TYPE(workspace)) == g_workspace) {
+        keep->o = PyObject_GetAttr(workspace, g_bufName);
+        if (keep->o == nullptr) {
+            throw Raised{};
+        }
+        if (THPVariable_Check(keep->o) && static_cast<uint64_t>(THPVariable_Unpack(keep->o).numel()) >= size) {
+            return THPVariable_Unpack(keep->o).data_ptr();
+        }
+        Py_CLEAR(keep->o);
+    }
+    PyObject* got = PyObject_CallMethod(workspace, "get", "K", static_cast<unsigned long long>(size));
+    if (got == nullptr) {
+        throw Raised{};
+    }
+    keep->o = PySequence_GetItem(got, 0);
+    Py_DECREF(got);
+    if (keep->o == nullptr) {
+        throw Raised{};
+    }
+    if (keep->o == Py_None) {
+        return nullptr;
+    }
+    if (THPVariable_Check(keep->o)) {
+        return THPVariable_Unpack(keep->o).data_ptr();
+    }
+    PyObject* at = PyObject_CallMethod(keep->o, "data_ptr", nullptr);
+    if (at == nullptr) {
+        throw Raised{};
+    }
+    void* p = PyLong_AsVoidPtr(at);
+    Py_DECREF(at);
+    if (p == nullptr && PyErr_Occurred()) {
+        throw Raised{};
+    }
+    return p;
+}
+
+// Both phases: `first` runs the first phase, `second` is the entry point of the second. The workspace is the caller's or a
+// fresh allocation.
 template <typename First>
 void TwoPhase(const char* name, First first, decltype(&aclnnUpsampleNearest2d) second, const at::Device& device,
               PyObject* workspace)
@@ -188,31 +239,15 @@ void TwoPhase(const char* name, First first, decltype(&aclnnUpsampleNearest2d) s
         RaiseStatus(std::string(name) + "GetWorkspaceSize", status);
     }
     at::Tensor fresh;
+    Held held;
     void* buffer = nullptr;
     try {
         if (size > 0 && workspace != Py_None) {
-            PyObject* held = PyObject_GetAttr(workspace, g_bufName);
-            if (held == nullptr) {
-                throw Raised{};
-            }
-            if (!THPVariable_Check(held) || static_cast<uint64_t>(THPVariable_Unpack(held).numel()) < size) {
-                Py_DECREF(held);
-                PyObject* got = PyObject_CallMethod(workspace, "get", "K", static_cast<unsigned long long>(size));
-                if (got == nullptr) {
-                    throw Raised{};
-                }
-                held = PySequence_GetItem(got, 0);
-                Py_DECREF(got);
-                if (held == nullptr) {
-                    throw Raised{};
-                }
-            }
-            fresh = TensorOf(held);
-            Py_DECREF(held);
+            buffer = CallersBuffer(workspace, size, &held);
         } else if (size > 0) {
             fresh = at::empty({static_cast<int64_t>(size)}, at::TensorOptions().dtype(at::kByte).device(device));
+            buffer = fresh.data_ptr();
         }
-        buffer = fresh.defined() ? fresh.data_ptr() : nullptr;
         if (!device.is_cuda()) {
             Raise(PyExc_ValueError, "expected a cuda device");
         }
@@ -596,16 +631,22 @@ PyObject* Entry(PyObject*, PyObject* const* args, Py_ssize_t n)
 #define OPSCV_METHOD(name, fn, count) \
     {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(Entry<fn, count>)), METH_FASTCALL, nullptr}
 
-PyObject* SetErrorClass(PyObject*, PyObject* cls)
+// (AclnnError, Workspace)
+PyObject* SetClasses(PyObject*, PyObject* const* args, Py_ssize_t n)
 {
-    Py_XDECREF(g_error);
-    Py_INCREF(cls);
-    g_error = cls;
+    if (n != 2) {
+        PyErr_Format(PyExc_TypeError, "expected 2 arguments, got %zd", n);
+        return nullptr;
+    }
+    Py_INCREF(args[0]);
+    Py_INCREF(args[1]);
+    Py_XSETREF(g_error, args[0]);
+    Py_XSETREF(g_workspace, args[1]);
     Py_RETURN_NONE;
 }
 
 PyMethodDef kMethods[] = {
-    {"set_error_class", SetErrorClass, METH_O, nullptr},
+    {"set_classes", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(SetClasses)), METH_FASTCALL, nullptr},
     OPSCV_METHOD("upsample_nearest2d", Nearest2d, 6),
     OPSCV_METHOD("upsample_nearest2d_backward", Nearest2dBackward, 7),
     OPSCV_METHOD("upsample_nearest_exact2d", NearestExact2d, 6),
