@@ -504,7 +504,9 @@ aclnnStatus PlanTrilinearBwd(const char* api, const aclTensor* gradOut, const ac
         offW[a] = ws.Alloc(sizeof(float) * static_cast<uint64_t>(ins[a]) * static_cast<uint64_t>(taps[a]));
     }
     const Dt dt = ToDt(gradOut->dtype);
-    const uint64_t stageOff = ws.Alloc(Trilinear3dBwdWorkspace(g, cl ? gi.n : gi.n * gi.c));
+    const int64_t planes = cl ? gi.n : gi.n * gi.c;
+    const bool byPlanes = Trilinear3dBwdByPlanes(dt, g, taps, planes);
+    const uint64_t stageOff = ws.Alloc(Trilinear3dBwdWorkspace(g, planes, byPlanes));
     ex->steps.push_back([=](char* w, cudaStream_t s) {
         TrilinearBwdTables t;
         for (int a = 0; a < 3; ++a) {
@@ -517,7 +519,7 @@ aclnnStatus PlanTrilinearBwd(const char* api, const aclTensor* gradOut, const ac
         if (e != cudaSuccess) {
             return e;
         }
-        return Trilinear3dBwd(dt, g0.At(w), y.At(w), reinterpret_cast<float*>(w + stageOff), g, t, s);
+        return Trilinear3dBwd(dt, g0.At(w), y.At(w), reinterpret_cast<float*>(w + stageOff), g, t, byPlanes, s);
     });
     FinishOutput(gradInput, y, ex);
     ex->workspaceSize = ws.Size();

@@ -466,7 +466,7 @@ void LaunchAxis(const T* x, T* y, const Trilinear3dGeom& g, const RowLaunch& rl,
 // of grad_input rows of it, copies the slice's rows into shared memory as they are (asynchronous 16-byte copies), forms
 // the W sums of those rows there and the H sums from them: the sums of the two stage kernels in the same order, so the
 // bits are theirs. The W stage's buffer, the largest of the operator (fp16 2x32 planes 32x56x56 <- 64x112x112: 103 MB
-// written and read again, more than the L2 keeps), is gone, and a tap is a shared-memory read instead of a 2-byte global
+// written and read again, more than the L2 keeps), is gone, from the workspace as well, and a tap is a shared-memory read instead of a 2-byte global
 // load. What bounds it is instruction issue on the taps (76 % of the slots). At those sizes: 95 us in two kernels -> 59 us.
 struct PlaneShape {
     int64_t slices;
@@ -598,13 +598,14 @@ __global__ void __launch_bounds__(kThreads, 4)
 }
 
 // Shape and shared memory of the plane kernel; false where a band of at least eight rows (or all of them) does not fit
-// 56 KB (four blocks per SM). More bands than that asks for where slices alone leave SMs idle.
-bool PlanPlane(const Trilinear3dGeom& g, const TrilinearBwdTables& t, int es, int64_t slices, PlaneShape* out, size_t* smem)
+// 56 KB (four blocks per SM). More bands than that asks for where slices alone leave SMs idle. The bound on a band's
+// grad_output rows holds while an index is exact in fp32.
+bool PlanPlane(const Trilinear3dGeom& g, const int32_t (&taps)[3], int es, int64_t slices, PlaneShape* out, size_t* smem)
 {
-    if (g.chan != 1 || t.taps[2] > 10 || t.taps[1] > 64) {
+    if (g.chan != 1 || taps[2] > 10 || taps[1] > 64 || g.ho > (1 << 24) || g.hi > (1 << 24)) {
         return false;
     }
-    PlaneShape p{slices, g.ho, g.wo, g.hi, g.wi, 0, 0, 0, t.taps[1], t.taps[2]};
+    PlaneShape p{slices, g.ho, g.wo, g.hi, g.wi, 0, 0, 0, taps[1], taps[2]};
     // grad_output rows of a band: source positions are scale apart
     const double perRow = g.sh > 0.0f ? 1.0 / static_cast<double>(g.sh) : static_cast<double>(g.ho);
     for (int32_t nb = 1; nb <= g.hi; ++nb) {
@@ -612,9 +613,9 @@ bool PlanPlane(const Trilinear3dGeom& g, const TrilinearBwdTables& t, int es, in
         if (nb > 1 && band < 8) {
             return p.bands > 0;
         }
-        const int32_t cap = static_cast<int32_t>(std::min<double>(g.ho, std::ceil((band + 2) * perRow) + t.taps[1] + 4));
+        const int32_t cap = static_cast<int32_t>(std::min<double>(g.ho, std::ceil((band + 2) * perRow) + taps[1] + 4));
         const size_t need = static_cast<size_t>(PlaneRawBytes(cap, g.wo, es)) +
-                            (static_cast<size_t>((cap * g.wi + 3) & ~3) + static_cast<size_t>(band) * (t.taps[1] + 2)) * 4;
+                            (static_cast<size_t>((cap * g.wi + 3) & ~3) + static_cast<size_t>(band) * (taps[1] + 2)) * 4;
         if (static_cast<int64_t>(cap) * (static_cast<int64_t>(g.wo) * es + static_cast<int64_t>(g.wi) * 4) > 56 * 1024 ||
             need > 60 * 1024) {
             continue;
@@ -745,16 +746,23 @@ cudaError_t BuildTrilinearBwdTables(TrilinearBwdTables t, Trilinear3dGeom g, cud
     return cudaGetLastError();
 }
 
-uint64_t Trilinear3dBwdWorkspace(const Trilinear3dGeom& g, int64_t planes)
+bool Trilinear3dBwdByPlanes(Dt dt, const Trilinear3dGeom& g, const int32_t (&taps)[3], int64_t planes)
 {
-    // after the W stage: planes * dout * ho * wi; after the H stage: planes * dout * hi * wi
-    const uint64_t t1 = static_cast<uint64_t>(planes) * g.dout * g.ho * g.wi * g.chan * sizeof(float);
+    PlaneShape ps;
+    size_t smem = 0;
+    return PlanPlane(g, taps, DtSize(dt), planes * g.dout, &ps, &smem);
+}
+
+uint64_t Trilinear3dBwdWorkspace(const Trilinear3dGeom& g, int64_t planes, bool byPlanes)
+{
+    // after the W stage (none of its own in the plane kernel): planes * dout * ho * wi; after the H stage: planes * dout * hi * wi
+    const uint64_t t1 = byPlanes ? 0 : static_cast<uint64_t>(planes) * g.dout * g.ho * g.wi * g.chan * sizeof(float);
     const uint64_t t2 = static_cast<uint64_t>(planes) * g.dout * g.hi * g.wi * g.chan * sizeof(float);
     return ((t1 + 255) & ~static_cast<uint64_t>(255)) + t2;
 }
 
 cudaError_t Trilinear3dBwd(Dt dt, const void* go, void* gi, float* stage, Trilinear3dGeom g, TrilinearBwdTables t,
-                           cudaStream_t s)
+                           bool byPlanes, cudaStream_t s)
 {
     const int64_t planes = g.rows / (static_cast<int64_t>(g.di) * g.hi);
     const uint64_t t1Bytes = static_cast<uint64_t>(planes) * g.dout * g.ho * g.wi * g.chan * sizeof(float);
@@ -763,15 +771,18 @@ cudaError_t Trilinear3dBwd(Dt dt, const void* go, void* gi, float* stage, Trilin
     OPSCV_DISPATCH_DT(dt, T, {
         // W: (planes * dout * ho) x wo x chan -> wi;  H: (planes * dout) x ho x (wi * chan) -> hi;  D: planes x dout x
         // (hi * wi * chan) -> di
-        PlaneShape ps;
-        size_t smem = 0;
-        if (PlanPlane(g, t, static_cast<int>(sizeof(T)), planes * g.dout, &ps, &smem)) {
+        if (byPlanes) {
+            PlaneShape ps;
+            size_t smem = 0;
+            if (!PlanPlane(g, t.taps, static_cast<int>(sizeof(T)), planes * g.dout, &ps, &smem)) {
+                return cudaErrorInvalidConfiguration; // the same question had another answer when the workspace was sized
+            }
             const T* pg = static_cast<const T*>(go);
-            const cudaError_t e = g.wi % 4 == 0 ? LaunchPlane<T, 4>(pg, t2, ps, t, smem, s) : LaunchPlane<T, 1>(pg, t2, ps, t, smem, s);
+            const cudaError_t e = g.wi % 4 == 0 ? LaunchPlane<T, 4>(pg, stage, ps, t, smem, s) : LaunchPlane<T, 1>(pg, stage, ps, t, smem, s);
             if (e != cudaSuccess) {
                 return e;
             }
-            LaunchBwdStage<float, T>(t2, static_cast<T*>(gi), planes, g.dout, g.di,
+            LaunchBwdStage<float, T>(stage, static_cast<T*>(gi), planes, g.dout, g.di,
                                      static_cast<int64_t>(g.hi) * g.wi * g.chan, t.start[0], t.count[0], t.w[0], t.taps[0], s);
             return cudaGetLastError();
         }

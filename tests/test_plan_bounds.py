@@ -1,10 +1,12 @@
 """The bounds that launch shapes are sized by, against a restatement of the kernels' index arithmetic: a block's shared memory
 holds what its rows, columns or windows can ask for. Host arithmetic only (opscvDebugPlan), no GPU."""
+import ctypes
 import random
 import time
 
 import numpy as np
 import pytest
+import torch
 
 F = np.float32
 
@@ -237,3 +239,26 @@ def test_aa_stream_takes_bands_that_fit(ops):
     assert ops.debug_plan("bilinear_aa_forward_stream", 4, (33, 8, 2397, 1331, 508, 282)) is not None
     wide = ops.debug_plan("bicubic_aa_forward_stream", 4, (62, 3, 2110, 1864, 875, 773))
     assert wide is not None and wide[4] == 1  # and the horizontal weights stay in shared memory
+
+
+def workspace_size(ops, name, *args):
+    ws, ex = ctypes.c_uint64(0), ctypes.c_void_p(None)
+    status = getattr(ops.lib(), name + "GetWorkspaceSize")(*args, ctypes.byref(ws), ctypes.byref(ex))
+    assert status == 0
+    assert ops.lib().aclDestroyAclOpExecutor(ex) == 0
+    return ws.value
+
+
+@pytest.mark.parametrize("shape,stages", [((2, 8, 8, 28, 28, 16, 56, 56), 1), ((1, 2, 4, 3, 5, 4, 200, 5), 2),
+                                          ((1, 2, 4, 4, 4, 4, 8, 50), 2)])
+def test_trilinear_backward_asks_for_the_scratch_that_it_uses(ops, shape, stages):
+    """By planes only the sums of the H stage go through memory; with longer lists of taps those of the W stage as well."""
+    n, c, di, hi, wi, do, ho, wo = shape
+    grad, gi = torch.zeros((n, c, do, ho, wo), dtype=torch.float16), torch.zeros((n, c, di, hi, wi), dtype=torch.float16)
+    tg, ti = ops.acl_tensor(grad, "NCDHW"), ops.acl_tensor(gi, "NCDHW")
+    osz, isz = ops.int_array([do, ho, wo]), ops.int_array([n, c, di, hi, wi])
+    size = workspace_size(ops, "aclnnUpsampleTrilinear3dBackward", tg.ptr, osz.ptr, isz.ptr, False, 0.0, 0.0, 0.0, ti.ptr)
+    w_stage, h_stage = n * c * do * ho * wi * 4, n * c * do * hi * wi * 4
+    tables = 20000  # starts, counts and weights of the three axes, every piece rounded up to 256 bytes
+    need = h_stage + (w_stage if stages == 2 else 0)
+    assert need <= size <= need + tables
