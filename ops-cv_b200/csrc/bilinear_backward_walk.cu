@@ -1,4 +1,6 @@
-// UpsampleBilinear2dBackward, the row walks that serve any up-scale.
+// UpsampleBilinear2dBackward, the row walks that serve up-scales by whole factors or not, up to where the grads of one group
+// (below) no longer fit the shared memory of a block: NCHW rows of 4096 grads columns at small factors, of fp32 2048 at a
+// factor of eight and 1280 at sixteen; NHWC a factor of about ten.
 //
 // Both kernels use the same view of an axis: lo(d), the lower of the two grad_input indices that grads index d feeds,
 // grows with d, so the grads indices with lo = y form one run ("group" y). grad_input index y is fed by group y - 1
@@ -728,17 +730,19 @@ int32_t PickBandRows(int32_t rows, int64_t blocksPerBand, int64_t slots)
     return static_cast<int32_t>(std::max<int64_t>(best, CeilDiv(rows, 65535)));
 }
 
-// Launch shape of the column kernel; false where it does not take the call.
+// Launch shape of the column kernel.
 struct ColumnsPlan {
     ColumnsShape q;
     int32_t k, threads, bands; // columns per thread
     int64_t planeGroups;
     size_t smem;
 };
-bool PlanColumns(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, ColumnsPlan* plan)
+constexpr int32_t kColumnsThreads = 256; // per block, to aim for
+
+// With so many planes per block; false where that needs more than mostSmem bytes of shared memory.
+bool PlanColumnsOf(int32_t planesPerBlock, size_t mostSmem, int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw,
+                   ColumnsPlan* plan)
 {
-    constexpr int32_t kTarget = 256; // threads per block to aim for
-    constexpr size_t kMostSmem = 96 * 1024;
     const int64_t planes = sh.n * sh.c;
     ColumnsShape& q = plan->q;
     q = ColumnsShape{};
@@ -746,17 +750,8 @@ bool PlanColumns(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw,
     q.win = sh.win;
     q.hout = sh.hout;
     q.wout = sh.wout;
-    // columns per thread: as many as leave a thread for every horizontal sum of a finished row, at least as many as the
-    // width of a row needs
-    int32_t k = 1;
-    while (k < 8 && ((k < 4 && CeilDiv(sh.wout, 2 * k) >= sh.win) || k * (kTarget + 64) < sh.wout)) {
-        k *= 2;
-    }
-    q.team = static_cast<int32_t>(CeilDiv(sh.wout, k));
-    if (q.team > 512) {
-        return false;
-    }
-    q.planesPerBlock = static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(planes, kTarget / q.team)));
+    q.team = static_cast<int32_t>(CeilDiv(sh.wout, plan->k));
+    q.planesPerBlock = planesPerBlock;
     const int32_t threads = static_cast<int32_t>(CeilDiv(q.planesPerBlock * q.team, 32)) * 32 + 32; // and the copying warp
     const int64_t planeGroups = CeilDiv(planes, q.planesPerBlock);
     // about eight grads rows per stage, no more than some twelve kilobytes of them; three stages unless they are large
@@ -765,7 +760,7 @@ bool PlanColumns(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw,
     q.stageGroups = static_cast<int32_t>(std::min(8.0f, 12288.0f / (static_cast<float>(rowBytes) * q.planesPerBlock)) / perGroup);
     q.stageGroups = std::max(1, std::min(q.stageGroups, kColumnsBatch));
     const int64_t slotBytes = (static_cast<int64_t>(MostRows(ah, q.stageGroups)) * rowBytes + 30) / 16 * 16;
-    if (slotBytes * q.planesPerBlock > static_cast<int64_t>(kMostSmem)) {
+    if (slotBytes * q.planesPerBlock > static_cast<int64_t>(mostSmem)) {
         return false;
     }
     q.slotBytes = static_cast<int32_t>(slotBytes);
@@ -779,12 +774,37 @@ bool PlanColumns(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw,
     while (q.lanesLog < 3 && (2 << q.lanesLog) <= perOutput) {
         ++q.lanesLog;
     }
-    plan->k = k;
     plan->threads = threads;
     plan->bands = bands;
     plan->planeGroups = planeGroups;
     plan->smem = ColumnsSmem(q);
-    return plan->smem <= kMostSmem && planeGroups <= 0x7fffffff && bands <= 65535;
+    return plan->smem <= mostSmem && planeGroups <= 0x7fffffff && bands <= 65535;
+}
+
+// False where the kernel does not take the call.
+bool PlanColumns(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, ColumnsPlan* plan)
+{
+    // columns per thread: as many as leave a thread for every horizontal sum of a finished row, at least as many as the
+    // width of a row needs
+    int32_t& k = plan->k;
+    k = 1;
+    while (k < 8 && ((k < 4 && CeilDiv(sh.wout, 2 * k) >= sh.win) || k * (kColumnsThreads + 64) < sh.wout)) {
+        k *= 2;
+    }
+    const int32_t team = static_cast<int32_t>(CeilDiv(sh.wout, k));
+    if (team > 512) {
+        return false;
+    }
+    // A stage holds a whole group of grads rows, which grows with the scale. Two blocks per SM, with fewer planes each if need
+    // be; a single block of one plane beats the kernel without a walk by far (fp32 4
+    // planes 160x160 <- 1280x1280: 569 us without, 15 with).
+    int32_t planes = static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(sh.n * sh.c, kColumnsThreads / team)));
+    for (; planes > 1; planes = (planes + 1) / 2) {
+        if (PlanColumnsOf(planes, 96 * 1024, es, sh, ah, aw, plan)) {
+            return true;
+        }
+    }
+    return PlanColumnsOf(1, 224 * 1024, es, sh, ah, aw, plan);
 }
 
 template <typename TIn, typename TOut>

@@ -151,8 +151,9 @@ bool BilinearFwdTakesPitch(Dt dt, Layout lay, const void* x, const void* y, Shap
 cudaError_t BilinearBwdGather(Dt dtIn, Dt dtOut, Layout lay, const void* go, void* gi, Shape4 sh, LerpAxis th,
                               LerpAxis tw, RangeAxis rh, RangeAxis rw, const BilinearPlan& plan, cudaStream_t s,
                               bool buildTables = false, const ViewStrides* gradsPitch = nullptr);
-// The row walks that serve any up-scale (bilinear_backward_walk.cu): launches one and returns true, or returns false
-// without a launch (down-scales, user scales that run past the input, rows too long for a block).
+// The row walks that serve up-scales (bilinear_backward_walk.cu): launches one and returns true, or returns false without a
+// launch (down-scales, user scales that run past the input, grads rows of a group or grads columns of a tile that do not fit
+// a block's shared memory, extents past 2^24, NHWC channels that are no multiple of 16 bytes).
 bool BilinearBwdWalk(Dt dtIn, Dt dtOut, Layout lay, const void* go, void* gi, Shape4 sh, AxisGeom gh, AxisGeom gw,
                      bool halfPixel, cudaStream_t s);
 // The launch shape behind it (values as documented at opscvDebugPlan); false where it does not take the call.

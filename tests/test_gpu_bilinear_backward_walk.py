@@ -1,4 +1,4 @@
-"""The row walks of the bilinear backward that serve any up-scale (bilinear_backward_walk.cu): against the oracle's scatter
+"""The row walks of the bilinear backward at up-scales (bilinear_backward_walk.cu): against the oracle's scatter
 kernel at the edges of their tiles. NHWC adds the scatter's products in its order: the same bits. NCHW sums rows first:
 a sum of n terms of magnitude m is off by at most n * 2^-24 * m, here n <= 400 terms of weight sum 1 per axis step."""
 import numpy as np
@@ -29,8 +29,8 @@ NCHW = [
     (2, 5, 7, 13, 13, 25),     # 2h - 1: odd rows, one column per thread short of two
     (3, 7, 25, 21, 50, 42),    # 2x with rows that are no multiple of 4
     (1, 2, 65, 65, 513, 513),  # eight times: lanes share a sum, bands split the rows
-    (1, 1, 3, 50, 40, 1300),   # rows wider than a block of one column per thread
-    (1, 1, 2, 9, 3, 3000),     # eight columns per thread
+    (1, 1, 3, 50, 40, 1300),   # a factor of 26 at which grads of four bytes do not fit a block: the kernel without a walk
+    (1, 1, 2, 9, 3, 3000),     # a factor of 333 along the row
     (40, 9, 3, 4, 5, 7),       # many planes per block, a partial last group
     (1, 1, 300, 2, 301, 3),    # long columns, narrow rows
     (1, 1, 2, 3, 2, 5000),     # a row too long for the walk: the direct kernel
@@ -90,3 +90,47 @@ def test_nonfinite_grads(ops, oracle, dev, fmt, align, shape):
     ref = oracle.bilinear2d_bwd(g32, (hi, wi), align, fmt=getattr(oracle, fmt))
     for test in (np.isnan, np.isposinf, np.isneginf):
         assert np.array_equal(test(got), test(ref))
+
+
+# (shape, columns per thread, planes per block): every instantiation, one block per SM, few planes for want of shared memory
+REACHED = [((2, 3, 5, 40, 9, 45), 1, 5), ((3, 5, 9, 30, 20, 70), 2, 7), ((1, 1, 10, 500, 20, 1000), 4, 1),
+           ((2, 1, 20, 900, 40, 1800), 8, 1), ((1, 2, 4, 1500, 9, 4000), 8, 1), ((1, 1, 3, 2000, 5, 4096), 8, 1),
+           ((1, 2, 33, 65, 260, 520), 4, 1), ((2, 3, 16, 16, 256, 256), 4, 1)]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("align", [False, True])
+@pytest.mark.parametrize("shape,per_thread,planes", REACHED)
+def test_nchw_columns_are_reached(ops, oracle, dev, dtype, align, shape, per_thread, planes):
+    n, c, hi, wi, ho, wo = shape
+    plan = ops.debug_plan("bilinear_backward_walk", 4 if dtype == torch.float32 else 2, shape, "NCHW", align)
+    assert plan is not None and plan[4] == per_thread and planes <= plan[5] <= max(planes, 4)
+    g, g32 = _grads((n, c, ho, wo), dtype, 10)
+    got = ops.upsample_bilinear2d_backward(g.to(dev), (ho, wo), (n, c, hi, wi), align)
+    _close(got, oracle.bilinear2d_bwd(g32, (hi, wi), align), dtype)
+
+
+@pytest.mark.parametrize("fmt", ["NCHW", "NHWC"])
+@pytest.mark.parametrize("scale,taken", [(2.2, False), (2.4, True), (2.5, True), (2.7, True), (4.0, True)])
+def test_user_scales(ops, oracle, dev, fmt, scale, taken):
+    """Scales that run past the input pile grads up on its last row and column: to the other kernels; smaller steps than the
+    extents suggest leave the last rows and columns without grads."""
+    n, c, hi, wi, ho, wo = 2, 8, 24, 20, 60, 50
+    plan = ops.debug_plan("bilinear_backward_walk", 4, (n, c, hi, wi, ho, wo), fmt, False, (scale, scale))
+    assert (plan is not None) == taken
+    full, size = ((n, ho, wo, c), (n, hi, wi, c)) if fmt == "NHWC" else ((n, c, ho, wo), (n, c, hi, wi))
+    g, g32 = _grads(full, torch.float32, 11)
+    got = ops.upsample_bilinear2d_backward(g.to(dev), (ho, wo), size, False, fmt, scales=(scale, scale))
+    ref = oracle.bilinear2d_bwd(g32, (hi, wi), False, (scale, scale), fmt=getattr(oracle, fmt))
+    _close(got, ref, torch.float32)
+
+
+@pytest.mark.parametrize("fmt,c,hi,ho", [("NHWC", 48, 5000, 12001), ("NCHW", 3, 5000, 12001), ("NHWC", 8, 5000, 9001)])
+def test_tall_planes(ops, oracle, dev, fmt, c, hi, ho):
+    """More than 64 bands, and the narrow image that the gather kernel serves."""
+    plan = ops.debug_plan("bilinear_backward_walk", 4, (1, c, hi, 5, ho, 9), fmt)
+    assert plan is None if c == 8 else -(-hi // plan[0]) > 64
+    full, size = ((1, ho, 9, c), (1, hi, 5, c)) if fmt == "NHWC" else ((1, c, ho, 9), (1, c, hi, 5))
+    g, g32 = _grads(full, torch.float32, 12)
+    got = ops.upsample_bilinear2d_backward(g.to(dev), (ho, 9), size, False, fmt)
+    _close(got, oracle.bilinear2d_bwd(g32, (hi, 5), False, fmt=getattr(oracle, fmt)), torch.float32)

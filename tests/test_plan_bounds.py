@@ -39,7 +39,7 @@ def check_walk(ops, fmt, elem, n, c, hi, wi, ho, wo, align):
     if plan is None:
         return False
     band, band_cap, group, group_cap, _, _, _, smem = plan
-    assert 0 < smem <= 112 * 1024
+    assert 0 < smem <= (224 if fmt == "NCHW" else 112) * 1024
     rows = group_starts(hi, ho, align)
     assert most(rows, np.arange(0, hi, band) - 1, band + 1) <= band_cap
     if fmt == "NCHW":  # a stage: any run of groups that starts a multiple of them from a band's first
