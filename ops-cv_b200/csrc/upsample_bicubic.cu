@@ -540,36 +540,34 @@ __device__ float BwdElementDirect(const T* __restrict__ pg, const BicubicGeom& g
 // so the sum has the same bits. The additions of a thread are one chain; what it must not wait for one by one are the
 // loads, so the grads values of kListBatch columns are fetched before the first of them is used (border columns of
 // fp32 8x64 planes 60x80 <- 150x199: 58 us with one load at a time, 38 us in batches).
-// The blocks of a launch divide its element positions (of all columns, or of the first and the last, or of those between)
-// by x and its rows by y; colsPB positions per block, further threads take further rows.
-// TAPS: most taps of a list's column, one where the border columns are not among them.
+// The blocks of a launch divide its element positions (of all columns, or of the first and the last) by x and its rows by y;
+// colsPB positions per block, further threads take further rows.
 constexpr int kListBatch = 8;
 constexpr int kListTaps = 3; // a fourth needs an extent of 1
 constexpr int kListThreads = 128;
-constexpr int ListBytes(int taps) { return 4 + 4 * taps; } // per column and thread
-enum ListColumns { kAllColumns, kBorderColumns, kInteriorColumns };
+constexpr int kListBytes = 4 + 4 * kListTaps; // per column and thread
+constexpr int kInteriorBytes = 4;             // and of a list of interior columns
 struct ListShape {
     int32_t colsPB, entries, x, y;
 };
 
-template <typename T, bool NHWC, int TAPS>
+template <typename T, bool NHWC>
 __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __restrict__ gi, const BicubicGeom& g,
-                                             int32_t maxW, int32_t colsPB, ListColumns columns, float* sList, int32_t blockX,
+                                             int32_t maxW, int32_t colsPB, bool borderOnly, float* sList, int32_t blockX,
                                              int64_t blockY, int64_t blocksY)
 {
     const int32_t nt = blockDim.x, tid = threadIdx.x;
-    float* sCoef = sList; // [maxW][TAPS][nt]
-    int32_t* sCol = reinterpret_cast<int32_t*>(sList + static_cast<size_t>(maxW) * TAPS * nt); // column << 2 | taps
+    float* sCoef = sList; // [maxW][kListTaps][nt]
+    int32_t* sCol = reinterpret_cast<int32_t*>(sList + static_cast<size_t>(maxW) * kListTaps * nt); // column << 2 | taps
     const int32_t inner = g.win * g.chan;
     const int32_t rowsPB = nt / colsPB;
     const int32_t rowLane = tid / colsPB;
     const int32_t pos = blockX * colsPB + (tid - rowLane * colsPB);
-    const int32_t positions = columns == kAllColumns ? inner : (columns == kBorderColumns ? 2 * g.chan : inner - 2 * g.chan);
-    if (rowLane >= rowsPB || pos >= positions) {
+    if (rowLane >= rowsPB || pos >= (borderOnly ? 2 * g.chan : inner)) {
         return;
     }
-    int32_t t = columns == kInteriorColumns ? pos + g.chan : pos;
-    if (columns == kBorderColumns) {
+    int32_t t = pos;
+    if (borderOnly) {
         const int32_t side = NHWC ? pos / g.chan : pos;
         t = side == 0 ? pos : inner - 2 * g.chan + pos; // column 0 or column win - 1, same channel
     }
@@ -578,7 +576,7 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
     const int64_t planeGo = static_cast<int64_t>(g.hout) * g.wout * g.chan;
     const int64_t rowGo = static_cast<int64_t>(g.wout) * g.chan;
     const float offset = g.align ? 0.0f : 0.5f;
-    const bool borderW = columns != kInteriorColumns && (yw == 0 || yw == g.win - 1);
+    const bool borderW = yw == 0 || yw == g.win - 1;
 
     // the column walk, once
     int32_t cnt = 0;
@@ -599,8 +597,8 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (!overflow && ClampIdx(fw - 1 + j, g.win - 1) == yw) {
-                        if (n < TAPS) {
-                            sCoef[(cnt * TAPS + n) * nt + tid] = cwTap[j];
+                        if (n < kListTaps) {
+                            sCoef[(cnt * kListTaps + n) * nt + tid] = cwTap[j];
                             ++n;
                         } else {
                             overflow = true;
@@ -617,7 +615,7 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
                 }
                 overflow = cnt >= maxW || w >= (1 << 29);
                 if (!overflow) {
-                    sCoef[cnt * TAPS * nt + tid] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
+                    sCoef[cnt * kListTaps * nt + tid] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
                     sCol[cnt * nt + tid] = w << 2 | 1;
                     ++cnt;
                 }
@@ -685,12 +683,12 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
                     if (taps[u] == 0) {
                         break;
                     }
-                    const float* cu = sCoef + (k0 + u) * TAPS * nt + tid;
+                    const float* cu = sCoef + (k0 + u) * kListTaps * nt + tid;
                     for (int i = 0; i < nH; ++i) {
                         const float gc = Mul(gv[u], i == 0 ? chv[0] : (i == 1 ? chv[1] : (i == 2 ? chv[2] : chv[3])));
 #pragma unroll
-                        for (int j = 0; j < TAPS; ++j) {
-                            if (TAPS == 1 || j < taps[u]) {
+                        for (int j = 0; j < kListTaps; ++j) {
+                            if (j < taps[u]) {
                                 add = Add(add, Mul(gc, cu[j * nt]));
                             }
                         }
@@ -702,9 +700,131 @@ __device__ __forceinline__ void BwdListBlock(const T* __restrict__ go, T* __rest
     }
 }
 
+// The same for the interior columns, whose grads columns follow one another from the start of the walk with one coefficient
+// each: a list is its coefficients, 4 bytes per column and thread, and a term is one load, two products and one addition.
+// All terms of a batch are formed before the first is added. What bounds it is instruction issue on the terms, which the general
+// block spends on columns, taps and bounds as well (fp32 8x38 planes 97x104 <- 35x712: 377 us by general lists).
+template <typename T, bool NHWC>
+__device__ __forceinline__ void BwdInteriorListBlock(const T* __restrict__ go, T* __restrict__ gi, const BicubicGeom& g,
+                                                     int32_t maxW, int32_t colsPB, float* sCoef, int32_t blockX, int64_t blockY,
+                                                     int64_t blocksY)
+{
+    const int32_t nt = blockDim.x, tid = threadIdx.x; // sCoef: [maxW][nt]
+    const int32_t inner = g.win * g.chan;
+    const int32_t rowsPB = nt / colsPB, rowLane = tid / colsPB;
+    const int32_t pos = blockX * colsPB + (tid - rowLane * colsPB);
+    if (rowLane >= rowsPB || pos >= inner - 2 * g.chan) {
+        return;
+    }
+    const int32_t t = pos + g.chan;
+    const int32_t yw = NHWC ? t / g.chan : t;
+    const int32_t c = NHWC ? t - yw * g.chan : 0;
+    const int64_t rowGo = static_cast<int64_t>(g.wout) * g.chan, planeGo = g.hout * rowGo;
+    const float offset = g.align ? 0.0f : 0.5f;
+    const int32_t wStart = WalkStart(yw, g.invW, offset);
+    const float* coef = sCoef + tid;
+    int32_t cnt = 0;
+    bool overflow = false;
+    for (int32_t w = wStart; w < g.wout; ++w) {
+        const float rw = BwdSrc(g.scaleW, w, g.align);
+        if (!(rw < Add(static_cast<float>(yw), 2.0f))) {
+            break;
+        }
+        overflow = cnt >= maxW;
+        if (overflow) {
+            break;
+        }
+        sCoef[cnt * nt + tid] = PointCoeff(fabsf(Sub(rw, static_cast<float>(yw))));
+        ++cnt;
+    }
+    const int32_t step = NHWC ? g.chan : 1;
+    for (int64_t row = blockY * rowsPB + rowLane; row < g.rows; row += blocksY * rowsPB) {
+        const int64_t plane = row / g.hin;
+        const int32_t yh = static_cast<int32_t>(row - plane * g.hin);
+        const T* pg = go + plane * planeGo;
+        T* dst = gi + row * inner + t;
+        if (overflow) {
+            *dst = DType<T>::FromF(BwdElementDirect<T>(pg, g, yh, yw, c, rowGo, offset));
+            continue;
+        }
+        const bool borderH = yh == 0 || yh == g.hin - 1;
+        float add = 0.0f;
+        for (int32_t h = WalkStart(yh, g.invH, offset); h < g.hout; ++h) {
+            const float rh = BwdSrc(g.scaleH, h, g.align);
+            float chv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            int nH = 1;
+            if (!borderH) {
+                if (!(rh < Add(static_cast<float>(yh), 2.0f))) {
+                    break;
+                }
+                chv[0] = PointCoeff(fabsf(Sub(rh, static_cast<float>(yh))));
+            } else {
+                const long long fh = static_cast<long long>(floorf(rh));
+                if (yh == 0 && fh > 1 && g.hin > 1) {
+                    break;
+                }
+                float chTap[4];
+                TapCoeff(Sub(rh, static_cast<float>(fh)), chTap);
+                nH = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (ClampIdx(fh - 1 + i, g.hin - 1) == yh) { // compacted in tap order
+                        chv[3] = chTap[i];
+                        if (nH == 0) chv[0] = chTap[i];
+                        if (nH == 1) chv[1] = chTap[i];
+                        if (nH == 2) chv[2] = chTap[i];
+                        ++nH;
+                    }
+                }
+            }
+            const T* p = pg + h * rowGo + static_cast<int64_t>(wStart) * step + c;
+            const float* cp = coef;
+            int32_t k = 0;
+            if (nH == 1) {
+                const float ch = chv[0];
+#pragma unroll 1
+                for (; k + kListBatch <= cnt; k += kListBatch, p += kListBatch * static_cast<int64_t>(step), cp += kListBatch * nt) {
+                    float term[kListBatch];
+#pragma unroll
+                    for (int u = 0; u < kListBatch; ++u) {
+                        term[u] = DType<T>::Load(p + u * step);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kListBatch; ++u) {
+                        term[u] = Mul(Mul(term[u], ch), cp[u * nt]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kListBatch; ++u) {
+                        add = Add(add, term[u]);
+                    }
+                }
+                float term[kListBatch]; // what is left, all loads in flight as well
+#pragma unroll
+                for (int u = 0; u < kListBatch - 1; ++u) {
+                    term[u] = k + u < cnt ? DType<T>::Load(p + u * step) : 0.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < kListBatch - 1; ++u) {
+                    if (k + u < cnt) {
+                        add = Add(add, Mul(Mul(term[u], ch), cp[u * nt]));
+                    }
+                }
+            } else {
+#pragma unroll 4
+                for (; k < cnt; ++k, p += step, cp += nt) {
+                    const float gv = DType<T>::Load(p), cw = *cp;
+                    for (int i = 0; i < nH; ++i) {
+                        add = Add(add, Mul(Mul(gv, i == 0 ? chv[0] : (i == 1 ? chv[1] : (i == 2 ? chv[2] : chv[3]))), cw));
+                    }
+                }
+            }
+        }
+        *dst = DType<T>::FromF(add);
+    }
+}
+
 // All columns by lists (scales beyond four, user scales that contradict the extents, extents of two): the border columns in
-// the first blocks, whose chains are the longest, the interior ones behind them with one coefficient per column. With room
-// for three in every list fewer of them fit (fp32 4x16 planes 32x64 <- 512x1024: 4223 us; so 2072 us).
+// the first blocks, whose chains are the longest, the interior ones behind them.
 template <typename T, bool NHWC>
 __global__ void __launch_bounds__(kListThreads) Bicubic2dBwdListKernel(const T* __restrict__ go, T* __restrict__ gi, BicubicGeom g,
                                                                         ListShape border, ListShape interior)
@@ -712,14 +832,14 @@ __global__ void __launch_bounds__(kListThreads) Bicubic2dBwdListKernel(const T* 
     extern __shared__ __align__(16) float sList[];
     const int32_t block = blockIdx.x, borders = border.x * border.y;
     if (g.win <= 2) {
-        BwdListBlock<T, NHWC, kListTaps>(go, gi, g, border.entries, border.colsPB, kAllColumns, sList, block % border.x,
+        BwdListBlock<T, NHWC>(go, gi, g, border.entries, border.colsPB, false, sList, block % border.x,
                                          block / border.x, border.y);
     } else if (block < borders) {
-        BwdListBlock<T, NHWC, kListTaps>(go, gi, g, border.entries, border.colsPB, kBorderColumns, sList, block % border.x,
+        BwdListBlock<T, NHWC>(go, gi, g, border.entries, border.colsPB, true, sList, block % border.x,
                                          block / border.x, border.y);
     } else {
-        BwdListBlock<T, NHWC, 1>(go, gi, g, interior.entries, interior.colsPB, kInteriorColumns, sList,
-                                 (block - borders) % interior.x, (block - borders) / interior.x, interior.y);
+        BwdInteriorListBlock<T, NHWC>(go, gi, g, interior.entries, interior.colsPB, sList, (block - borders) % interior.x,
+                                      (block - borders) / interior.x, interior.y);
     }
 }
 
@@ -764,7 +884,7 @@ __global__ void __launch_bounds__(kWalkThreads, (NHWC && K > 14) ? 3 : ((NHWC ||
     extern __shared__ __align__(16) float sWalk[];
     const int32_t lists = ws.list.x * ws.list.y;
     if (static_cast<int32_t>(blockIdx.x) < lists) {
-        BwdListBlock<T, NHWC, kListTaps>(go, gi, g, ws.list.entries, ws.list.colsPB, kBorderColumns, sWalk,
+        BwdListBlock<T, NHWC>(go, gi, g, ws.list.entries, ws.list.colsPB, true, sWalk,
                                          static_cast<int32_t>(blockIdx.x) % ws.list.x,
                                          static_cast<int32_t>(blockIdx.x) / ws.list.x, ws.list.y);
         return;
@@ -1535,15 +1655,15 @@ dim3 RowGrid(int64_t rows, int64_t inner)
 }
 
 // ---- launch shapes of the general backward ------------------------------------------------------------------------
-// A launch of `positions` element positions per row, columns of up to `taps` taps, `threads` threads per block. Columns of one
+// A launch of `positions` element positions per row, lists of `bytes` per column, `threads` threads per block. Columns of one
 // list: four source pixels for an interior column, two and a half for a first or last one (three, for user scales). Lists that
 // would not fit make their thread fall back to the uncached walk, so the bound only has to be good, not safe; a
 // single-column image (every grads column is a tap) always falls back.
-ListShape PlanBwdList(const BicubicGeom& g, int64_t positions, int taps, int threads, double span)
+ListShape PlanBwdList(const BicubicGeom& g, int64_t positions, int bytes, int threads, double span)
 {
     const double perScale = g.invW > 0.0f ? static_cast<double>(g.invW) : 1.0;
     const int64_t maxW = static_cast<int64_t>(std::ceil(span * perScale)) + 4;
-    const int64_t cap = (taps == 1 ? 96 : 192) * 1024 / (ListBytes(taps) * threads);
+    const int64_t cap = (bytes == kInteriorBytes ? 96 : 192) * 1024 / (bytes * threads);
     ListShape l;
     l.colsPB = static_cast<int32_t>(std::min<int64_t>(threads, positions));
     const int rowsPB = threads / l.colsPB;
@@ -1553,9 +1673,9 @@ ListShape PlanBwdList(const BicubicGeom& g, int64_t positions, int taps, int thr
     l.y = static_cast<int32_t>(std::min<int64_t>(std::min<int64_t>(CeilDiv(g.rows, rowsPB), gyCap), 65535));
     return l;
 }
-size_t ListSmem(const ListShape& l, int taps, int threads)
+size_t ListSmem(const ListShape& l, int bytes, int threads)
 {
-    return static_cast<size_t>(l.entries) * threads * ListBytes(taps);
+    return static_cast<size_t>(l.entries) * threads * bytes;
 }
 
 // The list kernel alone.
@@ -1571,19 +1691,19 @@ BwdListPlan PlanBwdLists(const BicubicGeom& g)
     BwdListPlan p{};
     if (g.win <= 2) {
         p.threads = kListThreads;
-        p.border = PlanBwdList(g, inner, kListTaps, p.threads, 4.0);
+        p.border = PlanBwdList(g, inner, kListBytes, p.threads, 4.0);
     } else {
         // equal shares of a row for its blocks, so that none of them is nearly empty, and no more threads than that needs:
         // fewer threads leave room for longer lists
         const int64_t positions = inner - 2LL * g.chan, share = CeilDiv(positions, CeilDiv(positions, kListThreads));
         p.threads = static_cast<int32_t>(std::max<int64_t>(64, (share + 31) / 32 * 32));
-        p.border = PlanBwdList(g, 2LL * g.chan, kListTaps, p.threads, 3.0);
-        p.interior = PlanBwdList(g, positions, 1, p.threads, 4.0);
+        p.border = PlanBwdList(g, 2LL * g.chan, kListBytes, p.threads, 3.0);
+        p.interior = PlanBwdList(g, positions, kInteriorBytes, p.threads, 4.0);
         p.blocks = static_cast<int64_t>(p.interior.x) * p.interior.y;
-        p.smem = ListSmem(p.interior, 1, p.threads);
+        p.smem = ListSmem(p.interior, kInteriorBytes, p.threads);
     }
     p.blocks += static_cast<int64_t>(p.border.x) * p.border.y;
-    p.smem = std::max(p.smem, ListSmem(p.border, kListTaps, p.threads));
+    p.smem = std::max(p.smem, ListSmem(p.border, kListBytes, p.threads));
     return p;
 }
 
@@ -1613,7 +1733,7 @@ bool PlanBwdWalk(const BicubicGeom& g, BwdWalkPlan* plan)
         return false;
     }
     const int64_t planes = g.rows / g.hin;
-    const ListShape l = PlanBwdList(g, 2LL * g.chan, kListTaps, kListThreads, 4.0);
+    const ListShape l = PlanBwdList(g, 2LL * g.chan, kListBytes, kListThreads, 4.0);
     WalkShape& ws = plan->ws;
     ws = WalkShape{};
     ws.positions = planes * (inner - 2LL * g.chan);
@@ -1651,7 +1771,7 @@ bool PlanBwdWalk(const BicubicGeom& g, BwdWalkPlan* plan)
     ws.maxRows = static_cast<int32_t>(bandReads(ws.bandRows));
     ws.walkX = static_cast<int32_t>(gx);
     ws.list = l;
-    plan->smem = std::max(ListSmem(l, kListTaps, kListThreads), bandSmem(ws.bandRows));
+    plan->smem = std::max(ListSmem(l, kListBytes, kListThreads), bandSmem(ws.bandRows));
     return true;
 }
 
