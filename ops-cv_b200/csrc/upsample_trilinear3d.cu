@@ -605,6 +605,14 @@ bool PlanPlane(const Trilinear3dGeom& g, const int32_t (&taps)[3], int es, int64
     if (g.chan != 1 || taps[2] > 10 || taps[1] > 64 || g.ho > (1 << 24) || g.hi > (1 << 24)) {
         return false;
     }
+    // Many small slices: a block's phases take their latency whatever the slice holds, while the stage kernels pack rows of all
+    // slices (and four columns per thread where rows allow it). us by planes and by stages, 4800 slices, fp32, twice the extents:
+    // 4x4 28 / 17, 16x16 31 / 24, 24x24 39 / 40, 32x32 48 / 59; 7x9 27 / 23, 28x11 35 / 35, 15x17 33 / 35; with 1024 slices
+    // no size is faster by stages. 107x6 <- 56x9: 37 / 47.
+    const int64_t slice = static_cast<int64_t>(g.ho) * g.wo;
+    if (slices > 1536 && slice < (g.wi % 4 == 0 ? 2000 : 500)) {
+        return false;
+    }
     PlaneShape p{slices, g.ho, g.wo, g.hi, g.wi, 0, 0, 0, taps[1], taps[2]};
     // grad_output rows of a band: source positions are scale apart
     const double perRow = g.sh > 0.0f ? 1.0 / static_cast<double>(g.sh) : static_cast<double>(g.ho);

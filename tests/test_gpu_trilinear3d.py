@@ -155,3 +155,18 @@ def test_trilinear3d_backward_planes(ops, oracle, dev, dtype, align, shape):
     g, g32 = quant(torch.randn((n, c, do, ho, wo), generator=gen(140)), dtype)
     gi = ops.upsample_trilinear3d_backward(g.to(dev), (do, ho, wo), (n, c, di, hi, wi), align)
     check(gi, oracle.trilinear3d_bwd(g32, (di, hi, wi), align), dtype, exact=(dtype == torch.float32))
+
+
+# either side of the line between the plane kernel (one launch for the W and the H stage) and the stage kernels
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape,launches", [((1, 100, 8, 4, 4, 16, 8, 8), 4), ((1, 64, 8, 4, 4, 16, 8, 8), 3),
+                                            ((2, 50, 8, 7, 9, 16, 14, 18), 4), ((2, 50, 8, 15, 17, 16, 30, 34), 3),
+                                            ((1, 100, 8, 24, 24, 16, 48, 48), 3), ((1, 100, 8, 20, 20, 16, 40, 40), 4)])
+def test_trilinear3d_backward_of_many_slices(ops, oracle, dev, dtype, shape, launches):
+    n, c, di, hi, wi, do, ho, wo = shape
+    g, g32 = quant(torch.randn((n, c, do, ho, wo), generator=gen(141)), dtype)
+    g = g.to(dev)
+    ops.reset_launch_count()
+    gi = ops.upsample_trilinear3d_backward(g, (do, ho, wo), (n, c, di, hi, wi))
+    assert ops.launch_count() == launches
+    check(gi, oracle.trilinear3d_bwd(g32, (di, hi, wi), False), dtype, exact=(dtype == torch.float32))
