@@ -784,11 +784,14 @@ bool PlanColumnsOf(int32_t planesPerBlock, size_t mostSmem, int es, const Shape4
 // False where the kernel does not take the call.
 bool PlanColumns(int es, const Shape4& sh, const BwdAxis& ah, const BwdAxis& aw, ColumnsPlan* plan)
 {
-    // columns per thread: as many as leave a thread for every horizontal sum of a finished row, at least as many as the
-    // width of a row needs
+    // columns per thread: at least as many as the width of a row needs, and no more than leave a thread for every horizontal
+    // sum of a finished row (a second round of sums costs as much as the walk: fp32 400 planes 72x225 <- 108x337, 89 us)
     int32_t& k = plan->k;
     k = 1;
-    while (k < 8 && ((k < 4 && CeilDiv(sh.wout, 2 * k) >= sh.win) || k * (kColumnsThreads + 64) < sh.wout)) {
+    while (k < 8 && CeilDiv(sh.wout, k) > 512) {
+        k *= 2;
+    }
+    while (k < 8 && CeilDiv(sh.wout, 2 * k) >= sh.win && (k < 4 || k * (kColumnsThreads + 64) < sh.wout)) {
         k *= 2;
     }
     const int32_t team = static_cast<int32_t>(CeilDiv(sh.wout, k));
