@@ -1995,7 +1995,9 @@ aclnnStatus opscvDebugPlan(int32_t kind, int32_t elemSize, aclFormat format, con
         case 0: {
             const AxisGeom gh{sh.hin, sh.hout, BilinearGradScale(in.h, out.h, align, static_cast<float>(scales[0]))};
             const AxisGeom gw{sh.win, sh.wout, BilinearGradScale(in.w, out.w, align, static_cast<float>(scales[1]))};
-            *taken = DebugBilinearBwdWalk(elemSize, lay, sh, gh, gw, !align, values) ? 1 : 0;
+            const BilinearPlan p = MakeBilinearBwdPlan(elemSize == 4 ? Dt::F32 : Dt::F16, lay, sh, gh, gw, !align);
+            const bool tiles = p.schedule != BilinearPlan::kDirect && p.tileRows > 0;
+            *taken = DebugBilinearBwdWalk(elemSize, lay, sh, gh, gw, !align, tiles, values) ? 1 : 0;
             return ACLNN_SUCCESS;
         }
         case 1: {

@@ -153,11 +153,13 @@ cudaError_t BilinearBwdGather(Dt dtIn, Dt dtOut, Layout lay, const void* go, voi
                               bool buildTables = false, const ViewStrides* gradsPitch = nullptr);
 // The row walks that serve up-scales (bilinear_backward_walk.cu): launches one and returns true, or returns false without a
 // launch (down-scales, user scales that run past the input, grads rows of a group or grads columns of a tile that do not fit
-// a block's shared memory, extents past 2^24, NHWC channels that are no multiple of 16 bytes).
+// a block's shared memory, extents past 2^24, NHWC channels that are no multiple of 16 bytes; NCHW calls that the tile kernel
+// does sooner, where `tiles` says that it takes them).
 bool BilinearBwdWalk(Dt dtIn, Dt dtOut, Layout lay, const void* go, void* gi, Shape4 sh, AxisGeom gh, AxisGeom gw,
-                     bool halfPixel, cudaStream_t s);
+                     bool halfPixel, bool tiles, cudaStream_t s);
 // The launch shape behind it (values as documented at opscvDebugPlan); false where it does not take the call.
-bool DebugBilinearBwdWalk(int elemSize, Layout lay, Shape4 sh, AxisGeom gh, AxisGeom gw, bool halfPixel, int64_t values[8]);
+bool DebugBilinearBwdWalk(int elemSize, Layout lay, Shape4 sh, AxisGeom gh, AxisGeom gw, bool halfPixel, bool tiles,
+                          int64_t values[8]);
 bool BilinearBwdTakesPitch(Dt dtIn, Dt dtOut, Layout lay, const void* go, const void* gi, Shape4 sh,
                            const BilinearPlan& plan, const ViewStrides& grads);
 // Scatter backward with fp32 atomics into `acc` (fp32, N*C*hin*win, zeroed by this call). If dtOut is fp32 the

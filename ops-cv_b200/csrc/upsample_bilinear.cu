@@ -1774,7 +1774,8 @@ cudaError_t LaunchGather(Layout lay, const void* go, void* gi, Shape4 sh, LerpAx
                 BilinearBwdW2Kernel<TIn, TOut><<<grid, block, 0, s>>>(pg, po, planes, sh.hin, sh.win, sh.hout, th, tw,
                                                                       rh, tileRows);
             }
-        } else if (BilinearBwdWalk(DtOf<TIn>(), DtOf<TOut>(), lay, go, gi, sh, plan.geomH, plan.geomW, plan.halfPixel, s)) {
+        } else if (BilinearBwdWalk(DtOf<TIn>(), DtOf<TOut>(), lay, go, gi, sh, plan.geomH, plan.geomW, plan.halfPixel,
+                                   plan.schedule != BilinearPlan::kDirect && plan.tileRows > 0, s)) {
             // launched
         } else if (plan.schedule != BilinearPlan::kDirect && plan.tileRows > 0) {
             needTables();
@@ -1806,7 +1807,7 @@ cudaError_t LaunchGather(Layout lay, const void* go, void* gi, Shape4 sh, LerpAx
                 }
             });
         }
-    } else if (!BilinearBwdWalk(DtOf<TIn>(), DtOf<TOut>(), lay, go, gi, sh, plan.geomH, plan.geomW, plan.halfPixel, s)) {
+    } else if (!BilinearBwdWalk(DtOf<TIn>(), DtOf<TOut>(), lay, go, gi, sh, plan.geomH, plan.geomW, plan.halfPixel, false, s)) {
         needTables();
         const int elem = sizeof(TIn) > sizeof(TOut) ? sizeof(TIn) : sizeof(TOut);
         const int v = PickVec(elem, sh.c, {go, gi});

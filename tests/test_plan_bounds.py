@@ -262,3 +262,10 @@ def test_trilinear_backward_asks_for_the_scratch_that_it_uses(ops, shape, stages
     tables = 20000  # starts, counts and weights of the three axes, every piece rounded up to 256 bytes
     need = h_stage + (w_stage if stages == 2 else 0)
     assert need <= size <= need + tables
+
+
+@pytest.mark.parametrize("elem,size,walk", [(4, (1, 400, 100, 130, 110, 143), False), (2, (1, 400, 100, 130, 150, 195), False),
+                                            (4, (1, 400, 100, 130, 150, 195), True), (4, (1, 400, 100, 130, 200, 261), True),
+                                            (4, (1, 25, 100, 130, 110, 143), True), (2, (8, 21, 65, 65, 513, 513), True)])
+def test_bilinear_walk_leaves_large_calls_at_small_scales_to_the_tiles(ops, elem, size, walk):
+    assert (ops.debug_plan("bilinear_backward_walk", elem, size) is not None) == walk
